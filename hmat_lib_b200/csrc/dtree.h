@@ -16,6 +16,7 @@ namespace hb {
 
 struct ProductPlan;
 struct MixedState;
+struct MvItem;
 
 // A captured launch sequence of one product (CUDA graph), replayed by later
 // calls with the same tree, op, sizes, buffers and stream.
@@ -45,8 +46,12 @@ struct DeviceTree {
   std::mutex plan_mutex;
   std::shared_ptr<MixedState> mixed;   // int8 slices of the factors (mixed precision)
   std::shared_ptr<DeviceTree> transposed;   // H^T with the same geometry (mixed op T / L)
-  int *mv_woff = nullptr;              // single-vector product: W offset of every block
-  double *mv_w = nullptr;              // and W (made on the first such product)
+  // single-vector product (made on the first one): W offset of every block
+  // with the projection's work items behind it, and W
+  int *mv_woff = nullptr;
+  MvItem *mv_items = nullptr;          // inside mv_woff's allocation
+  int mv_nwide = 0, mv_nitems = 0;
+  double *mv_w = nullptr;
 
   DeviceTree() = default;
   DeviceTree(const DeviceTree &) = delete;
