@@ -31,6 +31,7 @@
 #include <numeric>
 
 #include "bjacobi.h"
+#include "dmma.cuh"
 #include "dtree.h"
 #include "jacobi.h"
 #include "tsqr.h"
@@ -116,12 +117,6 @@ struct PairSmem {
   int work;      // the pair failed the convergence test
 };
 
-__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(c[0]), "+d"(c[1])
-               : "d"(a), "d"(b));
-}
-
 // The test of a column pair with squared norms al, be and product ga: true
 // when it must be rotated.  Columns at or below theta are neither rotated nor
 // tested (all of them together hold at most sqrt(L) theta = 1e-3 tol ||A||_F
@@ -155,7 +150,7 @@ __device__ __forceinline__ void rotate_rows(double *xa, double *xb, long long ld
     for (int nt = 0; nt < kPair / 8; ++nt) {
       double c[2] = {0.0, 0.0};
 #pragma unroll
-      for (int kk = 0; kk < kPair / 4; ++kk) dmma(c, a[kk], wp[(4 * kk + tq) + (8 * nt + gq) * kLd]);
+      for (int kk = 0; kk < kPair / 4; ++kk) dmma884(c, a[kk], wp[(4 * kk + tq) + (8 * nt + gq) * kLd]);
       if (in) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -216,7 +211,7 @@ bj_pair_kernel(const BjDev *__restrict__ probs, const int2 *__restrict__ slots, 
 #pragma unroll
       for (int I = 0; I < 8; ++I)
 #pragma unroll
-        for (int J = I; J < 8; ++J) dmma(acc[t++], f[I], f[J]);
+        for (int J = I; J < 8; ++J) dmma884(acc[t++], f[I], f[J]);
 #pragma unroll
       for (int I = 0; I < 8; ++I) f[I] = nf[I];
     }

@@ -13,6 +13,7 @@
 #include <cstring>
 #include <memory>
 
+#include "dmma.cuh"
 #include "gemm_f64.h"
 
 namespace hb {
@@ -270,12 +271,6 @@ __device__ __forceinline__ void cp_async16(void *smem, const void *gmem, int src
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem),
                "r"(src_bytes));
-}
-
-__device__ __forceinline__ void dmma884(double (&c)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(c[0]), "+d"(c[1])
-               : "d"(a), "d"(b));
 }
 
 template <int BM, int BN, int WM, int WN, int BK>

@@ -1,4 +1,4 @@
-// Batched TSQR (Householder QR of 256-row chunks in shared memory, reduced
+// Batched TSQR (Householder QR of 256-row chunks in registers, reduced
 // up a tree of stacked R factors, explicit Q rebuilt top-down) plus the
 // small utility kernels of the randomized compression: Gaussian test
 // matrices, column norms.
@@ -9,6 +9,7 @@
 #include <algorithm>
 #include <chrono>
 
+#include "dmma.cuh"
 #include "gemm_f64.h"
 #include "tsqr.h"
 
@@ -16,7 +17,7 @@ namespace hb {
 
 namespace {
 
-constexpr int kQT = 256;   // threads per CTA (one row of a chunk each)
+constexpr int kQT = 256;   // threads per CTA
 
 struct QrChunk {
   double *A;
@@ -40,103 +41,200 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-__device__ __forceinline__ double block_sum(double v, double *red) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  v = warp_sum(v);
-  if (lane == 0) red[warp] = v;
-  __syncthreads();
-  double s = 0.0;
-#pragma unroll
-  for (int k = 0; k < kQT / 32; ++k) s += red[k];
-  __syncthreads();
-  return s;
-}
-
-constexpr size_t kQrSmem = sizeof(double) * (2 * kChunk * kPanel + 2 * kPanel + kQT / 32);
-static_assert(kChunk == kQT, "one thread per row of a chunk");
+constexpr int kQWarps = kQT / 32;
+constexpr int kLdG = kPanel + 1;   // leading dimension of the reflectors' products
+constexpr int kLdM = kPanel + 4;   // of M: fragment loads of a half-warp hit 16 banks
+static_assert(kChunk == 32 * kQWarps && kPanel == 32, "a warp per 32 rows, 4 x 8 values per lane");
 
 // Householder QR of one chunk (rows <= 256, w <= 32), LAPACK dlarfg
 // convention: H_j = I - tau_j v_j v_j^T, v_j(j) = 1, beta_j = -sign(x0)||x||.
-__global__ void __launch_bounds__(kQT) qr_chunk_kernel(const QrChunk *__restrict__ descs) {
+//
+// The chunk lives in registers in the fragment layout of the FP64 tensor-core
+// product: lane l of a warp holds rows l / 4 + 8 i (i < 4) of the warp's 32
+// and columns 4 s + l % 4 (s < 8).  A step is bound by its latency (one
+// reduction, a square root, two divisions), so it has a single barrier: the
+// products of column j's tail with every column, itself included, are summed
+// together, and the reflector is scaled afterwards.  The same products with
+// the finished columns are v_j^T v_c, which make the block form
+// Q = I - V T V^T: T^-1 has 1 / tau on the diagonal and v_l^T v_j above it, so
+// M = T V_1^T comes from one triangular solve and Q's columns are
+// [I; 0] - V M on the tensor cores, straight from V's registers.  The slots
+// rotate by one every four columns, so column j is always in slot 0 and no
+// register is indexed at run time.
+// 1024 chunks of 256 x 32 (a panel of every block at n = 32768): 1092 us with the
+// chunk in shared memory (one CTA per SM, five barriers a step), 191 us so.
+__global__ void __launch_bounds__(kQT, 2) qr_chunk_kernel(const QrChunk *__restrict__ descs) {
   const QrChunk D = descs[blockIdx.x];
-  extern __shared__ double sm[];
-  double *S = sm;                          // chunk, column-major, ld kChunk
-  double *E = S + kChunk * kPanel;         // explicit Q under construction
-  double *tau = E + kChunk * kPanel;
-  double *wv = tau + kPanel;
-  double *red = wv + kPanel;
+  __shared__ double red[2][kQWarps][kPanel];   // per warp: products with the columns by position
+  __shared__ double rowj[2][kPanel];           // row j before its step, by position
+  __shared__ double coef[kQWarps][kPanel];     // per warp: tau_j v_j^T a_c
+  __shared__ double G[kPanel * kLdG];          // v_j^T v_c at [j][c], c < j
+  __shared__ double M[kPanel * kLdM];          // V_1^T, then T V_1^T
+  __shared__ double tau[kPanel];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rg = lane >> 2, cg = lane & 3, row0 = 32 * warp + rg;
   const int r = D.rows, w = D.w, k = min(r, w);
 
-  for (int e = tid; e < kChunk * kPanel; e += kQT) {
-    const int i = e % kChunk, j = e / kChunk;
-    S[e] = (i < r && j < w) ? D.A[i + (long long)j * D.lda] : 0.0;
+  double a[4][8];
+#pragma unroll
+  for (int s = 0; s < 8; ++s)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int row = row0 + 8 * i, c = 4 * s + cg;
+      a[i][s] = (row < r && c < w) ? D.A[row + (long long)c * D.lda] : 0.0;
+    }
+
+  for (int j = 0; j < kPanel; ++j) {
+    const int cj = j & 3, par = j & 1;
+    if (j < k) {
+      // x = rows below j of column j, for every lane of the row
+      double x[4], d[8];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        x[i] = __shfl_sync(0xffffffffu, a[i][0], (lane & ~3) | cj);
+        if (row0 + 8 * i <= j) x[i] = 0.0;
+      }
+#pragma unroll
+      for (int s = 0; s < 8; ++s) {
+        d[s] = x[0] * a[0][s];
+#pragma unroll
+        for (int i = 1; i < 4; ++i) d[s] = fma(x[i], a[i][s], d[s]);
+      }
+      // summed over the eight row groups; lane l ends with slot l / 4, its
+      // own column group: position l
+#pragma unroll
+      for (int b = 4; b >= 1; b >>= 1) {
+        const bool hi = (rg & b) != 0;
+#pragma unroll
+        for (int q = 0; q < b; ++q) {
+          const double send = hi ? d[q] : d[q + b], keep = hi ? d[q + b] : d[q];
+          d[q] = keep + __shfl_xor_sync(0xffffffffu, send, 4 * b);
+        }
+      }
+      red[par][warp][lane] = d[0];
+      if (warp == 0 && rg == (j & 7)) {   // row j's owners
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+          const int i = j >> 3;
+          rowj[par][4 * s + cg] = i == 0 ? a[0][s] : i == 1 ? a[1][s] : i == 2 ? a[2][s] : a[3][s];
+        }
+      }
+      __syncthreads();   // the buffers of step j are written again in step j + 2
+      double dp = 0.0;
+#pragma unroll
+      for (int q = 0; q < kQWarps; ++q) dp += red[par][q][lane];
+      const double ajp = rowj[par][lane];
+      const double sigma2 = __shfl_sync(0xffffffffu, dp, cj);
+      const double x0 = __shfl_sync(0xffffffffu, ajp, cj);
+      double beta = x0, t = 0.0, scale = 0.0;
+      if (sigma2 > 0.0) {
+        const double nrm = sqrt(fma(x0, x0, sigma2));
+        beta = x0 >= 0.0 ? -nrm : nrm;
+        t = (beta - x0) / beta;
+        scale = 1.0 / (x0 - beta);
+      }
+      const int c = 4 * (((j >> 2) + rg) & 7) + cg;   // column at this lane's position
+      const double g = fma(scale, dp, ajp);           // v_j^T a_c
+      coef[warp][lane] = c > j ? t * g : 0.0;
+      if (warp == 0) {
+        if (c < j) G[j * kLdG + c] = g;
+        if (lane == 0) tau[j] = t;
+      }
+      __syncwarp();
+      double v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[i] = row0 + 8 * i == j ? 1.0 : x[i] * scale;
+#pragma unroll
+      for (int s = 0; s < 8; ++s) {
+        const double wv = coef[warp][4 * s + cg];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) a[i][s] = fma(-v[i], wv, a[i][s]);
+      }
+      if (cg == cj) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int row = row0 + 8 * i;
+          if (row < w)
+            D.R[row + (long long)j * D.ldr] = row < j ? a[i][0] : row == j ? beta : 0.0;
+          a[i][0] = v[i];
+        }
+      }
+    } else {
+      // no reflector: a column past the rows (its R entries are final) or
+      // past the panel (zero)
+      if (cg == cj) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int row = row0 + 8 * i;
+          if (j < w && row < w) D.R[row + (long long)j * D.ldr] = row < k ? a[i][0] : 0.0;
+          a[i][0] = 0.0;
+        }
+      }
+      if (warp == 0) {
+        if (lane < j) G[j * kLdG + lane] = 0.0;
+        if (lane == 0) tau[j] = 0.0;
+      }
+    }
+    if (cj == 3) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const double first = a[i][0];
+#pragma unroll
+        for (int s = 0; s < 7; ++s) a[i][s] = a[i][s + 1];
+        a[i][7] = first;
+      }
+    }
+  }
+
+  // M = T V_1^T by back substitution, a lane per column, in two halves of 16
+  // rows held in registers (warp 0 owns the first 32 rows and wrote G, tau)
+  if (warp == 0) {
+#pragma unroll
+    for (int s = 0; s < 8; ++s)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) M[(4 * s + cg) * kLdM + rg + 8 * i] = a[i][s];
+    __syncwarp();
+#pragma unroll
+    for (int h = 1; h >= 0; --h) {
+      double m[16];
+#pragma unroll
+      for (int l = 0; l < 16; ++l) m[l] = M[(16 * h + l) * kLdM + lane];
+      if (h == 0)
+        for (int j = 16; j < 32; ++j) {
+          const double mj = M[j * kLdM + lane];
+#pragma unroll
+          for (int l = 0; l < 16; ++l) m[l] = fma(-G[j * kLdG + l], mj, m[l]);
+        }
+#pragma unroll
+      for (int j = 15; j >= 0; --j) {
+        m[j] *= tau[16 * h + j];
+#pragma unroll
+        for (int l = 0; l < j; ++l)
+          m[l] = fma(-G[(16 * h + j) * kLdG + 16 * h + l], m[j], m[l]);
+      }
+#pragma unroll
+      for (int l = 0; l < 16; ++l) M[(16 * h + l) * kLdM + lane] = m[l];
+    }
   }
   __syncthreads();
-
-  for (int j = 0; j < k; ++j) {
-    double part = 0.0;
-    for (int i = j + 1 + tid; i < r; i += kQT) part = fma(S[i + j * kChunk], S[i + j * kChunk], part);
-    const double sigma2 = block_sum(part, red);
-    const double x0 = S[j + j * kChunk];
-    double beta = x0, t = 0.0, scale = 0.0;
-    if (sigma2 > 0.0) {
-      const double nrm = sqrt(fma(x0, x0, sigma2));
-      beta = x0 >= 0.0 ? -nrm : nrm;
-      t = (beta - x0) / beta;
-      scale = 1.0 / (x0 - beta);
+  // Q = [I; 0] - V M (M upper triangular)
+#pragma unroll
+  for (int nt = 0; nt < 4; ++nt) {
+    double q[4][2] = {};
+#pragma unroll
+    for (int s = 0; s < 2 * nt + 2; ++s) {
+      const double b = M[(4 * s + cg) * kLdM + 8 * nt + rg];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) dmma884(q[i], a[i][s], b);
     }
-    __syncthreads();
-    for (int i = j + 1 + tid; i < r; i += kQT) S[i + j * kChunk] *= scale;
-    if (tid == 0) {
-      S[j + j * kChunk] = beta;
-      tau[j] = t;
-    }
-    __syncthreads();
-    for (int c = j + 1 + warp; c < w; c += kQT / 32) {
-      double dot = lane == 0 ? S[j + c * kChunk] : 0.0;
-      for (int i = j + 1 + lane; i < r; i += 32) dot = fma(S[i + j * kChunk], S[i + c * kChunk], dot);
-      dot = warp_sum(dot);
-      if (lane == 0) wv[c] = dot * t;
-    }
-    __syncthreads();
-    // trailing update, one thread per row (no index division)
-    if (tid >= j && tid < r) {
-      const double vi = (tid == j) ? 1.0 : S[tid + j * kChunk];
-      for (int c = j + 1; c < w; ++c) S[tid + c * kChunk] -= vi * wv[c];
-    }
-    __syncthreads();
-  }
-
-  // R (w x w): upper triangle of the first k rows
-  for (int e = tid; e < w * w; e += kQT) {
-    const int i = e % w, c = e / w;
-    D.R[i + (long long)c * D.ldr] = (i <= c && i < k) ? S[i + c * kChunk] : 0.0;
-  }
-  // explicit Q = H_0 ... H_{k-1} [I; 0]
-  for (int e = tid; e < kChunk * kPanel; e += kQT) {
-    const int i = e % kChunk, c = e / kChunk;
-    E[e] = (i == c && i < r && c < w) ? 1.0 : 0.0;
-  }
-  __syncthreads();
-  for (int j = k - 1; j >= 0; --j) {
-    const double t = tau[j];
-    for (int c = j + warp; c < w; c += kQT / 32) {
-      double dot = lane == 0 ? E[j + c * kChunk] : 0.0;
-      for (int i = j + 1 + lane; i < r; i += 32) dot = fma(S[i + j * kChunk], E[i + c * kChunk], dot);
-      dot = warp_sum(dot);
-      if (lane == 0) wv[c] = dot * t;
-    }
-    __syncthreads();
-    if (tid >= j && tid < r) {
-      const double vi = (tid == j) ? 1.0 : S[tid + j * kChunk];
-      for (int c = j; c < w; ++c) E[tid + c * kChunk] -= vi * wv[c];
-    }
-    __syncthreads();
-  }
-  for (int e = tid; e < r * w; e += kQT) {
-    const int i = e % r, c = e / r;
-    D.A[i + (long long)c * D.lda] = E[i + c * kChunk];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int row = row0 + 8 * i, c = 8 * nt + 2 * cg + h;
+        if (row < r && c < w)
+          D.A[row + (long long)c * D.lda] = (row == c ? 1.0 : 0.0) - q[i][h];
+      }
   }
 }
 
@@ -359,16 +457,10 @@ std::unique_ptr<TsqrPlan, TsqrPlanDeleter> tsqr_plan(const std::vector<TsqrProb>
 }
 
 void tsqr_run(const TsqrPlan &plan, cudaStream_t s) {
-  static bool configured = false;
-  if (!configured) {
-    HB_CUDA(cudaFuncSetAttribute(qr_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kQrSmem));
-    configured = true;
-  }
   for (size_t l = 0; l < plan.up.size(); ++l)
     for (int off = 0; off < plan.up_n[l]; off += 65535) {
       const int cnt = std::min(65535, plan.up_n[l] - off);
-      qr_chunk_kernel<<<cnt, kQT, kQrSmem, s>>>(plan.up[l] + off);
+      qr_chunk_kernel<<<cnt, kQT, 0, s>>>(plan.up[l] + off);
       HB_LAUNCHED();
     }
   for (size_t l = 0; l < plan.down.size(); ++l)
