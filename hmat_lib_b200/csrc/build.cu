@@ -199,15 +199,13 @@ std::vector<float> block_features(const std::vector<SketchBlock> &sk,
   JacobiParams prm;
   prm.trunc = Truncation::None;
   prm.max_sweeps = 30;
-  JacobiProb *d_jp = upload_vec(jp, stream);
-  jacobi_svd_batched(d_jp, nsk, prm, d_rank + nsk, F, stream);
+  jacobi_svd_batched(jp, prm, d_rank + nsk, stream);
   std::vector<double> sig((size_t)nsk * F);
   {
     std::vector<CopyDesc> gd;
     for (int i = 0; i < nsk; ++i) gd.push_back(CopyDesc{w + sg[i], F, nullptr, 0, F, 1});
     gather_to_host(gd, F, sig.data(), stream);
   }
-  cudaFreeAsync(d_jp, stream);
   cudaFreeAsync(d_rank, stream);
   dev_free(w, stream);
   // kernel length scale: option kernel_length, else (matrix-free build) the
@@ -300,7 +298,6 @@ std::vector<std::shared_ptr<DeviceTree>> build_attempt(
   };
   struct ExactSlot { long long ws, u, v, sig; };
   std::vector<ExactSlot> eslots;
-  int max_c = 0;
   for (int b : exact) {
     const BlockDesc &B = blk[b].B;
     const int C = std::min(B.m, B.n);
@@ -310,7 +307,6 @@ std::vector<std::shared_ptr<DeviceTree>> build_attempt(
     s.v = take((long long)B.n * C);
     s.sig = take(C);
     eslots.push_back(s);
-    max_c = std::max(max_c, C);
   }
   // Option build_precision = 1 (dense input only): the sketch products
   // Y = A Omega and B^T = A^T Q on the int8 tensor cores, every block sliced
@@ -552,11 +548,7 @@ std::vector<std::shared_ptr<DeviceTree>> build_attempt(
     jp.sweeps = d_sweeps + p;
     eprobs.push_back(jp);
   }
-  JacobiProb *d_eprobs = nullptr;
-  if (!eprobs.empty()) {
-    d_eprobs = upload_vec(eprobs, stream);
-    jacobi_svd_batched(d_eprobs, (int)eprobs.size(), prm, d_status, max_c, stream, gspec);
-  }
+  jacobi_svd_batched(eprobs, prm, d_status, stream, gspec);
 
   HB_CUDA(cudaEventRecord(ev[1], stream));
 
@@ -806,12 +798,10 @@ std::vector<std::shared_ptr<DeviceTree>> build_attempt(
   const int bj_min = (int)option("jacobi_block_min_c", 128);
   std::vector<JacobiProb> sprobs;
   std::vector<long long> s_u(sk.size()), s_v(sk.size());
-  int max_l = 0;
   long long jscratch = 0;
   for (size_t i = 0; i < sk.size(); ++i) {
     const int L = sk[i].ell;
     const bool big = L >= bj_min;
-    if (!big) max_l = std::max(max_l, L);
     jscratch += (big ? 0 : jacobi_workspace(L, L)) + 2 * align_up((long long)L * L) + align_up(L);
   }
   double *jwork = sk.empty() ? nullptr : dev_alloc(jscratch, stream);
@@ -848,7 +838,6 @@ std::vector<std::shared_ptr<DeviceTree>> build_attempt(
       sprobs.push_back(jp);
     }
   }
-  JacobiProb *d_sprobs = nullptr;
   {
     std::vector<JacobiProb> small;
     std::vector<BjProb> big;
@@ -859,10 +848,7 @@ std::vector<std::shared_ptr<DeviceTree>> build_attempt(
       else
         small.push_back(jp);
     }
-    if (!small.empty()) {
-      d_sprobs = upload_vec(small, stream);
-      jacobi_svd_batched(d_sprobs, (int)small.size(), prm, d_status, max_l, stream);
-    }
+    jacobi_svd_batched(small, prm, d_status, stream);
     if (!big.empty()) block_jacobi_svd(big, tol, prm.max_sweeps, d_status, stream);
   }
   HB_CUDA(cudaEventRecord(ev[3], stream));
@@ -962,8 +948,6 @@ std::vector<std::shared_ptr<DeviceTree>> build_attempt(
   float stage_ms[4] = {0.f, 0.f, 0.f, 0.f};
   for (int i = 0; i < 4; ++i) cudaEventElapsedTime(&stage_ms[i], ev[i], ev[i + 1]);
   for (auto &e : ev) cudaEventDestroy(e);
-  dev_free(d_eprobs, stream);
-  dev_free(d_sprobs, stream);
   dev_free(d_int, stream);
   dev_free(jwork, stream);
   dev_free(work, stream);

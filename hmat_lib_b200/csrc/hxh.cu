@@ -117,11 +117,9 @@ struct RecompJob {
   bool active() const { return std::min(m, n) > 0 && S > 0; }
 };
 
-// Workspace of every job (`take(e)` returns the offset of e doubles);
-// returns the widest Jacobi problem.
+// Workspace of every job (`take(e)` returns the offset of e doubles).
 template <class Take>
-int recomp_layout(std::vector<RecompJob> &jobs, Take take) {
-  int max_c = 1;
+void recomp_layout(std::vector<RecompJob> &jobs, Take take) {
   for (RecompJob &j : jobs) {
     const int mn = std::min(j.m, j.n);
     if (mn == 0) continue;
@@ -132,7 +130,6 @@ int recomp_layout(std::vector<RecompJob> &jobs, Take take) {
       j.jo_u = take((long long)j.m * mn);
       j.jo_v = take((long long)j.n * mn);
       j.jsig = take(mn);
-      max_c = std::max(max_c, mn);
     } else {
       j.ru = take((long long)Sb * Sb);
       j.rv = take((long long)Sb * Sb);
@@ -142,17 +139,15 @@ int recomp_layout(std::vector<RecompJob> &jobs, Take take) {
       j.jo_u = take((long long)Sb * Sb);
       j.jo_v = take((long long)Sb * Sb);
       j.jsig = take(Sb);
-      max_c = std::max(max_c, Sb);
     }
   }
-  return max_c;
 }
 
 // Runs the QRs, the dense products and the Jacobi SVDs of every job (the R
 // blocks of the workspace must be zero); returns each job's rank (0 for
 // inactive jobs) and the Jacobi status in *status.  Synchronises.
 std::vector<int> recomp_run(const std::vector<RecompJob> &jobs, double *work, double tol,
-                            int max_c, cudaStream_t s, int *status) {
+                            cudaStream_t s, int *status) {
   GemmBases gb{};
   for (int i = 0; i < kGemmBases; ++i) gb.p[i] = work;
   const int nj = (int)jobs.size();
@@ -221,9 +216,7 @@ std::vector<int> recomp_run(const std::vector<RecompJob> &jobs, double *work, do
     prm.trunc = Truncation::Absolute;
     prm.scale_u = 1;
     prm.max_sweeps = (int)option("jacobi_max_sweeps", 60);
-    JacobiProb *d_jp = upload_vec(jp, s);
-    jacobi_svd_batched(d_jp, (int)jp.size(), prm, d_int + nj, max_c, s);
-    cudaFreeAsync(d_jp, s);
+    jacobi_svd_batched(jp, prm, d_int + nj, s);
   }
   std::vector<int> ints(nj + 1, 0);
   HB_CUDA(cudaMemcpyAsync(ints.data(), d_int, sizeof(int) * (nj + 1), cudaMemcpyDeviceToHost, s));
@@ -353,7 +346,7 @@ std::shared_ptr<DeviceTree> hxh_multiply(DeviceTree &A, DeviceTree &B, double to
     const int mn = std::min(o.m, o.n);
     j.dense = mn > 0 && S[b] >= mn && mn <= dense_max;
   }
-  const int max_c = recomp_layout(jobs, take);
+  recomp_layout(jobs, take);
   // diagonal leaves: products and ancestor intermediates T = U_A[rows] core
   std::vector<long long> leaf_out(nleaf), tmat;
   std::vector<std::vector<std::pair<int, long long>>> leaf_terms(nleaf);
@@ -459,7 +452,7 @@ std::shared_ptr<DeviceTree> hxh_multiply(DeviceTree &A, DeviceTree &B, double to
   }
 
   // ---- 4. recompression ----------------------------------------------------------------
-  const std::vector<int> ranks = recomp_run(jobs, work, tol, max_c, s, status);
+  const std::vector<int> ranks = recomp_run(jobs, work, tol, s, status);
 
   // ---- 5. diagonal leaves ----------------------------------------------------------------
   {
@@ -534,7 +527,7 @@ int recompress_one(int m, int n, int S, const double *d_u, int ldu, const double
   j.dense = dense;
   j.u = take((long long)m * S);
   j.v = take((long long)n * S);
-  const int max_c = recomp_layout(jobs, take);
+  recomp_layout(jobs, take);
   const int cap = std::max(S, std::min(m, n));
   const long long uo = take((long long)m * cap), vo = take((long long)n * cap);
   double *work = dev_alloc(ws, s);
@@ -544,7 +537,7 @@ int recompress_one(int m, int n, int S, const double *d_u, int ldu, const double
   HB_CUDA(cudaMemcpy2DAsync(work + j.v, sizeof(double) * n, d_v, sizeof(double) * ldv,
                             sizeof(double) * n, S, cudaMemcpyDeviceToDevice, s));
   int status = SUCCESS;
-  const std::vector<int> ranks = recomp_run(jobs, work, tol, max_c, s, &status);
+  const std::vector<int> ranks = recomp_run(jobs, work, tol, s, &status);
   recomp_finish(jobs, ranks, work, work, {uo}, {vo}, s);
   *rank = ranks[0];
   if (ranks[0] > 0) {

@@ -17,9 +17,9 @@ struct JacobiProb {
   int m, n;
   double *G;        // workspace R x C
   double *W;        // workspace C x C
-  double *U;        // out: m x C, ld ldu (left vectors, times sigma if scale_u)
-  long long ldu;
-  double *V;        // out: n x C, ld ldv (right vectors)
+  double *U;        // out: m x rank, ld ldu (left vectors, times sigma if scale_u);
+  long long ldu;    //   room for C columns
+  double *V;        // out: n x rank, ld ldv (right vectors); room for C columns
   long long ldv;
   double *sigma;    // out: C singular values, descending
   int *rank;        // out: truncation rank (>= 1 unless the block is empty)
@@ -58,9 +58,10 @@ inline long long jacobi_workspace(int m, int n) {
 }
 
 // status: device int, set to SVD_FAILURE by any problem that did not
-// converge within max_sweeps (left untouched otherwise).
-void jacobi_svd_batched(const JacobiProb *d_probs, int nprobs, const JacobiParams &prm,
-                        int *d_status, int max_c, cudaStream_t stream,
+// converge within max_sweeps (left untouched otherwise).  The descriptors are
+// uploaded stream-ordered.
+void jacobi_svd_batched(const std::vector<JacobiProb> &probs, const JacobiParams &prm,
+                        int *d_status, cudaStream_t stream,
                         const KernelSpec &gen = KernelSpec());
 
 struct CopyDesc {
