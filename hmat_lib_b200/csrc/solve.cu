@@ -8,108 +8,329 @@
 #include <algorithm>
 #include <cmath>
 
+#include <cooperative_groups.h>
+
+#include "dmma.cuh"
 #include "gemm_f64.h"
 #include "jacobi.h"
 #include "solve.h"
+
+namespace cg = cooperative_groups;
 
 namespace hb {
 
 namespace {
 
-constexpr int kGjThreads = 256;
+constexpr int kGjThreads = 512;
+constexpr int kGjWarps = kGjThreads / 32;
+constexpr int kGjB = 32;             // columns per panel, columns per update strip
+constexpr int kGjMaxCluster = 8;
+constexpr size_t kGjSmem = 200 * 1024;
+constexpr int kGjMaxN = 25600;       // row numbers are kept as short
 
 struct GjProb {
   const double *A;   // n x n input (ld lda)
   long long lda;
   int n;
-  double *work;      // n x 2n scratch, ld n
+  double *work;      // n x n scratch, ld n
   double *inv;       // n x n output (ld ldi)
   long long ldi;
+  int2 *moves;       // 2 kGjB row moves (to, from) of the current panel
+  int *flag;         // set when a pivot is at rounding level
 };
 
-// Gauss-Jordan inversion with partial pivoting, one CTA per matrix, on the
-// augmented [A | I] in global memory.  A pivot at rounding level relative to
-// the matrix's largest entry sets *status (the output is then not used).
-__global__ void __launch_bounds__(kGjThreads)
-gj_inverse_kernel(const GjProb *__restrict__ probs, int *status) {
-  const GjProb P = probs[blockIdx.x];
-  const int n = P.n, tid = threadIdx.x;
-  extern __shared__ double f[];              // n: the pivot column before elimination
-  __shared__ double s_val[kGjThreads];
-  __shared__ int s_idx[kGjThreads];
-  __shared__ int s_stop;
+// Leading dimension of the panel in shared memory: 4 mod 16, so that eight
+// rows by four columns hit every bank once.
+__host__ __device__ inline int gj_ldp(int n) { return (n + 15) / 16 * 16 + 4; }
+// Shared memory beside the panel: the pivot rows of a strip, row numbers.
+__host__ __device__ inline size_t gj_base_smem(int n) {
+  return sizeof(double) * kGjB * (kGjB + 4) + 2 * sizeof(short) * ((size_t)n + 8);
+}
+inline size_t gj_panel_smem(int n) { return sizeof(double) * kGjB * (size_t)gj_ldp(n); }
+
+// In-place blocked Gauss-Jordan inversion with partial pivoting, a cluster of
+// CTAs per matrix.  Per panel of 32 columns:
+//   1. rank 0 runs the 32 elimination steps on the panel alone, in shared
+//      memory, pivots searched over all rows not yet used; what is left in
+//      the panel is the matrix T whose product with the pivot rows is the
+//      steps' effect on any other column;
+//   2. every CTA takes its share of the 32-column strips: rows moved as the
+//      panel's swaps moved them, then W <- W + T W[pivot rows] (pivot rows:
+//      T W[pivot rows]) on the FP64 tensor cores.
+// The matrix ends as the inverse of the row-permuted input, whose columns go
+// to their places in the output.  The steps are a chain of n pivot searches,
+// each two barriers and a pass over n x 32 values in shared memory; the rest
+// is 2 n^3 flops on up to eight SMs.  W is written and read by the CTAs of the
+// cluster in turn, ordered by the cluster barrier, and read past L1.  A panel
+// taller than shared memory stays in global memory (ld n).  A pivot at rounding level relative to the matrix's
+// largest entry sets *status (the output is then not used).
+// All inverses of an n = 16384 factorisation (128 leaves of 128 rows, Schur
+// complements of 60 to 280 rows): 88 ms with one CTA per matrix eliminating
+// column by column in global memory, 2.5 ms so.
+template <bool kShared>
+__device__ void gj_invert(const GjProb &P, int *status, double *sm, int crank, int ncl) {
+  cg::cluster_group cl = cg::this_cluster();
+  const int n = P.n, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int gq = lane >> 2, tq = lane & 3;
+  __shared__ double s_val[kGjWarps];
+  __shared__ double s_amax;
+  __shared__ unsigned s_hi[2][kGjWarps], s_lo[2][kGjWarps];
+  __shared__ int s_idx[2][kGjWarps], s_piv[kGjB], s_fail;
+  double *Bs = sm;                                       // [k][column], ld kGjB + 4
+  short *perm = reinterpret_cast<short *>(sm + kGjB * (kGjB + 4));   // rows of A by place
+  short *src = perm + n + 8;                             // this panel's row moves
+  double *Ps = reinterpret_cast<double *>(reinterpret_cast<char *>(sm) +
+                                          (gj_base_smem(n) + 15) / 16 * 16);
+  constexpr int LDB = kGjB + 4;
   double *W = P.work;
+  const long long ldp = kShared ? gj_ldp(n) : n;
+  const int nstrip = (n + kGjB - 1) / kGjB, ntile = (n + 7) / 8;
+
+  // ---- copy, largest entry -----------------------------------------------------------
   double amax = 0.0;
-  for (long long e = tid; e < (long long)n * n; e += blockDim.x) {
-    const int r = (int)(e % n), c = (int)(e / n);
-    const double a = P.A[r + (long long)c * P.lda];
-    W[e] = a;
-    W[(long long)n * n + e] = (r == c) ? 1.0 : 0.0;
-    amax = fmax(amax, fabs(a));
-  }
-  s_val[tid] = amax;
-  if (tid == 0) s_stop = 0;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (tid < o) s_val[tid] = fmax(s_val[tid], s_val[tid + o]);
-    __syncthreads();
-  }
-  const double tiny = fmax(64.0 * 2.220446049250313e-16 * s_val[0], 1e-300);
-  __syncthreads();
-  for (int k = 0; k < n; ++k) {
-    // pivot: largest |W[r, k]|, r >= k
-    double best = -1.0;
-    int bi = k;
-    for (int r = k + tid; r < n; r += blockDim.x) {
-      const double v = fabs(W[r + (long long)k * n]);
-      if (v > best) {
-        best = v;
-        bi = r;
+  for (int st = crank; st < nstrip; st += ncl)
+    for (int c = st * kGjB + warp; c < min(n, (st + 1) * kGjB); c += kGjWarps)
+      for (int r = lane; r < n; r += 32) {
+        const double a = P.A[r + (long long)c * P.lda];
+        W[r + (long long)c * n] = a;
+        amax = fmax(amax, fabs(a));
       }
-    }
-    s_val[tid] = best;
-    s_idx[tid] = bi;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-      if (tid < o && (s_val[tid + o] > s_val[tid] ||
-                      (s_val[tid + o] == s_val[tid] && s_idx[tid + o] < s_idx[tid]))) {
-        s_val[tid] = s_val[tid + o];
-        s_idx[tid] = s_idx[tid + o];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  if (lane == 0) s_val[warp] = amax;
+  for (int r = tid; r < n; r += kGjThreads) perm[r] = (short)r;
+  __syncthreads();
+  if (tid == 0) {
+    for (int w = 0; w < kGjWarps; ++w) amax = fmax(amax, s_val[w]);
+    s_amax = amax;
+    s_fail = 0;
+  }
+  cl.sync();
+  amax = 0.0;
+  for (int rk = 0; rk < ncl; ++rk) amax = fmax(amax, *cl.map_shared_rank(&s_amax, rk));
+  const double tiny = fmax(64.0 * 2.220446049250313e-16 * amax, 1e-300);
+  cl.sync();
+
+  for (int K0 = 0; K0 < n; K0 += kGjB) {
+    const int b = min(kGjB, n - K0);
+    double *Pp = kShared ? Ps : W + (long long)K0 * n;
+    auto pl = [](const double *q) { return kShared ? *q : __ldcg(q); };
+    // ---- 1. the panel ------------------------------------------------------------------
+    if (crank == 0) {
+      if (kShared)
+        for (int c = warp; c < kGjB; c += kGjWarps)
+          for (int r = lane; r < 8 * ntile; r += 32)
+            Pp[r + c * ldp] = (c < b && r < n) ? __ldcg(W + r + (long long)(K0 + c) * n) : 0.0;
+      for (int r = tid; r < n; r += kGjThreads) src[r] = (short)r;
+      __syncthreads();
+      double best = -1.0;
+      int bi = 0x7fffffff;
+      for (int r = K0 + tid; r < n; r += kGjThreads) {
+        const double v = fabs(pl(Pp + r));
+        if (v > best) {
+          best = v;
+          bi = r;
+        }
+      }
+      for (int kk = 0; kk < b; ++kk) {
+        const int k = K0 + kk, par = kk & 1;
+        // pivot: the largest magnitude, ties to the smallest row
+        auto reduce = [&](unsigned hi, unsigned lo, int id, unsigned &mh, unsigned &ml, int &mi) {
+          mh = __reduce_max_sync(0xffffffffu, hi);
+          ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+          mi = __reduce_min_sync(0xffffffffu, hi == mh && lo == ml ? id : 0x7fffffff);
+        };
+        unsigned hi = 0, lo = 0, mh, ml;
+        int mi;
+        if (best >= 0.0) {
+          hi = (unsigned)__double2hiint(best);
+          lo = (unsigned)__double2loint(best);
+        }
+        reduce(hi, lo, bi, mh, ml, mi);
+        if (lane == 0) {
+          s_hi[par][warp] = mh;
+          s_lo[par][warp] = ml;
+          s_idx[par][warp] = mi;
+        }
+        __syncthreads();
+        const bool in = lane < kGjWarps;
+        reduce(in ? s_hi[par][lane] : 0u, in ? s_lo[par][lane] : 0u,
+               in ? s_idx[par][lane] : 0x7fffffff, mh, ml, mi);
+        const double big = __hiloint2double((int)mh, (int)ml);
+        if (mi >= n || big <= tiny) {      // the same in every thread
+          if (tid == 0) s_fail = 1;
+          break;
+        }
+        const int p = mi;
+        // swap rows k and p, scale row k by 1 / pivot, which takes the pivot's place
+        if (tid < kGjB) {
+          const double inv = 1.0 / pl(Pp + p + kk * ldp);
+          __syncwarp();
+          if (tid < b) {
+            const double a = pl(Pp + k + tid * ldp), v = pl(Pp + p + tid * ldp);
+            Pp[p + tid * ldp] = a;
+            Pp[k + tid * ldp] = tid == kk ? inv : v * inv;
+          }
+        }
+        if (tid == kGjB) {
+          const short a = perm[k], v = src[k];
+          perm[k] = perm[p];
+          perm[p] = a;
+          src[k] = src[p];
+          src[p] = v;
+          s_piv[kk] = p;
+        }
+        __syncthreads();
+        // eliminate column kk from the other rows; a warp takes 8 rows, lane
+        // (gq, tq) columns 4 s + tq; the next column's pivot search on the way
+        const double inv = pl(Pp + k + kk * ldp);
+        double prow[kGjB / 4];
+#pragma unroll
+        for (int s = 0; s < kGjB / 4; ++s)
+          prow[s] = 4 * s + tq < b ? pl(Pp + k + (4 * s + tq) * ldp) : 0.0;
+        best = -1.0;
+        bi = 0x7fffffff;
+        for (int t = warp; t < ntile; t += kGjWarps) {
+          const int r = 8 * t + gq;
+          const bool live = r < n && r != k;
+          const double f = live ? pl(Pp + r + kk * ldp) : 0.0;
+          __syncwarp();                    // f is read before column kk is written
+          if (live) {
+#pragma unroll
+            for (int s = 0; s < kGjB / 4; ++s) {
+              const int c = 4 * s + tq;
+              if (c < b) {
+                const double a = c == kk ? -f * inv : fma(-f, prow[s], pl(Pp + r + c * ldp));
+                Pp[r + c * ldp] = a;
+                if (c == kk + 1 && r > k && fabs(a) > best) {
+                  best = fabs(a);
+                  bi = r;
+                }
+              }
+            }
+          }
+        }
       }
       __syncthreads();
-    }
-    const int p = s_idx[0];
-    if (s_val[0] <= tiny) {
-      if (tid == 0) {
-        s_stop = 1;
-        atomicExch(status, 1);
+      if (s_fail) {
+        if (tid == 0) *P.flag = 1;
+      } else {
+        if (kShared)
+          for (int c = warp; c < b; c += kGjWarps)
+            for (int r = lane; r < n; r += 32) W[r + (long long)(K0 + c) * n] = Pp[r + c * ldp];
+        for (int i = tid; i < 2 * kGjB; i += kGjThreads) {
+          int2 mv = make_int2(-1, -1);
+          if (i < b) {
+            mv = make_int2(K0 + i, src[K0 + i]);
+          } else if (i >= kGjB && i - kGjB < b) {
+            const int q = s_piv[i - kGjB];   // a row may appear twice: the same move
+            if (q >= K0 + b) mv = make_int2(q, src[q]);
+          }
+          P.moves[i] = mv;
+        }
       }
     }
-    __syncthreads();
-    if (s_stop) break;
-    // swap rows k and p, scale row k
-    const double inv = 1.0 / W[p + (long long)k * n];
-    for (int c = tid; c < 2 * n; c += blockDim.x) {
-      const double a = W[k + (long long)c * n], b = W[p + (long long)c * n];
-      W[p + (long long)c * n] = a;
-      W[k + (long long)c * n] = b * inv;
+    cl.sync();
+    if (*(volatile int *)P.flag) {
+      if (crank == 0 && tid == 0) atomicExch(status, 1);
+      return;                              // the whole cluster
+    }
+    // ---- 2. the other columns ------------------------------------------------------------
+    if (kShared && crank != 0) {
+      for (int c = warp; c < kGjB; c += kGjWarps)
+        for (int r = lane; r < 8 * ntile; r += 32)
+          Ps[r + c * ldp] = (c < b && r < n) ? __ldcg(W + r + (long long)(K0 + c) * n) : 0.0;
     }
     __syncthreads();
-    for (int r = tid; r < n; r += blockDim.x) f[r] = W[r + (long long)k * n];
-    __syncthreads();
-    // eliminate column k from every other row (columns < k of row k are 0)
-    const long long cols = 2LL * n - k;
-    for (long long e = tid; e < (long long)n * cols; e += blockDim.x) {
-      const int r = (int)(e % n);
-      const long long c = k + e / n;
-      if (r != k) W[r + c * n] -= f[r] * W[k + c * n];
+    for (int st = crank; st < nstrip; st += ncl) {
+      if (st == K0 / kGjB) continue;
+      const int c0 = st * kGjB, nc = min(kGjB, n - c0);
+      // move rows; the pivot rows go to shared memory ([k][column])
+      {
+        const int c = tid >> 4, i0 = tid & 15;
+        double v[4];
+        int to[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int2 mv = P.moves[i0 + 16 * u];
+          to[u] = c < nc ? mv.x : -1;
+          v[u] = to[u] >= 0 ? __ldcg(W + mv.y + (long long)(c0 + c) * n) : 0.0;
+        }
+        __syncthreads();                   // every old value read; Bs free
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          if (u < 2) Bs[(i0 + 16 * u) * LDB + c] = v[u];   // moves 0 .. 31: pivot rows
+          else if (to[u] >= 0) W[to[u] + (long long)(c0 + c) * n] = v[u];
+        }
+        __syncthreads();
+      }
+      // W += T Bs, a warp per 32 rows
+      for (int t = warp; t < nstrip; t += kGjWarps) {
+        const bool piv_rows = t == K0 / kGjB;
+        double acc[4][4][2];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int jn = 0; jn < 4; ++jn)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const int r = 32 * t + 8 * i + gq, c = 8 * jn + 2 * tq + h;
+              acc[i][jn][h] =
+                  (!piv_rows && r < n && c < nc) ? __ldcg(W + r + (long long)(c0 + c) * n) : 0.0;
+            }
+#pragma unroll
+        for (int s = 0; s < kGjB / 4; ++s) {
+          double a[4], bb[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int r = 32 * t + 8 * i + gq, kx = 4 * s + tq;
+            if (kShared)
+              a[i] = 4 * t + i < ntile ? Ps[r + kx * ldp] : 0.0;
+            else
+              a[i] = (r < n && kx < b) ? __ldcg(W + r + (long long)(K0 + kx) * n) : 0.0;
+          }
+#pragma unroll
+          for (int jn = 0; jn < 4; ++jn) bb[jn] = Bs[(4 * s + tq) * LDB + 8 * jn + gq];
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int jn = 0; jn < 4; ++jn) dmma884(acc[i][jn], a[i], bb[jn]);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int jn = 0; jn < 4; ++jn)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const int r = 32 * t + 8 * i + gq, c = 8 * jn + 2 * tq + h;
+              if (r < n && c < nc) W[r + (long long)(c0 + c) * n] = acc[i][jn][h];
+            }
+      }
     }
-    __syncthreads();
+    cl.sync();
   }
-  for (long long e = tid; e < (long long)n * n; e += blockDim.x) {
-    const int r = (int)(e % n), c = (int)(e / n);
-    P.inv[r + (long long)c * P.ldi] = W[(long long)n * n + e];
-  }
+
+  // ---- columns to their places: inv[:, perm[c]] = W[:, c] --------------------------------
+  const short *pm = cl.map_shared_rank(perm, 0);
+  for (int st = crank; st < nstrip; st += ncl)
+    for (int c = st * kGjB + warp; c < min(n, (st + 1) * kGjB); c += kGjWarps) {
+      const long long to = pm[c];
+      for (int r = lane; r < n; r += 32) P.inv[r + to * P.ldi] = __ldcg(W + r + (long long)c * n);
+    }
+  cl.sync();                               // rank 0's shared memory is read until here
+}
+
+__global__ void __launch_bounds__(kGjThreads, 1)
+gj_inverse_kernel(const GjProb *__restrict__ probs, int *status, int smem_bytes) {
+  extern __shared__ __align__(16) double gj_sm[];
+  cg::cluster_group cl = cg::this_cluster();
+  const int ncl = (int)cl.num_blocks(), crank = (int)cl.block_rank();
+  const GjProb P = probs[blockIdx.x / ncl];
+  if ((gj_base_smem(P.n) + 15) / 16 * 16 + sizeof(double) * kGjB * gj_ldp(P.n) <=
+      (size_t)smem_bytes)
+    gj_invert<true>(P, status, gj_sm, crank, ncl);
+  else
+    gj_invert<false>(P, status, gj_sm, crank, ncl);
 }
 
 struct EyeDesc {
@@ -138,25 +359,48 @@ T *upload_tmp(const std::vector<T> &v, cudaStream_t s) {
 
 void gj_inverse(std::vector<GjProb> probs, int *d_status, cudaStream_t s) {
   if (probs.empty()) return;
-  int nmax = 0;
+  const int np = (int)probs.size();
   long long work = 0;
+  size_t smem = 0;
   for (auto &p : probs) {
-    nmax = std::max(nmax, p.n);
-    work += align_up(2LL * p.n * p.n);
+    HB_REQUIRE(p.n <= kGjMaxN, INPUT_ERROR, "solve: capacitance matrix too large");
+    work += align_up((long long)p.n * p.n);
+    const size_t base = (gj_base_smem(p.n) + 15) / 16 * 16, all = base + gj_panel_smem(p.n);
+    smem = std::max(smem, all <= kGjSmem ? all : base);
   }
-  double *w = dev_alloc(work, s);
+  // the matrices, then per matrix its row moves and its flag
+  const long long ints = (long long)np * (4 * kGjB + 1);
+  double *w = dev_alloc(work + (ints + 1) / 2, s);
+  int2 *moves = reinterpret_cast<int2 *>(w + work);
+  int *flags = reinterpret_cast<int *>(moves + (long long)np * 2 * kGjB);
+  HB_CUDA(cudaMemsetAsync(flags, 0, sizeof(int) * np, s));
   long long o = 0;
-  for (auto &p : probs) {
+  for (int i = 0; i < np; ++i) {
+    GjProb &p = probs[i];
     p.work = w + o;
-    o += align_up(2LL * p.n * p.n);
+    o += align_up((long long)p.n * p.n);
+    p.moves = moves + (long long)i * 2 * kGjB;
+    p.flag = flags + i;
   }
   GjProb *d = upload_tmp(probs, s);
-  const size_t smem = sizeof(double) * std::max(nmax, 1);
-  HB_REQUIRE(smem <= 200 * 1024, INPUT_ERROR, "solve: capacitance matrix too large");
-  if (smem > 48 * 1024)
-    HB_CUDA(cudaFuncSetAttribute(gj_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
-  gj_inverse_kernel<<<(int)probs.size(), kGjThreads, smem, s>>>(d, d_status);
+  HB_CUDA(cudaFuncSetAttribute(gj_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)kGjSmem));
+  // as many CTAs per matrix as keep one CTA per SM
+  int ncl = 1;
+  while (2 * ncl <= kGjMaxCluster && 2 * ncl * np <= num_sms()) ncl *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(np * ncl));
+  cfg.blockDim = dim3(kGjThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)ncl;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  HB_CUDA(cudaLaunchKernelEx(&cfg, gj_inverse_kernel, (const GjProb *)d, d_status, (int)smem));
   HB_LAUNCHED();
   cudaFreeAsync(d, s);
   dev_free(w, s);
@@ -381,7 +625,7 @@ std::unique_ptr<HodlrFactor> hodlr_factorize(std::shared_ptr<DeviceTree> tp, cud
       const LeafDesc &lf = t.leaves[i];
       if (lf.m == 0) continue;
       probs.push_back(GjProb{t.arena + lf.off, lf.m, lf.m, nullptr,
-                             f->buf + f->leaf_inv_off[i], lf.m});
+                             f->buf + f->leaf_inv_off[i], lf.m, nullptr, nullptr});
     }
     gj_inverse(probs, d_status, s);
   }
@@ -446,7 +690,7 @@ std::unique_ptr<HodlrFactor> hodlr_factorize(std::shared_ptr<DeviceTree> tp, cud
       p = gs.add(kS_T, s_off[j], s2, s2, s2, -1.0, 1.0);           // S = I - Q P
       gs.seg(p, kS_T, q_off[j], s2, 0, kS_T, p_off[j], s1, 0, s1);
       s_eye.push_back(EyeDesc{Ps + s_off[j], s2, s2});
-      inv.push_back(GjProb{Ps + s_off[j], s2, s2, nullptr, f->buf + br, q});   // S^-1 -> C^-1[bl, bl]
+      inv.push_back(GjProb{Ps + s_off[j], s2, s2, nullptr, f->buf + br, q, nullptr, nullptr});   // S^-1 -> C^-1[bl, bl]
       p = c1.add(kS_Buf, tr_off, q, s1, s2, -1.0);                 // C^-1[tr, bl] = -P S^-1
       c1.seg(p, kS_T, p_off[j], s1, 0, kS_Buf, br, q, 0, s2);
       p = c1.add(kS_Buf, bl_off, q, s2, s1, -1.0);                 // C^-1[bl, tr] = -S^-1 Q
