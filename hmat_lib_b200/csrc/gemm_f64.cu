@@ -253,7 +253,11 @@ gemm_f64_kernel(const GemmSeg *__restrict__ segs, const GemmProb *__restrict__ p
 // when the operand's offset and leading dimension (and, for K-contiguous
 // operands, the first K index) are even, else 8; elements past M, N or the K
 // range are zero-filled.  The ring is as deep as two CTAs per SM allow (2 to
-// 4 stages).
+// 4 stages).  Ranks and leaf sizes are rarely multiples of a tile, so at an
+// edge a warp issues only the 8 x 8 MMA tiles and the 4-deep K steps that hold
+// something, and a segment's pointers are kept in registers until it ends:
+// H X at n = 32768, k = 256 (ranks 38 to 349) 1637 -> 1512 us, H x H at
+// n = 16384 (many products of 5 to 40 columns) 3.44 -> 2.90 ms.
 template <int BM, int BN, int BK>
 struct MmaSmem {
   static constexpr int LDKM = BM + 4;      // [k][m] layout
@@ -273,6 +277,78 @@ __device__ __forceinline__ void cp_async16(void *smem, const void *gmem, int src
                "r"(src_bytes));
 }
 
+// One operand tile of ROWS lines (M or N side) x BK into stage memory, by
+// cp.async.  `src` is element (line 0, K index 0) of the stage; K-contiguous
+// operands go to [line][k], the others to [k][line].  Lines past `nlines` and
+// K values past `kin` are zero-filled.  A thread's copies differ by a constant
+// step in both memories, so a copy costs an addition, a comparison and the
+// copy itself.
+template <int ROWS, int BK>
+__device__ __forceinline__ void stage_operand(double *dst, const double *src, int ld, bool kcontig,
+                                              bool vec, int nlines, int kin) {
+  const int tid = threadIdx.x;
+  if (kcontig) {
+    constexpr int CH = BK / 2, LS = kThreads / CH;   // 16-byte chunks per line, lines per pass
+    const int l0 = tid / CH, k = 2 * (tid % CH);
+    const int nk = min(2, max(0, kin - k));
+    double *d = dst + l0 * (BK + 4) + k;
+    const double *q = src + (long long)l0 * ld + k;
+    const long long step = (long long)LS * ld;
+#pragma unroll
+    for (int i = 0; i < (ROWS + LS - 1) / LS; ++i) {
+      if (ROWS % LS != 0 && l0 + i * LS >= ROWS) break;
+      const int take = l0 + i * LS < nlines ? nk : 0;
+      const double *from = take > 0 ? q + i * step : src;
+      if (vec) {
+        cp_async16(d + i * LS * (BK + 4), from, 8 * take);
+      } else {
+        cp_async8(d + i * LS * (BK + 4), from, take > 0);
+        cp_async8(d + i * LS * (BK + 4) + 1, take > 1 ? from + 1 : src, take > 1);
+      }
+    }
+  } else {
+    constexpr int CH = ROWS / 2, KS = kThreads / CH;   // chunks per K value, K values per pass
+    const int line = 2 * (tid % CH), k0 = tid / CH;
+    const int nl = min(2, max(0, nlines - line));
+    double *d = dst + k0 * (ROWS + 4) + line;
+    const double *q = src + (long long)k0 * ld + line;
+    const long long step = (long long)KS * ld;
+#pragma unroll
+    for (int i = 0; i < BK / KS; ++i) {
+      const int take = k0 + i * KS < kin ? nl : 0;
+      const double *from = take > 0 ? q + i * step : src;
+      if (vec) {
+        cp_async16(d + i * KS * (ROWS + 4), from, 8 * take);
+      } else {
+        cp_async8(d + i * KS * (ROWS + 4), from, take > 0);
+        cp_async8(d + i * KS * (ROWS + 4) + 1, take > 1 ? from + 1 : src, take > 1);
+      }
+    }
+  }
+}
+
+// The same for a generated kernel matrix: (r, c) of the block at
+// gen_offset(row0, col0), computed entry by entry.
+template <int ROWS, int BK>
+__device__ __forceinline__ void stage_generated(double *dst, const KernelSpec &gen, long long off,
+                                                bool kcontig, int row0, int nlines, int kk,
+                                                int kin) {
+  const int gr0 = (int)(off >> 32), gc0 = (int)(off & 0xffffffffLL);
+  for (int e = threadIdx.x; e < ROWS * BK; e += kThreads) {
+    const int line = kcontig ? e / BK : e % ROWS, k = kcontig ? e % BK : e / ROWS;
+    double v = 0.0;
+    if (line < nlines && k < kin) {
+      const int r = kcontig ? kk + k : row0 + line;
+      const int c = kcontig ? row0 + line : kk + k;
+      v = kernel_entry(gen, gr0 + r, gc0 + c);
+    }
+    if (kcontig)
+      dst[line * (BK + 4) + k] = v;
+    else
+      dst[k * (ROWS + 4) + line] = v;
+  }
+}
+
 template <int BM, int BN, int WM, int WN, int BK>
 __global__ void __launch_bounds__(kThreads, 2)
 gemm_f64_mma_kernel(const GemmSeg *__restrict__ segs, const GemmProb *__restrict__ probs,
@@ -290,6 +366,10 @@ gemm_f64_mma_kernel(const GemmSeg *__restrict__ segs, const GemmProb *__restrict
   const int g = lane >> 2, t = lane & 3;
   const int wm0 = (warp / WARPS_N) * WM, wn0 = (warp % WARPS_N) * WN;
   const int seg_end = P.seg0 + P.nseg;
+  // 8-row and 8-column MMA tiles of this warp that lie inside the problem
+  const int mt_in = max(0, min(MT, (P.M - tile.m0 - wm0 + 7) / 8));
+  const int nt_in = max(0, min(NT, (P.N - tile.n0 - wn0 + 7) / 8));
+  const bool whole = mt_in == MT && nt_in == NT;
 
   double acc[MT][NT][2];
 #pragma unroll
@@ -320,106 +400,74 @@ gemm_f64_mma_kernel(const GemmSeg *__restrict__ segs, const GemmProb *__restrict
     }
   };
 
-  // One operand tile of `rows` lines (M or N side) x BK into stage memory.
-  // `kcontig`: K is the contiguous dimension in global memory (stored
-  // [line][k] in shared memory), otherwise lines are ([k][line]).  Element
-  // (line, k) of the tile is global (row0 + line, kk + k) of the operand,
-  // stored at base + off + r + c ld with (r, c) = (line, k), or (k, line) when
-  // kcontig; lines >= nlines and k >= kend are zero.
-  auto load_operand = [&](double *dst, bool gen, const double *base, long long off, long long ld,
-                          bool kcontig, int rows, int row0, int nlines, int kk, int kend) {
-    if (gen) {
-      // generated kernel-matrix entries: (r, c) of the block at gen_offset(row0, col0)
-      const int gr0 = (int)(off >> 32), gc0 = (int)(off & 0xffffffffLL);
-      for (int e = tid; e < rows * BK; e += kThreads) {
-        int line, k;
-        if (kcontig) {
-          line = e / BK;
-          k = e % BK;
-        } else {
-          k = e / rows;
-          line = e % rows;
-        }
-        const bool p = (row0 + line) < nlines && (kk + k) < kend;
-        double v = 0.0;
-        if (p) {
-          const int r = kcontig ? kk + k : row0 + line;
-          const int c = kcontig ? row0 + line : kk + k;
-          v = kernel_entry(bases.gen, gr0 + r, gc0 + c);
-        }
-        if (kcontig)
-          dst[line * SM::LDK + k] = v;
-        else
-          dst[k * (rows + 4) + line] = v;
-      }
-      return;
+  // the segment being loaded: operand pointers at (this tile's first line,
+  // K = 0), leading dimensions, and flags (1: A K-contiguous, 2: B, 4: A by
+  // 16-byte copies, 8: B, 16: A generated, 32: B)
+  const double *pa = nullptr, *pb = nullptr;
+  long long goff = 0;   // offset of the generated operand
+  int lda = 0, ldb = 0;
+  unsigned fl = 0;
+  auto open_segment = [&](const KIter &it) {
+    const GemmSeg S = segs[it.si];
+    // op(A) is M x K: ta = 0 stores (m, k) at m + k lda (lines contiguous),
+    // ta = 1 at k + m lda (K contiguous); op(B) is K x N: tb = 0 stores (k, n)
+    // at k + n ldb (K contiguous), tb = 1 at n + k ldb
+    const bool ka = S.ta == 1, kb = S.tb == 0;
+    const bool ga = S.abase == kGenSlot, gb = S.bbase == kGenSlot;
+    lda = (int)S.lda;
+    ldb = (int)S.ldb;
+    fl = (ka ? 1u : 0u) | (kb ? 2u : 0u) | (ga ? 16u : 0u) | (gb ? 32u : 0u);
+    goff = ga ? S.a_off : S.b_off;
+    // 16-byte copies need an even element offset from a 16-byte boundary:
+    // operand, leading dimension, and the first K index of a K-contiguous one
+    if (!ga) {
+      const double *base = base_ptr(bases, S.abase) + S.a_off;
+      if (((lda | (ka ? it.kk : 0)) & 1) == 0 && ((unsigned long long)base & 15) == 0) fl |= 4u;
+      pa = base + (ka ? (long long)tile.m0 * lda : tile.m0);
     }
-    // 16-byte copies need even element offsets: the operand's offset and
-    // leading dimension, and for K-contiguous operands the first K index
-    const bool vec = ((off | ld | (kcontig ? kk : 0)) & 1) == 0 &&
-                     (((unsigned long long)base) & 15) == 0;
-    if (kcontig) {
-      // per line BK contiguous K values: BK / 2 chunks of 16 bytes
-      constexpr int CH = BK / 2;
-      for (int e = tid; e < rows * CH; e += kThreads) {
-        const int line = e / CH, k = 2 * (e % CH);
-        const bool lok = (row0 + line) < nlines;
-        const int nk = lok ? min(2, max(0, kend - (kk + k))) : 0;
-        double *d = dst + line * SM::LDK + k;
-        const double *src = base + off + (long long)(row0 + line) * ld + (kk + k);
-        if (vec) {
-          cp_async16(d, nk > 0 ? src : base, 8 * nk);
-        } else {
-          cp_async8(d, nk > 0 ? src : base, nk > 0);
-          cp_async8(d + 1, nk > 1 ? src + 1 : base, nk > 1);
-        }
-      }
-    } else {
-      // per k, `rows` contiguous lines: rows / 2 chunks of 16 bytes
-      const int CH = rows / 2;
-      for (int e = tid; e < BK * CH; e += kThreads) {
-        const int k = e / CH, line = 2 * (e % CH);
-        const bool kok = (kk + k) < kend;
-        const int nl = kok ? min(2, max(0, nlines - (row0 + line))) : 0;
-        double *d = dst + k * (rows + 4) + line;
-        const double *src = base + off + (row0 + line) + (long long)(kk + k) * ld;
-        if (vec) {
-          cp_async16(d, nl > 0 ? src : base, 8 * nl);
-        } else {
-          cp_async8(d, nl > 0 ? src : base, nl > 0);
-          cp_async8(d + 1, nl > 1 ? src + 1 : base, nl > 1);
-        }
-      }
+    if (!gb) {
+      const double *base = base_ptr(bases, S.bbase) + S.b_off;
+      if (((ldb | (kb ? it.kk : 0)) & 1) == 0 && ((unsigned long long)base & 15) == 0) fl |= 8u;
+      pb = base + (kb ? (long long)tile.n0 * ldb : tile.n0);
     }
   };
 
   // Stage `buf` <- K-block `it`; returns its layout bits (1: A stored [m][k],
   // 2: B stored [n][k]).
-  auto load = [&](int buf, const KIter &it) -> int {
-    const GemmSeg S = segs[it.si];
-    const bool ga = S.abase == kGenSlot, gb = S.bbase == kGenSlot;
+  auto load = [&](int buf, const KIter &it) -> unsigned {
     double *as = smem + buf * SM::STAGE;
     double *bs = as + SM::A_ELEMS;
-    // op(A) is M x K: ta = 0 stores (m, k) at m + k lda (lines contiguous),
-    // ta = 1 stores it at k + m lda (K contiguous)
-    load_operand(as, ga, ga ? nullptr : base_ptr(bases, S.abase), S.a_off, S.lda, S.ta == 1, BM,
-                 tile.m0, P.M, it.kk, it.le);
-    // op(B) is K x N: tb = 0 stores (k, n) at k + n ldb (K contiguous),
-    // tb = 1 at n + k ldb (lines contiguous)
-    load_operand(bs, gb, gb ? nullptr : base_ptr(bases, S.bbase), S.b_off, S.ldb, S.tb == 0, BN,
-                 tile.n0, P.N, it.kk, it.le);
-    return (S.ta == 1 ? 1 : 0) | (S.tb == 0 ? 2 : 0);
+    const int kin = min(BK, it.le - it.kk);
+    const bool ka = fl & 1u, kb = fl & 2u;
+    if (fl & 16u)
+      stage_generated<BM, BK>(as, bases.gen, goff, ka, tile.m0, P.M - tile.m0, it.kk, kin);
+    else
+      stage_operand<BM, BK>(as, pa + (ka ? (long long)it.kk : (long long)it.kk * lda), lda, ka,
+                            fl & 4u, P.M - tile.m0, kin);
+    if (fl & 32u)
+      stage_generated<BN, BK>(bs, bases.gen, goff, kb, tile.n0, P.N - tile.n0, it.kk, kin);
+    else
+      stage_operand<BN, BK>(bs, pb + (kb ? (long long)it.kk : (long long)it.kk * ldb), ldb, kb,
+                            fl & 8u, P.N - tile.n0, kin);
+    return fl & 3u;
+  };
+  // the next K-block of the load side, opening its segment when it changes
+  auto advance_load = [&](KIter &it) {
+    const int si = it.si;
+    advance(it);
+    if (it.si != si && it.si < seg_end) open_segment(it);
   };
 
   // ring of kMmaStages buffers; `lay` keeps 2 layout bits per buffer
   KIter it{P.seg0, 0, 0, 0};
   settle(it);
+  if (it.si < seg_end) open_segment(it);
   unsigned lay = 0;
 #pragma unroll
   for (int st = 0; st < kMmaStages - 1; ++st) {
     if (it.si < seg_end) {
-      lay |= (unsigned)load(st, it) << (2 * st);
-      advance(it);
+      lay |= load(st, it) << (2 * st);
+      advance_load(it);
     }
     cp_async_commit();
   }
@@ -432,8 +480,8 @@ gemm_f64_mma_kernel(const GemmSeg *__restrict__ segs, const GemmProb *__restrict
     {
       const int nb = (buf + kMmaStages - 1) % kMmaStages;
       if (it.si < seg_end) {
-        lay = (lay & ~(3u << (2 * nb))) | ((unsigned)load(nb, it) << (2 * nb));
-        advance(it);
+        lay = (lay & ~(3u << (2 * nb))) | (load(nb, it) << (2 * nb));
+        advance_load(it);
       }
       cp_async_commit();
     }
@@ -447,17 +495,37 @@ gemm_f64_mma_kernel(const GemmSeg *__restrict__ segs, const GemmProb *__restrict
     const int b_k_step = (l & 2) ? 1 : SM::LDKN;
     const double *ap = as + (wm0 + g) * a_line_step + t * a_k_step;
     const double *bp = bs + (wn0 + g) * b_line_step + t * b_k_step;
+    const int kin = min(BK, cit.le - cit.kk);   // K values of this stage
+    if (whole && kin == BK) {
 #pragma unroll
-    for (int k4 = 0; k4 < BK / 4; ++k4) {
-      double a[MT], b[NT];
+      for (int k4 = 0; k4 < BK / 4; ++k4) {
+        double a[MT], b[NT];
 #pragma unroll
-      for (int i = 0; i < MT; ++i) a[i] = ap[(8 * i) * a_line_step + 4 * k4 * a_k_step];
+        for (int i = 0; i < MT; ++i) a[i] = ap[(8 * i) * a_line_step + 4 * k4 * a_k_step];
 #pragma unroll
-      for (int j = 0; j < NT; ++j) b[j] = bp[(8 * j) * b_line_step + 4 * k4 * b_k_step];
+        for (int j = 0; j < NT; ++j) b[j] = bp[(8 * j) * b_line_step + 4 * k4 * b_k_step];
 #pragma unroll
-      for (int i = 0; i < MT; ++i)
+        for (int i = 0; i < MT; ++i)
 #pragma unroll
-        for (int j = 0; j < NT; ++j) dmma884(acc[i][j], a[i], b[j]);
+          for (int j = 0; j < NT; ++j) dmma884(acc[i][j], a[i], b[j]);
+      }
+    } else if (mt_in > 0 && nt_in > 0) {
+      // edge of the problem or of a K range: only the MMA tiles and 4-deep
+      // steps that hold something (all uniform over the warp)
+      for (int k4 = 0; 4 * k4 < kin; ++k4) {
+        double b[NT];
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+          if (j < nt_in) b[j] = bp[(8 * j) * b_line_step + 4 * k4 * b_k_step];
+#pragma unroll
+        for (int i = 0; i < MT; ++i)
+          if (i < mt_in) {
+            const double a = ap[(8 * i) * a_line_step + 4 * k4 * a_k_step];
+#pragma unroll
+            for (int j = 0; j < NT; ++j)
+              if (j < nt_in) dmma884(acc[i][j], a, b[j]);
+          }
+      }
     }
     buf = (buf + 1) % kMmaStages;
     advance(cit);
