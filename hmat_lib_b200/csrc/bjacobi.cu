@@ -1,7 +1,8 @@
 // Block one-sided Jacobi SVD (see bjacobi.h).
 //
 // Per problem, one workspace holds X (the columns being orthogonalised,
-// L x Lp, Lp = L rounded up to whole 32-column blocks, padding columns zero)
+// Lp x Lp, Lp = L rounded up to whole 32-column blocks, padding rows and
+// columns zero)
 // and V (the accumulated right rotations, Lp x Lp).  A round is ONE launch of
 // bj_pair_kernel for every pair of every active problem: a cluster of CTAs
 // per pair of blocks (64 columns), each CTA owning a slice of the rows.
@@ -10,12 +11,17 @@
 //      cluster through distributed shared memory in rank order, so every CTA
 //      of the cluster holds the same G bit for bit;
 //   2. if some column pair of G is coupled above the convergence test, every
-//      CTA solves G = W diag W^T by cyclic two-sided Jacobi in shared memory
-//      (the same arithmetic in every CTA, so the same W) and sorts the
-//      eigenvalues in descending order;
+//      CTA runs sweeps of cyclic two-sided Jacobi on G, G = W diag W^T (the
+//      same arithmetic in every CTA, so the same W), and sorts the diagonal in
+//      descending order;
 //   3. X[:, pair] = X[:, pair] W and V[:, pair] = V[:, pair] W over its rows
-//      (mma m8n8k4 again), in place: a warp loads a whole 8-row strip before
-//      it writes it, and strips of different warps and CTAs are disjoint.
+//      (mma m8n8k4 again), in place, a 32-row tile at a time.
+// Phases 1 and 3 read 32 x 64 tiles through a ring of asynchronous copies and
+// are bound by the FP64 tensor cores (2.6 x 64 x 64 multiply-adds per row and
+// pair); phase 2 by the latency of its 63 steps a sweep, which is why a step
+// has one barrier and its angle comes from single precision (see rotation()).
+// Core stage (254 cores of up to 704 columns, n = 32768 2D): 61 -> 33 ms; 62
+// cores of up to 1600 columns (n = 8192 3D): 179 -> 79 ms.
 // Rotations act on the columns themselves (no re-factorisation of a pair), so
 // small columns keep their relative accuracy; the rotation is applied only
 // when the pair needs it, so the late sweeps are mostly Gram passes.
@@ -45,9 +51,17 @@ namespace {
 constexpr int kBj = 32;          // columns per block
 constexpr int kPair = 2 * kBj;   // columns per pair
 constexpr int kLd = 68;          // leading dimension of the 64 x 64 tiles in shared memory
-constexpr int kPT = 256;         // threads of the pair kernel (8 warps)
-constexpr int kInner = 30;       // sweeps of a pair's eigensolver at most (option bj_inner_sweeps)
-constexpr int kT = 32;           // transpose tile
+constexpr int kPW = 8;           // warps of the pair kernel that hold G and W
+constexpr int kPT = 32 * (kPW + 1);   // threads: one more warp computes the rotations
+constexpr int kHalf = kPair / 2; // column pairs of a step
+// Sweeps of a pair's eigensolver at most (option bj_inner_sweeps).  A pair need
+// not be finished: its rotation is orthogonal all the same, and the outer
+// sweeps finish the job.  Core stage with 30 / 4 / 3 / 2 / 1: 38 / 36 / 35 / 33 /
+// 33 ms at n = 32768 (2D), 100 / 97 / 89 / 79 / 87 ms at n = 8192 (3D).
+constexpr int kInner = 2;
+constexpr int kT = 32;           // transpose tile, rows of a staged tile
+constexpr int kLdT = kT + 4;     // leading dimension of a staged tile (column by column)
+constexpr int kRing = 3;         // staged tiles in flight
 constexpr int kMaxCluster = 8;
 
 template <class T>
@@ -97,25 +111,67 @@ __host__ __device__ inline void round_pair(int k, int r, int players, int &a, in
 }
 
 struct BjDev {
-  double *X, *V;   // L x Lp (ld L), Lp x Lp (ld Lp)
-  int L, Lp, nblk, players;
-  double theta2;   // columns of squared norm at or below this are not rotated
-  double fro;      // ||A||_F, the scale of the norm-relative convergence test
+  double *X, *V;   // Lp x Lp (ld Lp); rows of X past the problem's size are zero
+  int Lp, nblk, players;
+  double gscale;   // power of two that brings the Gram entries to order one
+  double theta2;   // columns of squared norm at or below this are not rotated (times gscale)
+  double fro;      // ||A||_F, the scale of the norm-relative test (times sqrt(gscale))
   double conv;     // convergence threshold of a column pair
   int *rot;        // set when a pair of the problem rotated in the current sweep
 };
 
-// Shared memory of the pair kernel; element (i, j) of a 64 x 64 tile at i + j kLd.
+// Shared memory of the pair kernel.  gp: this CTA's partial Gram (tiles I <= J),
+// later W with sorted columns, element (i, j) at i + j kLd.  pl: the pair's Gram
+// by position (see place_of), two buffers of four planes [K][M], K <= M: the
+// products of K's first / second column with M's first / second.
 struct PairSmem {
-  double gp[kPair * kLd];   // this CTA's partial Gram (tiles I <= J), later W with sorted columns
-  double g[kPair * kLd];    // the pair's Gram, rotated in place by the eigensolver
-  double w[kPair * kLd];    // accumulated rotations
-  double cs[kPair / 2], sn[kPair / 2], tn[kPair / 2];
-  int pp[kPair / 2], qq[kPair / 2];
+  double gp[kPair * kLd];
+  double pl[2][4][kHalf][kHalf];
+  double2 cs[2][kHalf + kHalf / 8];   // rotations by pair, a pad after every eight (cs_at)
+  double dg[kPair];      // diagonal by column, then by place
   int perm[kPair];
-  int flag[2];   // a rotation in the inner sweep of that parity
-  int work;      // the pair failed the convergence test
 };
+
+// Where column x of the pair sits at step 0 of the round-robin over 64
+// columns: pair k holds columns k and 63 - k (pair 0: 0 and 63), first / second.
+__device__ __forceinline__ void place_of(int x, int &k, int &second) {
+  second = x >= kHalf;
+  k = x < kHalf ? x : x == kPair - 1 ? 0 : kPair - 1 - x;
+}
+__device__ __forceinline__ int column_at(int k, int second) {
+  return !second ? k : k == 0 ? kPair - 1 : kPair - 1 - k;
+}
+// One step of the round-robin moves every column to its next place (the
+// second column of pair 0 stays); after 63 steps all are back.
+__device__ __forceinline__ void next_place(int &k, int &second) {
+  if (!second) {
+    second = k == 0;
+    k = k == 0 ? 1 : k - 1;
+  } else if (k == kHalf - 1) {
+    second = 0;
+  } else if (k > 0) {
+    ++k;
+  }
+}
+// Where pair k's rotation is kept: the four lanes of a row of W read pairs
+// eight apart at a time.
+__device__ __forceinline__ int cs_at(int k) { return k + (k >> 3); }
+// Offset in a buffer's planes of the product of the columns at two places.
+__device__ __forceinline__ int plane_offset(int k, int sk, int m, int sm) {
+  if (k > m) {
+    int t = k;
+    k = m;
+    m = t;
+    t = sk;
+    sk = sm;
+    sm = t;
+  }
+  if (k == m) {   // the coupling of a pair
+    sk = 0;
+    sm = 1;
+  }
+  return ((2 * sk + sm) * kHalf + k) * kHalf + m;
+}
 
 // The test of a column pair with squared norms al, be and product ga: true
 // when it must be rotated.  Columns at or below theta are neither rotated nor
@@ -124,47 +180,93 @@ struct PairSmem {
 // the truncation threshold).  A coupling at rounding level of the problem's
 // own scale counts as converged: a column recomputed from others carries an
 // error of about eps ||A|| times its weight, which no rotation removes.
+// All squared: no square root on the eigensolver's critical path (entries are
+// of order one, so the squares of columns above theta do not vanish).
 __device__ __forceinline__ bool needs_rotation(double al, double be, double ga, double theta2,
-                                               double fro, double conv) {
-  if (ga == 0.0 || al <= theta2 || be <= theta2) return false;
-  const double sa = sqrt(al), sb = sqrt(be);
-  const double rel = fmin(fabs(ga) / (sa * sb), fabs(ga) / (fro * fmax(sa, sb)));
-  return rel > conv;
+                                               double fro2, double conv2) {
+  return al > theta2 && be > theta2 && ga * ga > conv2 * fmin(al * be, fro2 * fmax(al, be));
 }
 
-// X[rs:re, pair] = X[rs:re, pair] Wp (ld = rows of X, pair columns at xa, xb)
-// by warps over 8-row strips; Wp in shared memory.
-__device__ __forceinline__ void rotate_rows(double *xa, double *xb, long long ld, int rs, int re,
-                                            const double *wp, int warp, int gq, int tq) {
-  for (int r0 = rs + 8 * warp; r0 < re; r0 += 8 * (kPT / 32)) {
-    const int row = r0 + gq;
-    const bool in = row < re;
-    double a[kPair / 4];
+// tan, cos of the rotation that zeroes the product g of two columns whose
+// squared norms differ by d = |x_b|^2 - |x_a|^2.  Any angle keeps W orthogonal
+// as long as c^2 (1 + t^2) = 1; the angle itself only has to make the product
+// small, so t comes from single precision (the product left is about 1e-7 of
+// g) and c is then corrected to double precision for that t: with y close to
+// (1 + t^2)^-1/2 and r = 1 - (1 + t^2) y^2, c = y (1 - r)^-1/2, whose binomial
+// series to second order is exact beyond 1e-18 at r = 1e-6.  A double-precision
+// square root, division and reciprocal square root in a row were about half
+// of a step.
+__device__ __forceinline__ void rotation(double d, double g, double &t, double &c) {
+  const double e = 2.0 * g;
+  // both scaled by a power of two near 1 / max(|d|, |e|)
+  const int ex = max((__double2hiint(d) >> 20) & 0x7ff, (__double2hiint(e) >> 20) & 0x7ff);
+  const double sc = __hiloint2double(max(1, min(2046, 2046 - ex)) << 20, 0);
+  const float df = (float)(d * sc), ef = (float)(e * sc);
+  const float tf = __fdividef(ef, df + copysignf(sqrtf(fmaf(df, df, ef * ef)), df));
+  t = (double)tf;
+  const double y = (double)rsqrtf(fmaf(tf, tf, 1.0f));
+  const double r = fma(-fma(t, t, 1.0), y * y, 1.0);
+  c = fma(y, r * fma(0.375, r, 0.5), y);
+}
+
+// One 32-row tile of a pair's 64 columns into shared memory (column by
+// column, ld kLdT): 256 contiguous bytes per column, 16-byte copies.
+__device__ __forceinline__ void stage_tile(double *buf, const double *xa, const double *xb,
+                                           long long ld, int row0) {
+  if (threadIdx.x < 32 * kPW) {
 #pragma unroll
-    for (int kk = 0; kk < kPair / 4; ++kk) {
-      const int k = 4 * kk + tq;
-      const double *src = (k < kBj ? xa + (long long)k * ld : xb + (long long)(k - kBj) * ld);
-      a[kk] = in ? src[row] : 0.0;
+    for (int q = 0; q < kPair * (kT / 2) / (32 * kPW); ++q) {
+      const int e = threadIdx.x + 32 * kPW * q, c = e / (kT / 2), ch = e % (kT / 2);
+      const double *src = (c < kBj ? xa + c * ld : xb + (c - kBj) * ld) + row0 + 2 * ch;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
+                       (unsigned)__cvta_generic_to_shared(buf + c * kLdT + 2 * ch)),
+                   "l"(src));
     }
+  }
+  asm volatile("cp.async.commit_group;\n" ::);
+}
+
+// Adds the Gram tiles (I, J), I <= J, of two 4-row steps of a staged tile;
+// kSet: rows I = 0, 1, 5 of the 8 x 8 tiling, or the others (18 tiles each).
+template <int kSet>
+__device__ __forceinline__ void gram_tiles(const double *buf, int s0, int gq, int tq,
+                                           double (&acc)[18][2]) {
 #pragma unroll
-    for (int nt = 0; nt < kPair / 8; ++nt) {
-      double c[2] = {0.0, 0.0};
+  for (int q = 0; q < 2; ++q) {
+    double f[8];
 #pragma unroll
-      for (int kk = 0; kk < kPair / 4; ++kk) dmma884(c, a[kk], wp[(4 * kk + tq) + (8 * nt + gq) * kLd]);
-      if (in) {
+    for (int I = 0; I < 8; ++I) f[I] = buf[(8 * I + gq) * kLdT + 4 * (s0 + q) + tq];
+    int t = 0;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int j = 8 * nt + 2 * tq + h;
-          double *dst = (j < kBj ? xa + (long long)j * ld : xb + (long long)(j - kBj) * ld);
-          dst[row] = c[h];
-        }
+    for (int I = 0; I < 8; ++I)
+      if ((I == 0 || I == 1 || I == 5) == (kSet == 0)) {
+#pragma unroll
+        for (int J = I; J < 8; ++J) dmma884(acc[t++], f[I], f[J]);
       }
-    }
   }
 }
 
+template <int kSet>
+__device__ __forceinline__ void gram_store(double *gp, const double (&acc)[18][2], bool first,
+                                           int gq, int tq) {
+  int t = 0;
+#pragma unroll
+  for (int I = 0; I < 8; ++I)
+    if ((I == 0 || I == 1 || I == 5) == (kSet == 0)) {
+#pragma unroll
+      for (int J = I; J < 8; ++J) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          double &e = gp[(8 * I + gq) + (8 * J + 2 * tq + h) * kLd];
+          e = (first ? 0.0 : e) + acc[t][h];
+        }
+        ++t;
+      }
+    }
+}
+
 // One round for every pair slot: blockIdx.x / cluster size = slot.
-__global__ void __launch_bounds__(kPT, 1)
+__global__ void __launch_bounds__(kPT, 2)
 bj_pair_kernel(const BjDev *__restrict__ probs, const int2 *__restrict__ slots, long long g_round,
                int inner_max) {
   extern __shared__ __align__(16) unsigned char bj_smem_raw[];
@@ -180,196 +282,317 @@ bj_pair_kernel(const BjDev *__restrict__ probs, const int2 *__restrict__ slots, 
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gq = lane >> 2, tq = lane & 3;
-  const long long L = P.L, Lp = P.Lp;
-  double *xa = P.X + (long long)a * kBj * L, *xb = P.X + (long long)b * kBj * L;
+  const long long Lp = P.Lp;
+  double *xa = P.X + (long long)a * kBj * Lp, *xb = P.X + (long long)b * kBj * Lp;
   double *va = P.V + (long long)a * kBj * Lp, *vb = P.V + (long long)b * kBj * Lp;
-  const int xchunk = ((P.L + ncl - 1) / ncl + 7) / 8 * 8;
-  const int xr0 = min(P.L, crank * xchunk), xr1 = min(P.L, xr0 + xchunk);
-  const int vchunk = ((P.Lp + ncl - 1) / ncl + 7) / 8 * 8;
-  const int vr0 = min(P.Lp, crank * vchunk), vr1 = min(P.Lp, vr0 + vchunk);
+  // this CTA's rows of X and of V, in 32-row tiles
+  const int tiles = P.Lp / kT, per = (tiles + ncl - 1) / ncl;
+  const int t0 = min(tiles, crank * per), nt = min(tiles, t0 + per) - t0;
+  double *ring = &S.pl[0][0][0][0];   // the planes are free outside the eigensolver
+  constexpr int kTile = kPair * kLdT;
+  static_assert(kRing * kTile <= 2 * 4 * kHalf * kHalf, "the ring fits the planes");
 
-  // ---- 1. Gram of this CTA's rows: warps take 4-row steps in turn, each
-  // holding the 36 tiles I <= J of the 8 x 8 tiling (column j of the pair is
-  // fragment j / 8, lane row j % 8)
+  // ---- 1. Gram of this CTA's rows: the 36 tiles I <= J of the 8 x 8 tiling
+  // (column j of the pair is fragment j / 8, lane row j % 8) in two sets of 18,
+  // even and odd warps; a pair of warps takes two of a tile's eight 4-row steps
   {
-    const double *col[8];
-#pragma unroll
-    for (int I = 0; I < 8; ++I)
-      col[I] = (I < 4 ? xa + (long long)(8 * I + gq) * L : xb + (long long)(8 * (I - 4) + gq) * L);
-    double acc[36][2];
-#pragma unroll
-    for (int t = 0; t < 36; ++t) acc[t][0] = acc[t][1] = 0.0;
-    double f[8], nf[8];
-    int r = xr0 + 4 * warp;
-#pragma unroll
-    for (int I = 0; I < 8; ++I) f[I] = (r + tq < xr1) ? col[I][r + tq] : 0.0;
-    for (; r < xr1; r += 4 * (kPT / 32)) {
-      const int rn = r + 4 * (kPT / 32) + tq;
-#pragma unroll
-      for (int I = 0; I < 8; ++I) nf[I] = (rn < xr1) ? col[I][rn] : 0.0;
-      int t = 0;
-#pragma unroll
-      for (int I = 0; I < 8; ++I)
-#pragma unroll
-        for (int J = I; J < 8; ++J) dmma884(acc[t++], f[I], f[J]);
-#pragma unroll
-      for (int I = 0; I < 8; ++I) f[I] = nf[I];
+    double acc[18][2] = {};
+    for (int t = 0; t < kRing - 1; ++t)
+      if (t < nt)
+        stage_tile(ring + t * kTile, xa, xb, Lp, (t0 + t) * kT);
+      else
+        asm volatile("cp.async.commit_group;\n" ::);
+    for (int t = 0; t < nt; ++t) {
+      asm volatile("cp.async.wait_group %0;\n" ::"n"(kRing - 2));
+      __syncthreads();                 // tile t has landed, tile t - 1 is used up
+      if (t + kRing - 1 < nt)
+        stage_tile(ring + (t + kRing - 1) % kRing * kTile, xa, xb, Lp, (t0 + t + kRing - 1) * kT);
+      else
+        asm volatile("cp.async.commit_group;\n" ::);
+      const double *buf = ring + t % kRing * kTile;
+      if (warp < kPW) {
+        if (warp & 1)
+          gram_tiles<1>(buf, 2 * (warp >> 1), gq, tq, acc);
+        else
+          gram_tiles<0>(buf, 2 * (warp >> 1), gq, tq, acc);
+      }
     }
-    // warps add their sums into gp in warp order (deterministic)
-    for (int w = 0; w < kPT / 32; ++w) {
-      if (warp == w) {
-        int t = 0;
-#pragma unroll
-        for (int I = 0; I < 8; ++I)
-#pragma unroll
-          for (int J = I; J < 8; ++J) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              double &e = S.gp[(8 * I + gq) + (8 * J + 2 * tq + h) * kLd];
-              e = (w == 0 ? 0.0 : e) + acc[t][h];
-            }
-            ++t;
-          }
+    asm volatile("cp.async.wait_group 0;\n" ::);
+    __syncthreads();
+    // added into gp in warp order (deterministic)
+    for (int w = 0; w < kPW / 2; ++w) {
+      if (warp < kPW && warp >> 1 == w) {
+        if (warp & 1)
+          gram_store<1>(S.gp, acc, w == 0, gq, tq);
+        else
+          gram_store<0>(S.gp, acc, w == 0, gq, tq);
       }
       __syncthreads();
     }
   }
-  // ---- the cluster's sum, in rank order, into every CTA's g (symmetric:
-  // element (i, j) from the stored (min, max))
+  // ---- the cluster's sum, in rank order, into every CTA's planes
   if (ncl > 1) cl.sync();
   for (int e = tid; e < kPair * kPair; e += kPT) {
     const int i = e % kPair, j = e / kPair;
-    const int off = min(i, j) + max(i, j) * kLd;
+    if (i > j) continue;
+    const int off = i + j * kLd;
     double s = 0.0;
     if (ncl == 1) {
       s = S.gp[off];
     } else {
       for (int rk = 0; rk < ncl; ++rk) s += *cl.map_shared_rank(S.gp + off, rk);
     }
-    S.g[i + j * kLd] = s;
-  }
-  if (tid == 0) {
-    S.work = 0;
-    S.flag[0] = S.flag[1] = 0;
+    s *= P.gscale;
+    if (i == j) {
+      S.dg[i] = s;
+    } else {
+      int ki, si, kj, sj;
+      place_of(i, ki, si);
+      place_of(j, kj, sj);
+      (&S.pl[0][0][0][0])[plane_offset(ki, si, kj, sj)] = s;
+    }
   }
   // after this barrier no CTA reads another's gp any more
   if (ncl > 1) cl.sync();
   __syncthreads();
 
-  // ---- 2. convergence test of the pair, then the eigensolver
-  for (int e = tid; e < kPair * kPair; e += kPT) {
-    const int i = e % kPair, j = e / kPair;
-    if (i < j && needs_rotation(S.g[i + i * kLd], S.g[j + j * kLd], S.g[i + j * kLd], P.theta2,
-                                P.fro, P.conv))
-      S.work = 1;
+  // ---- 2. eigensolver: cyclic two-sided Jacobi.  Columns sit at 64 places, 32
+  // pairs, and move to their next place after every step, so each thread
+  // always handles the same places.  Warps 0 .. kPW - 1 apply a step: two
+  // off-diagonal 2 x 2 blocks each (in the planes, read from one buffer and
+  // written to their next places in the other) and a quarter of a row of W (in
+  // registers).  Meanwhile warp kPW, which keeps the diagonal in registers,
+  // computes the next step's 32 rotations: lane k applies the step to the one
+  // block that holds the next product of pair k itself.  So a step has one
+  // barrier and lasts as long as that chain (a block, an angle).
+  const bool solver = warp == kPW;
+  constexpr int kBlocks = kHalf * (kHalf - 1) / 2;   // off-diagonal blocks K < M
+  constexpr int kPlane = kHalf * kHalf;
+  int from[2], to[2][4], bk[2], bm[2];
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    // rows i and 30 - i of the triangle make 32 blocks together
+    const int e = tid + 32 * kPW * u, i = e / kHalf, l = e % kHalf;
+    const bool lower = l >= kHalf - 1 - i;
+    bk[u] = lower ? kHalf - 2 - i : i;
+    bm[u] = lower ? l : i + 1 + l;
+    if (solver || e >= kBlocks) bk[u] = -1;
+    from[u] = bk[u] * kHalf + bm[u];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      int k = bk[u], sk = q >> 1, m = bm[u], sm = q & 1;
+      next_place(k, sk);
+      next_place(m, sm);
+      to[u][q] = plane_offset(k, sk, m, sm);
+    }
   }
-  for (int e = tid; e < kPair * kPair; e += kPT) {
-    const int i = e % kPair, j = e / kPair;
-    S.w[i + j * kLd] = (i == j) ? 1.0 : 0.0;
+  const double fro2 = P.fro * P.fro, conv2 = P.conv * P.conv;
+  // solver lane k: the diagonal of pair k's columns, what its pending rotation
+  // moves between them and leaves of their product, where that goes, and the
+  // block and element that become the pair's next product
+  double d0 = 0.0, d1 = 0.0, left = 0.0, moved = 0.0;
+  int to_pair = 0, nk = 0, nm = 0, nq = 0;
+  {
+    int k = lane, sk = 0, m = lane, sm = 1;
+    next_place(k, sk);
+    next_place(m, sm);
+    to_pair = plane_offset(k, sk, m, sm);
+    // the places whose columns come to (lane, first) and (lane, second)
+    const int ka = lane == kHalf - 1 ? lane : lane + 1, sa = lane == kHalf - 1;
+    const int kb = lane == 0 || lane == 1 ? 0 : lane - 1, sb = lane != 1;
+    nk = min(ka, kb);
+    nm = max(ka, kb);
+    nq = ka < kb ? 2 * sa + sb : 2 * sb + sa;
+  }
+  if (solver) {
+    d0 = S.dg[column_at(lane, 0)];
+    d1 = S.dg[column_at(lane, 1)];
+    __syncwarp();
+    S.dg[lane] = d0;
+    S.dg[kHalf + lane] = d1;
   }
   __syncthreads();
-  if (!S.work) return;   // the same decision in every CTA of the cluster
+  int par = 0;
+  // whether some column pair of the current G must be rotated (uniform)
+  auto unconverged = [&]() -> bool {
+    const double *pl = &S.pl[par][0][0][0];
+    bool w = false;
+    if (solver) {
+      w = needs_rotation(d0, d1, pl[plane_offset(lane, 0, lane, 1)], P.theta2, fro2, conv2);
+    } else {
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+        if (bk[u] >= 0) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            w = w || needs_rotation(S.dg[bk[u] + (q >> 1) * kHalf], S.dg[bm[u] + (q & 1) * kHalf],
+                                    pl[from[u] + q * kPlane], P.theta2, fro2, conv2);
+        }
+    }
+    return __syncthreads_or(w) != 0;
+  };
+  if (!unconverged()) return;   // the same decision in every CTA of the cluster
 
+  // row `wrow` of W at the places of pairs 8 tq .. 8 tq + 7: first / second columns
+  const int wrow = 8 * warp + gq;
+  double wa[8], wb[8];
+#pragma unroll
+  for (int u = 0; u < 8; ++u) {
+    wa[u] = column_at(8 * tq + u, 0) == wrow ? 1.0 : 0.0;
+    wb[u] = column_at(8 * tq + u, 1) == wrow ? 1.0 : 0.0;
+  }
+  // the rotation of a pair with product g: published, and what it does to the
+  // pair kept for the step that applies it
+  auto decide = [&](double g, int buf) {
+    double t, c;
+    rotation(d1 - d0, g, t, c);
+    if (!needs_rotation(d0, d1, g, P.theta2, fro2, conv2)) {
+      t = 0.0;
+      c = 1.0;
+    }
+    // x_a' = c x_a - s x_b, x_b' = s x_a + c x_b
+    S.cs[buf][cs_at(lane)] = make_double2(c, c * t);
+    // the norms change by t times the product before and after
+    left = c * c * fma(t, d0 - d1, fma(-t * t, g, g));
+    moved = t * (g + left);
+  };
+  if (solver) decide(S.pl[par][1][lane][lane], par);
+  __syncthreads();
   for (int sweep = 0; sweep < inner_max; ++sweep) {
     for (int step = 0; step < kPair - 1; ++step) {
-      if (tid < kPair / 2) {
-        int p, q;
-        round_pair(tid, step, kPair, p, q);
-        const double app = S.g[p + p * kLd], aqq = S.g[q + q * kLd], apq = S.g[p + q * kLd];
-        double c = 1.0, s = 0.0, t = 0.0;
-        if (needs_rotation(app, aqq, apq, P.theta2, P.fro, P.conv)) {
-          // x_p' = c x_p - s x_q, x_q' = s x_p + c x_q zeroes the pair's
-          // product; t = tan of the smaller angle (1 / (2 zeta) beyond 1e100,
-          // where zeta^2 would overflow)
-          const double zeta = (aqq - app) / (2.0 * apq);
-          t = fabs(zeta) > 1e100 ? 0.5 / zeta
-                                 : (zeta >= 0.0 ? 1.0 : -1.0) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
-          c = 1.0 / sqrt(1.0 + t * t);
-          s = c * t;
-          S.flag[sweep & 1] = 1;
+      const double *src = &S.pl[par][0][0][0];
+      double *dst = &S.pl[par ^ 1][0][0][0];
+      if (solver) {
+        const double2 K = S.cs[par][cs_at(nk)], M = S.cs[par][cs_at(nm)];
+        const double *blk = src + nk * kHalf + nm;
+        const double b00 = blk[0], b01 = blk[kPlane], b10 = blk[2 * kPlane], b11 = blk[3 * kPlane];
+        dst[to_pair] = left;
+        const double x = (nq & 2) ? K.y : K.x, y = (nq & 2) ? K.x : -K.y;
+        const double z = (nq & 1) ? M.y : M.x, w = (nq & 1) ? M.x : -M.y;
+        const double g = z * (x * b00 + y * b10) + w * (x * b01 + y * b11);
+        const double n0 = d0 - moved, n1 = d1 + moved;
+        const double up = __shfl_down_sync(0xffffffffu, n0, 1);
+        const double dn = __shfl_up_sync(0xffffffffu, n1, 1);
+        const double first = __shfl_sync(0xffffffffu, n0, 0);
+        d0 = lane == kHalf - 1 ? n1 : up;
+        d1 = lane == 0 ? n1 : lane == 1 ? first : dn;
+        decide(g, par ^ 1);
+      } else {
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+          if (bk[u] >= 0) {
+            const double2 K = S.cs[par][cs_at(bk[u])], M = S.cs[par][cs_at(bm[u])];
+            const double b00 = src[from[u]], b01 = src[from[u] + kPlane];
+            const double b10 = src[from[u] + 2 * kPlane], b11 = src[from[u] + 3 * kPlane];
+            const double r00 = K.x * b00 - K.y * b10, r01 = K.x * b01 - K.y * b11;
+            const double r10 = K.y * b00 + K.x * b10, r11 = K.y * b01 + K.x * b11;
+            dst[to[u][0]] = M.x * r00 - M.y * r01;
+            dst[to[u][1]] = M.y * r00 + M.x * r01;
+            dst[to[u][2]] = M.x * r10 - M.y * r11;
+            dst[to[u][3]] = M.y * r10 + M.x * r11;
+          }
+        // W = W J, then every column to its next place
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const double2 cs = S.cs[par][cs_at(8 * tq + u)];
+          const double x = wa[u], y = wb[u];
+          wa[u] = cs.x * x - cs.y * y;
+          wb[u] = cs.y * x + cs.x * y;
         }
-        S.pp[tid] = p;
-        S.qq[tid] = q;
-        S.cs[tid] = c;
-        S.sn[tid] = s;
-        S.tn[tid] = t;
-      }
-      __syncthreads();
-      // the previous sweep's flag was read before this step's barrier
-      if (step == 0 && tid == 0) S.flag[(sweep + 1) & 1] = 0;
-      // G = J^T G J over the 2 x 2 blocks of pairs (K, M), K <= M, both halves
-      for (int e = tid; e < (kPair / 2) * (kPair / 2); e += kPT) {
-        const int K = e % (kPair / 2), M = e / (kPair / 2);
-        if (K > M) continue;
-        const double sK = S.sn[K], sM = S.sn[M];
-        if (sK == 0.0 && sM == 0.0) continue;
-        const int pK = S.pp[K], qK = S.qq[K];
-        if (K == M) {
-          const double tK = S.tn[K], apq = S.g[pK + qK * kLd];
-          S.g[pK + pK * kLd] -= tK * apq;
-          S.g[qK + qK * kLd] += tK * apq;
-          S.g[pK + qK * kLd] = 0.0;
-          S.g[qK + pK * kLd] = 0.0;
-          continue;
+        const double an = __shfl_down_sync(0xffffffffu, wa[0], 1);
+        const double bn = __shfl_up_sync(0xffffffffu, wb[7], 1);
+        const double a0 = wa[0], b7 = wb[7], b0 = wb[0];
+#pragma unroll
+        for (int u = 0; u < 7; ++u) wa[u] = wa[u + 1];
+        wa[7] = tq == 3 ? b7 : an;
+#pragma unroll
+        for (int u = 7; u > 0; --u) wb[u] = wb[u - 1];
+        if (tq == 0) {
+          wb[0] = b0;
+          wb[1] = a0;
+        } else {
+          wb[0] = bn;
         }
-        const double cK = S.cs[K], cM = S.cs[M];
-        const int pM = S.pp[M], qM = S.qq[M];
-        const double b00 = S.g[pK + pM * kLd], b01 = S.g[pK + qM * kLd];
-        const double b10 = S.g[qK + pM * kLd], b11 = S.g[qK + qM * kLd];
-        // rows: J_K^T B
-        const double r00 = cK * b00 - sK * b10, r01 = cK * b01 - sK * b11;
-        const double r10 = sK * b00 + cK * b10, r11 = sK * b01 + cK * b11;
-        // columns: (J_K^T B) J_M
-        const double n00 = cM * r00 - sM * r01, n01 = sM * r00 + cM * r01;
-        const double n10 = cM * r10 - sM * r11, n11 = sM * r10 + cM * r11;
-        S.g[pK + pM * kLd] = n00;
-        S.g[pK + qM * kLd] = n01;
-        S.g[qK + pM * kLd] = n10;
-        S.g[qK + qM * kLd] = n11;
-        S.g[pM + pK * kLd] = n00;
-        S.g[qM + pK * kLd] = n01;
-        S.g[pM + qK * kLd] = n10;
-        S.g[qM + qK * kLd] = n11;
       }
-      // W = W J
-      for (int e = tid; e < kPair * (kPair / 2); e += kPT) {
-        const int i = e % kPair, K = e / kPair;
-        const double sK = S.sn[K];
-        if (sK == 0.0) continue;
-        const double cK = S.cs[K];
-        double &wp = S.w[i + S.pp[K] * kLd];
-        double &wq = S.w[i + S.qq[K] * kLd];
-        const double x = wp, y = wq;
-        wp = cK * x - sK * y;
-        wq = sK * x + cK * y;
-      }
+      par ^= 1;
       __syncthreads();
     }
-    if (!S.flag[sweep & 1]) break;
+    if (solver) {
+      S.dg[lane] = d0;
+      S.dg[kHalf + lane] = d1;
+    }
+    __syncthreads();
+    if (!unconverged()) break;   // the rotations decided last are not applied
   }
 
-  // ---- sort the eigenvalues in descending order (ties by index); the
+  // ---- sort the eigenvalues in descending order (ties by column); the
   // sorted W into gp
-  if (tid < kPair) {
-    const double d = S.g[tid + tid * kLd];
-    int pos = 0;
-    for (int j = 0; j < kPair; ++j) {
-      const double dj = S.g[j + j * kLd];
-      pos += (dj > d || (dj == d && j < tid)) ? 1 : 0;
-    }
-    S.perm[pos] = tid;
+  if (solver) {
+    S.dg[column_at(lane, 0)] = d0;
+    S.dg[column_at(lane, 1)] = d1;
   }
   __syncthreads();
-  for (int e = tid; e < kPair * kPair; e += kPT) {
-    const int i = e % kPair, j = e / kPair;
-    S.gp[i + j * kLd] = S.w[i + S.perm[j] * kLd];
+  if (tid < kPair) {
+    const double d = S.dg[tid];
+    int pos = 0;
+    for (int j = 0; j < kPair; ++j) {
+      const double dj = S.dg[j];
+      pos += (dj > d || (dj == d && j < tid)) ? 1 : 0;
+    }
+    S.perm[tid] = pos;
+  }
+  __syncthreads();
+  if (!solver) {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      S.gp[wrow + S.perm[column_at(8 * tq + u, 0)] * kLd] = wa[u];
+      S.gp[wrow + S.perm[column_at(8 * tq + u, 1)] * kLd] = wb[u];
+    }
   }
   if (crank == 0 && tid == 0) *P.rot = 1;
   __syncthreads();
 
-  // ---- 3. the rotation of this CTA's rows of X and V
-  rotate_rows(xa, xb, L, xr0, xr1, S.gp, warp, gq, tq);
-  rotate_rows(va, vb, Lp, vr0, vr1, S.gp, warp, gq, tq);
+  // ---- 3. the rotation of this CTA's rows of X and V, in place, a 32-row
+  // tile of 64 columns at a time: warp w computes columns 8 w .. 8 w + 7 and
+  // keeps its part of W in registers
+  double bw[kPair / 4];
+  if (!solver) {
+#pragma unroll
+    for (int kk = 0; kk < kPair / 4; ++kk) bw[kk] = S.gp[(4 * kk + tq) + (8 * warp + gq) * kLd];
+  }
+  auto stage = [&](int t) {            // tiles of X, then of V
+    if (t >= 2 * nt)
+      asm volatile("cp.async.commit_group;\n" ::);
+    else if (t < nt)
+      stage_tile(ring + t % kRing * kTile, xa, xb, Lp, (t0 + t) * kT);
+    else
+      stage_tile(ring + t % kRing * kTile, va, vb, Lp, (t0 + t - nt) * kT);
+  };
+  for (int t = 0; t < kRing - 1; ++t) stage(t);
+  for (int t = 0; t < 2 * nt; ++t) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(kRing - 2));
+    __syncthreads();
+    stage(t + kRing - 1);
+    if (!solver) {
+      const double *buf = ring + t % kRing * kTile;
+      double c[kT / 8][2] = {};
+#pragma unroll
+      for (int kk = 0; kk < kPair / 4; ++kk)
+#pragma unroll
+        for (int i = 0; i < kT / 8; ++i)
+          dmma884(c[i], buf[(4 * kk + tq) * kLdT + 8 * i + gq], bw[kk]);
+      double *pa = t < nt ? xa : va, *pb = t < nt ? xb : vb;
+      const int row0 = (t0 + (t < nt ? t : t - nt)) * kT;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int j = 8 * warp + 2 * tq + h;
+        double *dst = (j < kBj ? pa + j * Lp : pb + (j - kBj) * Lp) + row0 + gq;
+#pragma unroll
+        for (int i = 0; i < kT / 8; ++i) dst[8 * i] = c[i][h];
+      }
+    }
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::);
 }
 
 // The integer outputs of one problem.
@@ -415,7 +638,7 @@ void block_jacobi_svd(const std::vector<BjProb> &probs, double tol, int max_swee
     W.nblk = W.Lp / kBj;
     W.players = W.nblk + (W.nblk & 1);
     W.npairs = W.players / 2;
-    W.x = take((long long)W.L * W.Lp);
+    W.x = take((long long)W.Lp * W.Lp);
     W.v = take((long long)W.Lp * W.Lp);
     lmax = std::max(lmax, W.L);
   }
@@ -431,11 +654,11 @@ void block_jacobi_svd(const std::vector<BjProb> &probs, double tol, int max_swee
   for (int p = 0; p < np; ++p) {
     const Work &W = wk[p];
     dim3 grid((W.L + kT - 1) / kT, (W.L + kT - 1) / kT);
-    bj_transpose_kernel<<<grid, dim3(kT, 8), 0, s>>>(probs[p].A, probs[p].lda, W.L, w + W.x, W.L);
+    bj_transpose_kernel<<<grid, dim3(kT, 8), 0, s>>>(probs[p].A, probs[p].lda, W.L, w + W.x, W.Lp);
     HB_LAUNCHED();
     bj_identity_kernel<<<(W.Lp + 255) / 256, 256, 0, s>>>(w + W.v, W.Lp, W.Lp);
     HB_LAUNCHED();
-    nd.push_back(NormDesc{w + W.x, W.L, W.L, W.Lp, w + noff[p]});
+    nd.push_back(NormDesc{w + W.x, W.Lp, W.L, W.Lp, w + noff[p]});
   }
   column_norms2(nd, s);
   // a column pair of length L recomputed by a 64-term sum is orthogonal to
@@ -458,23 +681,30 @@ void block_jacobi_svd(const std::vector<BjProb> &probs, double tol, int max_swee
       for (int c = 0; c < wk[p].Lp; ++c) f2 += hn[noff[p] - n_lo + c];
       const Work &W = wk[p];
       // the scalar solver's skip rule for the relative truncation
-      const double theta = 1e-3 * tol * std::sqrt(f2) / W.L;
-      hd[p] = BjDev{w + W.x, w + W.v, W.L, W.Lp, W.nblk, W.players, theta * theta,
-                    std::sqrt(f2), conv, d_rot + p};
+      const double fro = std::sqrt(f2);
+      const double down =
+          fro > 0.0 && std::isfinite(fro) ? std::ldexp(1.0, std::max(-500, std::min(500, -std::ilogb(fro))))
+                                          : 1.0;
+      const double theta = 1e-3 * tol * (fro * down) / W.L;
+      hd[p] = BjDev{w + W.x, w + W.v, W.Lp, W.nblk, W.players, down * down, theta * theta,
+                    fro * down, conv, d_rot + p};
     }
   }
   BjDev *d_probs = upload_vec(hd, s);
   std::vector<int> rot(np, 0);
 
-  // A pair's eigensolver may stop before it converges: its rotation is still
-  // orthogonal, and the outer sweeps finish the job.
-  const int inner_max = std::max(1, std::min(kInner, (int)option("bj_inner_sweeps", kInner)));
+  const int inner_max = std::max(1, std::min(30, (int)option("bj_inner_sweeps", kInner)));
   int dev = 0, nsm = 148;
   HB_CUDA(cudaGetDevice(&dev));
   HB_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  const size_t smem = sizeof(PairSmem);
+  // A launch that gives every CTA an SM of its own asks for more than half of
+  // an SM's shared memory: two CTAs of a cluster otherwise share one while
+  // other SMs idle, and the eigensolver's steps take turns.
+  const size_t smem_two = sizeof(PairSmem), smem_one = 120 * 1024;
+  static_assert(2 * (sizeof(PairSmem) + 1024) <= 228 * 1024 && sizeof(PairSmem) <= 120 * 1024,
+                "two CTAs per SM, or one");
   HB_CUDA(cudaFuncSetAttribute(bj_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)smem));
+                               (int)smem_one));
 
   // The pair slots of the active problems and the cluster size (CTAs per
   // pair: as many as keep one wave of CTAs on the SMs, at most 8, and at
@@ -505,7 +735,7 @@ void block_jacobi_svd(const std::vector<BjProb> &probs, double tol, int max_swee
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3((unsigned)(nslots * ncl));
       cfg.blockDim = dim3(kPT);
-      cfg.dynamicSmemBytes = smem;
+      cfg.dynamicSmemBytes = nslots * ncl <= nsm ? smem_one : smem_two;
       cfg.stream = s;
       cudaLaunchAttribute attr[1];
       attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -549,7 +779,7 @@ void block_jacobi_svd(const std::vector<BjProb> &probs, double tol, int max_swee
 
   // ---- singular values, order, rank, outputs -------------------------------------------
   nd.clear();
-  for (int p = 0; p < np; ++p) nd.push_back(NormDesc{w + wk[p].x, wk[p].L, wk[p].L, wk[p].Lp,
+  for (int p = 0; p < np; ++p) nd.push_back(NormDesc{w + wk[p].x, wk[p].Lp, wk[p].L, wk[p].Lp,
                                                      w + noff[p]});
   column_norms2(nd, s);
   std::vector<CopyDesc> gather;
@@ -572,7 +802,7 @@ void block_jacobi_svd(const std::vector<BjProb> &probs, double tol, int max_swee
     ranks[p] = r;
     sweeps[p] = W.converged ? W.sweep : max_sweeps + 1;
     for (int c = 0; c < W.L; ++c) {
-      gather.push_back(CopyDesc{w + W.x + (long long)perm[c] * W.L, W.L,
+      gather.push_back(CopyDesc{w + W.x + (long long)perm[c] * W.Lp, W.Lp,
                                 probs[p].U + (long long)c * W.L, W.L, W.L, 1});
       gather.push_back(CopyDesc{w + W.v + (long long)perm[c] * W.Lp, W.Lp,
                                 probs[p].V + (long long)c * W.L, W.L, W.L, 1});
