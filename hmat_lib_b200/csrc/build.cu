@@ -66,14 +66,18 @@ struct SketchBlock {
 };
 
 // Device memory free or held unused by the device's default stream-ordered
-// pool (bytes).
+// pool or the library's scratch pool (bytes).
 double device_avail_bytes() {
   size_t free_b = 0, total_b = 0;
   HB_CUDA(cudaMemGetInfo(&free_b, &total_b));
   double avail = (double)free_b;
   int dev = 0;
-  cudaMemPool_t pool;
-  if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
+  cudaMemPool_t pools[2] = {nullptr, scratch_pool()};
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetDefaultMemPool(&pools[0], dev) != cudaSuccess)
+    pools[0] = nullptr;
+  for (cudaMemPool_t pool : pools) {
+    if (!pool) continue;
     uint64_t reserved = 0, used = 0;
     if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) ==
             cudaSuccess &&
@@ -440,6 +444,7 @@ std::vector<std::shared_ptr<DeviceTree>> build_attempt(
   std::vector<double *> grown;
   const double mem_frac = option("sketch_mem_frac", 0.6);
   double limited_avail = -1.0;   // device memory seen by the first growth that did not fit
+  double round_avail = -1.0;     // device memory left to this round's growths (-1: not asked yet)
   auto grow = [&](SketchBlock &S, int limit) {
     const long long wbw = std::max(S.first_w, w_next);
     const long long m = S.m, n = S.n, e = S.ell;
@@ -453,7 +458,8 @@ std::vector<std::shared_ptr<DeviceTree>> build_attempt(
     };
     // twice the width, else smaller steps, whichever fits the memory budget
     // together with the block's core SVD (about five c2^2 doubles)
-    const double avail = cap_opt > 0 ? 1e300 : device_avail_bytes();
+    if (round_avail < 0.0) round_avail = cap_opt > 0 ? 1e300 : device_avail_bytes();
+    const double avail = round_avail;
     int c2 = 0;
     long long parts[5];
     for (int cand : {2 * S.cap, S.cap + S.cap / 2, S.cap + 256, S.cap + kPanel}) {
@@ -472,6 +478,7 @@ std::vector<std::shared_ptr<DeviceTree>> build_attempt(
     const long long sq = parts[0], sb = parts[1], sr = parts[2], st = parts[3];
     double *g = dev_alloc(total, stream);
     grown.push_back(g);
+    round_avail = std::max(0.0, round_avail - 8.0 * (double)total);
     HB_CUDA(cudaMemsetAsync(g, 0, sizeof(double) * total, stream));
     const long long base = (long long)(g - work);
     const long long q = base, bt = q + sq, pp = bt + sb, rb = pp + sb, t = rb + sr, c = t + st;
@@ -562,6 +569,7 @@ std::vector<std::shared_ptr<DeviceTree>> build_attempt(
       if (!sk[i].done) act.push_back((int)i);
     if (act.empty()) break;
     std::vector<int> wb(sk.size(), 0);
+    round_avail = -1.0;
     for (int i : act) {
       const int wr = rounds == 0 ? sk[i].first_w : w_next;
       if (sk[i].ell >= sk[i].cap && sk[i].cap < memcap[i]) grow(sk[i], memcap[i]);

@@ -77,10 +77,59 @@ void keep_pool_memory() {
     (void)cudaGetLastError();
 }
 
+// Scratch of 32 MiB or more comes from a pool of the library's own, one per
+// device.  Trees and plans outlive a call, so in the default pool they land in
+// the holes that a build's gigabytes of scratch leave, and the next build maps
+// fresh memory: cudaMallocAsync calls of 30 to 1000 ms in every third or fourth
+// of a row of n = 32768 builds (170 ms of work each).  Here everything is free
+// again when a call ends, and sizes are rounded up to an eighth of a power of
+// two, so the next call finds the same blocks.  The pool keeps at most half of
+// the device's memory mapped (nothing with option pool_keep = 0), and gives all
+// of it back when an allocation would fail otherwise.
+cudaMemPool_t scratch_pool() {
+  static std::mutex mu;
+  static std::map<int, cudaMemPool_t> pools;
+  int dev = 0;
+  HB_CUDA(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lk(mu);
+  auto it = pools.find(dev);
+  if (it != pools.end()) return it->second;
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = dev;
+  cudaMemPool_t pool = nullptr;
+  HB_CUDA(cudaMemPoolCreate(&pool, &props));
+  size_t free_b = 0, total_b = 0;
+  HB_CUDA(cudaMemGetInfo(&free_b, &total_b));
+  uint64_t keep = option("pool_keep", 1.0) == 0.0 ? 0 : total_b / 2;
+  HB_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+  pools[dev] = pool;
+  return pool;
+}
+
 double *dev_alloc(size_t elems, cudaStream_t stream) {
   keep_pool_memory();
+  constexpr size_t kLarge = size_t(32) << 20;
+  size_t bytes = std::max<size_t>(elems, 1) * sizeof(double);
   void *p = nullptr;
-  HB_CUDA(cudaMallocAsync(&p, std::max<size_t>(elems, 1) * sizeof(double), stream));
+  if (bytes >= kLarge) {
+    size_t step = kLarge / 8;
+    while (step * 16 <= bytes) step *= 2;
+    bytes = (bytes + step - 1) / step * step;
+    const cudaMemPool_t pool = scratch_pool();
+    cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, pool, stream);
+    if (e == cudaErrorMemoryAllocation) {
+      // memory that other work has released but not returned
+      (void)cudaGetLastError();
+      HB_CUDA(cudaStreamSynchronize(stream));
+      HB_CUDA(cudaMemPoolTrimTo(pool, 0));
+      e = cudaMallocFromPoolAsync(&p, std::max<size_t>(elems, 1) * sizeof(double), pool, stream);
+    }
+    HB_CUDA(e);
+    return (double *)p;
+  }
+  HB_CUDA(cudaMallocAsync(&p, bytes, stream));
   return (double *)p;
 }
 

@@ -87,6 +87,8 @@ cudaStream_t lib_stream();
 // pool (once per device; option pool_keep).
 void keep_pool_memory();
 double *dev_alloc(size_t elems, cudaStream_t stream);
+// The pool that large scratch comes from.
+cudaMemPool_t scratch_pool();
 void dev_free(void *p, cudaStream_t stream);
 
 

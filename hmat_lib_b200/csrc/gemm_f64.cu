@@ -713,10 +713,9 @@ void gemm_plan_build(GemmPlan &plan, GemmBatch &batch, TileShape shape, bool all
   }
   plan.transient = transient;
   plan.stream = stream;
-  if (transient)
-    HB_CUDA(cudaMallocAsync(&plan.dev, total, stream));
-  else
-    HB_CUDA(cudaMalloc(&plan.dev, total));
+  // stream-ordered in both cases (a cudaMalloc stops the device); a kept plan
+  // is ready for any stream after the synchronisation below
+  HB_CUDA(cudaMallocAsync(&plan.dev, total, stream));
   char *base = (char *)plan.dev;
   plan.segs = (GemmSeg *)base;
   plan.probs = (GemmProb *)(base + align_up(bs, 256));

@@ -127,12 +127,14 @@ ProductPlan &product_plan(DeviceTree &t, ProdOp op, int k, long long ldx, long l
   std::vector<long long> w_off;
   const long long w_total = product_w_layout(t, k, w_off);
   plan->w_elems = w_total;
-  HB_CUDA(cudaMalloc(&plan->w, std::max<long long>(w_total, 1) * sizeof(double)));
+  HB_CUDA(cudaMallocAsync((void **)&plan->w, std::max<long long>(w_total, 1) * sizeof(double),
+                          stream));
   GemmBatch p1, p2;
   append_product(p1, p2, t, op, k, ldx, ldy, ProductSlots{kArena, kX, kY, kW, 0, 0, 0, 0}, w_off,
                  min_depth);
   if (!p1.empty()) gemm_plan_build(plan->phase1, p1, default_shape(op, k, 1), true, stream);
   if (!p2.empty()) gemm_plan_build(plan->phase2, p2, default_shape(op, k, 2), false, stream);
+  HB_CUDA(cudaStreamSynchronize(stream));   // W may be used on any stream from here
   auto &ref = *plan;
   t.plans[key] = std::move(plan);
   return ref;

@@ -353,7 +353,7 @@ T *upload_tmp(const std::vector<T> &v, cudaStream_t s) {
   T *d = nullptr;
   HB_CUDA(cudaMallocAsync((void **)&d, sizeof(T) * std::max<size_t>(v.size(), 1), s));
   if (!v.empty())
-    HB_CUDA(cudaMemcpyAsync(d, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, s));
+    h2d_async(d, v.data(), sizeof(T) * v.size(), s);
   return d;
 }
 
@@ -568,8 +568,9 @@ SolvePlan &solve_plan(HodlrFactor &f, int k, long long ldb, long long ldx, cudaS
     build_plan(*P->cz.back(), L.cz, kShapeCz, true, s);     // K = q: split near the root
     build_plan(*P->wx.back(), L.wx, kShapeWx, false, s);
   }
-  HB_CUDA(cudaMalloc(&P->T, sizeof(double) * std::max<long long>(scratch, 1)));
-  HB_CUDA(cudaMalloc(&P->Z, sizeof(double) * std::max<long long>(scratch, 1)));
+  HB_CUDA(cudaMallocAsync((void **)&P->T, sizeof(double) * std::max<long long>(scratch, 1), s));
+  HB_CUDA(cudaMallocAsync((void **)&P->Z, sizeof(double) * std::max<long long>(scratch, 1), s));
+  HB_CUDA(cudaStreamSynchronize(s));
   auto &ref = *P;
   f.plans[key] = std::move(P);
   return ref;
@@ -612,7 +613,7 @@ std::unique_ptr<HodlrFactor> hodlr_factorize(std::shared_ptr<DeviceTree> tp, cud
       f->q[node_index(d, j)] = q;
       total += align_up((long long)q * q);
     }
-  HB_CUDA(cudaMalloc(&f->buf, sizeof(double) * std::max<long long>(total, 1)));
+  HB_CUDA(cudaMallocAsync((void **)&f->buf, sizeof(double) * std::max<long long>(total, 1), s));
   HB_CUDA(cudaMemsetAsync(f->buf, 0, sizeof(double) * std::max<long long>(total, 1), s));
   int *d_status = nullptr;
   HB_CUDA(cudaMallocAsync((void **)&d_status, sizeof(int), s));

@@ -52,9 +52,11 @@ const char *hodlr_b200_last_error(void);
  *       4 from 128 columns), 1 one piece, n that many
  *   matvec_kernels (1): one right-hand side by the dedicated matvec kernels;
  *       0 = the GEMM engine
- *   pool_keep (1): freed stream-ordered scratch and tree arenas stay mapped in
- *       the device's default memory pool (release threshold unlimited); set
- *       0 before the library's first call on a device to leave that pool alone
+ *   pool_keep (1): freed tree arenas and small stream-ordered scratch stay
+ *       mapped in the device's default memory pool (release threshold
+ *       unlimited), scratch of 32 MiB or more in a pool of the library's own
+ *       (up to half of the device's memory); set 0 before the library's first
+ *       call on a device to leave the default pool alone and keep no scratch
  *   learned_ranks (0): size each sketch from the rank model (fallback to
  *       adaptive growth per block)
  *   learned_margin (0.1), learned_extra (40), learned_eta (1.0): one-shot width
