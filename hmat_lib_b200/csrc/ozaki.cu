@@ -4,8 +4,9 @@
 // Persistent kernel, one CTA of ten warps per SM, each taking the run of
 // tiles the host schedule gave it (ozaki_schedule):
 //   warp 0               producer: per K-block the A block (all S slices of
-//                        128 lines) and the B block, each as 1-8 bulk copies
-//                        issued by as many lanes, into a six-stage ring,
+//                        128 lines, or of the lines that hold rows) and the
+//                        B block, each as 1-8 bulk copies issued by as many
+//                        lanes, into a six-stage ring,
 //                        completion on full[stage]; the next tile's
 //                        descriptors are fetched while a tile streams;
 //   warp 1 (one thread)  MMA issuer: per K-block the S(S+1)/2 slice products
@@ -125,6 +126,10 @@ ozaki_gemm_kernel(const OzSeg *__restrict__ segs, const OzTile *__restrict__ til
       bool next_segs = !more;
       const uint32_t bbytes = (uint32_t)oz_bblock(T.nw);
       const uint32_t ca = (uint32_t)kOzABlock / split, cb = bbytes / split;
+      // a tile of fewer rows copies, slice by slice, only the 8-row groups
+      // that hold some; what the others leave in the stage ends in rows that
+      // are not stored
+      const uint32_t abytes = (uint32_t)((T.rows + 7) / 8) * (8 * kOzKBlock);
       for (int q = 0; q < T.nseg && !stop; ++q) {
         const uint8_t *ga = (const uint8_t *)__shfl_sync(0xffffffffu, (unsigned long long)Gl.a, q);
         const uint8_t *gb = (const uint8_t *)__shfl_sync(0xffffffffu, (unsigned long long)Gl.b, q);
@@ -142,14 +147,20 @@ ozaki_gemm_kernel(const OzSeg *__restrict__ segs, const OzTile *__restrict__ til
             break;
           }
           uint8_t *dst = sm + st * kStageBytes;
-          if (lane == 0) umma::mbar_expect_tx(&full[st], (uint32_t)kOzABlock + bbytes);
+          if (lane == 0)
+            umma::mbar_expect_tx(&full[st], (uint32_t)kOzSlices * abytes + bbytes);
           __syncwarp();
-          if (lane < split) {
-            umma::bulk_g2s(dst + lane * ca, ga + (long long)kb * kOzABlock + lane * ca, ca,
-                           &full[st]);
+          const uint8_t *gak = ga + (long long)kb * kOzABlock;
+          if (abytes < (uint32_t)kSliceBytesA) {
+            if (lane < kOzSlices)
+              umma::bulk_g2s(dst + lane * kSliceBytesA, gak + lane * kSliceBytesA, abytes,
+                             &full[st]);
+          } else if (lane < split) {
+            umma::bulk_g2s(dst + lane * ca, gak + lane * ca, ca, &full[st]);
+          }
+          if (lane < split)
             umma::bulk_g2s(dst + kOzABlock + lane * cb, gb + (long long)kb * bbytes + lane * cb,
                            cb, &full[st]);
-          }
           ++g;
           if (!next_segs) {
             if (lane < Tn.nseg) Gn = segs[Tn.seg0 + lane];
@@ -336,6 +347,13 @@ __device__ __forceinline__ int find_job(const Job *jobs, int njobs, long long it
   return lo;
 }
 
+// The job of the next item, `at` being the job of an earlier one.
+template <class Job>
+__device__ __forceinline__ int next_job(const Job *jobs, int njobs, int at, long long item) {
+  while (at + 1 < njobs && jobs[at + 1].item0 <= item) ++at;
+  return at;
+}
+
 constexpr int kMaxChunkK = 1024;   // K values per warp item, K-contiguous lines
 constexpr int kMaxChunkL = 16;     // K values per warp item, line-contiguous (32 lines)
 constexpr int kTileLines = 32;     // shared-memory transpose tile: lines x K values
@@ -439,24 +457,25 @@ __device__ __forceinline__ void slice16(const double (&y0)[16], int ex, uint8_t 
 
 // Line-contiguous sources: one item = 16 consecutive K positions of one
 // line; lines vary fastest, so loads are coalesced and eight neighbouring
-// items fill one 128-byte core matrix.
+// items fill one 128-byte core matrix.  A block takes a contiguous run of items
+// (one search of the job list per thread).
 __global__ void slice_lines_kernel(const SliceJob *__restrict__ jobs, int njobs, long long items,
                                    const double *xbase) {
-  for (long long it = blockIdx.x * (long long)blockDim.x + threadIdx.x; it < items;
-       it += (long long)gridDim.x * blockDim.x) {
-    const SliceJob &J = jobs[find_job(jobs, njobs, it)];
+  const long long it1 = items * (blockIdx.x + 1) / gridDim.x;
+  int job = -1;
+  for (long long it = items * blockIdx.x / gridDim.x + threadIdx.x; it < it1; it += blockDim.x) {
+    job = job < 0 ? find_job(jobs, njobs, it) : next_job(jobs, njobs, job, it);
+    const SliceJob &J = jobs[job];
     const double *src = J.src ? J.src : xbase;
     const long long local = it - J.item0;
-    const int L = J.ntiles * J.R;
-    const int line = (int)(local % L), c16 = (int)(local / L);
-    const bool live = line < J.lines;
-    const int ex = live ? scale_exponent(J.maxabs[line]) : 0;
-    if (J.exp_out && c16 == 0 && live) J.exp_out[line] = ex;
+    const int line = (int)(local % J.lines), c16 = (int)(local / J.lines);
+    const int ex = scale_exponent(J.maxabs[line]);
+    if (J.exp_out && c16 == 0) J.exp_out[line] = ex;
     double y[16];
 #pragma unroll
     for (int x = 0; x < 16; ++x) {
       const int k = c16 * 16 + x;
-      y[x] = (live && k < J.K) ? src[(long long)line * J.s_line + (long long)k * J.s_k] : 0.0;
+      y[x] = k < J.K ? src[(long long)line * J.s_line + (long long)k * J.s_k] : 0.0;
     }
     const int t = line / J.R, lr = line % J.R;
     slice16(y, ex, J.dst + (long long)t * J.tile_stride +
@@ -479,56 +498,91 @@ __device__ __forceinline__ void cp_async_wait_prev() {
   asm volatile("cp.async.wait_group 1;\n" ::: "memory");
 }
 
-// Stages block item `it` (32 lines x 64 K values) of a K-contiguous slice
-// batch into `buf` with asynchronous copies (zeros outside the source).
-__device__ __forceinline__ void stage_kcontig(const SliceJob *__restrict__ jobs, int njobs,
-                                              long long it, const double *xbase,
-                                              double (*buf)[kTileK + 1]) {
-  const SliceJob &J = jobs[find_job(jobs, njobs, it)];
+// 16-byte asynchronous copy of which `bytes` (0, 8 or 16) are read, the rest
+// zeros; both addresses 16-byte aligned.
+__device__ __forceinline__ void cp_async16z(void *smem, const void *gmem, int bytes) {
+  const uint32_t sa = (uint32_t)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sa), "l"(gmem), "r"(bytes)
+               : "memory");
+}
+
+// Row pitch of a staged tile: 16-byte reads of eight lanes, one per line, hit
+// every bank once.
+constexpr int kTilePitch = kTileK + 2;
+
+// Stages block item `it` (32 lines x 64 K values) of job J of a K-contiguous
+// slice batch into `buf` with asynchronous copies (zeros outside the source),
+// 16 bytes each where the source is aligned.
+__device__ __forceinline__ void stage_kcontig(const SliceJob &J, long long it, const double *xbase,
+                                              double (*buf)[kTilePitch]) {
   const double *src = J.src ? J.src : xbase;
   const long long local = it - J.item0;
   const int Kw = J.nkb * kOzKBlock;
   const int nkt = (Kw + kTileK - 1) / kTileK;
   const int line0 = (int)(local / nkt) * kTileLines, k0 = (int)(local % nkt) * kTileK;
-  for (int idx = threadIdx.x; idx < kTileLines * kTileK; idx += blockDim.x) {
-    const int l = idx / kTileK, kk = idx % kTileK;
-    const int line = line0 + l, k = k0 + kk;
-    const bool in = line < J.lines && k < J.K;
-    cp_async8z(&buf[l][kk], in ? src + (long long)line * J.s_line + k : src, in);
+  if (((J.s_line & 1) | (int)((uintptr_t)src & 15)) == 0) {
+    for (int idx = threadIdx.x; idx < kTileLines * kTileK / 2; idx += blockDim.x) {
+      const int l = idx / (kTileK / 2), kk = 2 * (idx % (kTileK / 2));
+      const int line = line0 + l, take = line < J.lines ? min(2, max(0, J.K - (k0 + kk))) : 0;
+      cp_async16z(&buf[l][kk], take > 0 ? src + (long long)line * J.s_line + k0 + kk : src, 8 * take);
+    }
+  } else {
+    for (int idx = threadIdx.x; idx < kTileLines * kTileK; idx += blockDim.x) {
+      const int l = idx / kTileK, kk = idx % kTileK;
+      const int line = line0 + l, k = k0 + kk;
+      const bool in = line < J.lines && k < J.K;
+      cp_async8z(&buf[l][kk], in ? src + (long long)line * J.s_line + k : src, in);
+    }
   }
 }
 
 // K-contiguous sources (s_k = 1): one block item = 32 lines x 64 K values,
 // brought into shared memory with coalesced asynchronous row copies (the next
 // item's copies in flight while the current one is sliced, two buffers),
-// then sliced 16 K values per thread.
+// then sliced 16 K values per thread.  A block takes a contiguous run of items
+// and steps through the job list.  Bound by HBM (8 bytes read, 6 written per
+// value) and, close behind, by some 30 integer instructions per value.
+// X of n = 32768, k = 256 (117 MB): 33 -> 27 us.  X of 96 trees (n 1024 to
+// 8192, k 16 to 128), 128 lines a tile whatever k was: 204 -> 93 us.
 __global__ void __launch_bounds__(kSliceThreads) slice_kcontig_kernel(const SliceJob *__restrict__ jobs,
                                                             int njobs, long long items,
                                                             const double *xbase) {
-  __shared__ double buf[2][kTileLines][kTileK + 1];
+  __shared__ __align__(16) double buf[2][kTileLines][kTilePitch];
   const int tid = threadIdx.x;
-  long long it = blockIdx.x;
-  if (it < items) stage_kcontig(jobs, njobs, it, xbase, buf[0]);
+  long long it = items * blockIdx.x / gridDim.x;
+  const long long it1 = items * (blockIdx.x + 1) / gridDim.x;
+  int job = 0, ahead = 0;          // jobs of this item and of the one being staged
+  if (it < it1) {
+    job = ahead = find_job(jobs, njobs, it);
+    stage_kcontig(jobs[ahead], it, xbase, buf[0]);
+  }
   cp_async_commit_group();
-  for (int b = 0; it < items; it += gridDim.x, b ^= 1) {
-    if (it + gridDim.x < items) stage_kcontig(jobs, njobs, it + gridDim.x, xbase, buf[b ^ 1]);
+  for (int b = 0; it < it1; ++it, b ^= 1) {
+    if (it + 1 < it1) {
+      ahead = next_job(jobs, njobs, ahead, it + 1);
+      stage_kcontig(jobs[ahead], it + 1, xbase, buf[b ^ 1]);
+    }
     cp_async_commit_group();
     cp_async_wait_prev();            // this item's group has landed
     __syncthreads();
-    const SliceJob &J = jobs[find_job(jobs, njobs, it)];
+    job = next_job(jobs, njobs, job, it);
+    const SliceJob &J = jobs[job];
     const long long local = it - J.item0;
     const int Kw = J.nkb * kOzKBlock;                   // K positions written
     const int nkt = (Kw + kTileK - 1) / kTileK;
     const int line0 = (int)(local / nkt) * kTileLines, k0 = (int)(local % nkt) * kTileK;
     const int l = tid % kTileLines, c = tid / kTileLines;   // kTileK / 16 chunks
     const int line = line0 + l, k = k0 + c * 16;
-    if (line < J.ntiles * J.R && k < Kw) {
-      const bool live = line < J.lines;
-      const int ex = live ? scale_exponent(J.maxabs[line]) : 0;
-      if (J.exp_out && k == 0 && live) J.exp_out[line] = ex;
+    if (line < J.lines && k < Kw) {
+      const int ex = scale_exponent(J.maxabs[line]);
+      if (J.exp_out && k == 0) J.exp_out[line] = ex;
       double y[16];
 #pragma unroll
-      for (int x = 0; x < 16; ++x) y[x] = buf[b][l][c * 16 + x];
+      for (int x = 0; x < 16; x += 2) {
+        const double2 v = *reinterpret_cast<const double2 *>(&buf[b][l][c * 16 + x]);
+        y[x] = v.x;
+        y[x + 1] = v.y;
+      }
       const int t = line / J.R, lr = line % J.R;
       slice16(y, ex, J.dst + (long long)t * J.tile_stride +
                          oz_offset(J.R, 0, lr, J.kb0 * kOzKBlock + k), J.R);
@@ -661,10 +715,9 @@ SliceBatch ozaki_slice_batch(std::vector<SliceJob> jobs, cudaStream_t stream) {
     HB_REQUIRE(j.R % 8 == 0 && j.R >= 8, INPUT_ERROR, "slice tile lines");
     HB_REQUIRE((j.s_k == 1) == b.kcontig, INPUT_ERROR, "mixed slice job kinds in one batch");
     j.item0 = b.items;
-    const long long L = (long long)j.ntiles * j.R;
-    b.items += b.kcontig ? ((L + kTileLines - 1) / kTileLines) *
+    b.items += b.kcontig ? (long long)((j.lines + kTileLines - 1) / kTileLines) *
                                ((j.nkb * kOzKBlock + kTileK - 1) / kTileK)
-                         : L * j.nkb * 2;
+                         : (long long)j.lines * j.nkb * 2;
   }
   b.n = (int)jobs.size();
   if (b.n) {

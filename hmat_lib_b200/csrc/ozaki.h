@@ -103,8 +103,9 @@ struct MaxJob {
 };
 
 // Scales every line by its exponent (from maxabs[line]) and writes the int8
-// slices in the blocked layout: lines [0, ntiles R) (zero past `lines`),
-// K-blocks [kb0, kb0 + nkb) of each tile (zero past K).  exp_out, if set,
+// slices in the blocked layout: lines [0, lines) of the ntiles R of its tiles
+// (the others stay as they are: they only reach rows and columns of a product
+// that are not stored), K-blocks [kb0, kb0 + nkb) of each tile (zero past K).  exp_out, if set,
 // receives the exponent of every line.
 struct SliceJob {
   const double *src;
