@@ -141,9 +141,8 @@ std::unique_ptr<GemmPlan> tune_phase(const GemmBatch &batch, int phase, ProdOp o
   GemmBases b{};
   for (int i = 0; i < kGemmBases; ++i) b.p[i] = P.base;
   for (const Cand &c : cands) {
-    GemmBatch copy = batch;
     auto plan = std::make_unique<GemmPlan>();
-    gemm_plan_build(*plan, copy, c.shape, c.split, s);
+    gemm_plan_build(*plan, batch, c.shape, c.split ? KSplit::All : KSplit::None, s);
     if (plan->ntiles == 0) continue;
     float ms = 0.f;
     if (cands.size() > 1) ms = time_best([&] { gemm_plan_run(*plan, b, s); }, s);
@@ -151,7 +150,7 @@ std::unique_ptr<GemmPlan> tune_phase(const GemmBatch &batch, int phase, ProdOp o
       best_ms = ms;
       best = std::move(plan);
       best_desc = std::string("phase") + std::to_string(phase) + " " + shape_name(c.shape) +
-                  (best->any_split ? " split" : " nosplit") +
+                  (best->nscale > 0 ? " split" : " nosplit") +
                   (cands.size() > 1 ? " " + std::to_string(ms) + " ms" : "");
     }
   }

@@ -2,7 +2,7 @@
 //
 // Two kernels (option gemm_f64_engine): the FP64 tensor-core (DMMA) kernel
 // (default, below), and a CUDA-core DFMA kernel: 256 threads, a BM x BN output tile per CTA
-// (128 x 64, 64 x 128, 32 x 128 or 32 x 256), K advanced 16 at a time through a two-stage
+// (128 x 64, 64 x 128, 64 x 64, 32 x 128 or 32 x 256), K advanced 16 at a time through a two-stage
 // cp.async pipeline (8-byte copies with zero fill, so any leading dimension
 // and any offset work), 32 accumulators per thread, operands read from shared
 // memory as double2.  FP64 has no tcgen05 path; this is the FP64 roofline
@@ -230,7 +230,7 @@ gemm_f64_kernel(const GemmSeg *__restrict__ segs, const GemmProb *__restrict__ p
       if (n >= P.N) continue;
       double *c = C + m + (long long)n * P.ldc;
       const double v = P.alpha * acc[i][j];
-      if (P.split > 1)
+      if (tile.atomic)
         atomicAdd(c, v);
       else
         *c = (P.beta == 0.0) ? v : v + P.beta * (*c);
@@ -255,9 +255,14 @@ gemm_f64_kernel(const GemmSeg *__restrict__ segs, const GemmProb *__restrict__ p
 // range are zero-filled.  The ring is as deep as two CTAs per SM allow (2 to
 // 4 stages).  Ranks and leaf sizes are rarely multiples of a tile, so at an
 // edge a warp issues only the 8 x 8 MMA tiles and the 4-deep K steps that hold
-// something, and a segment's pointers are kept in registers until it ends:
-// H X at n = 32768, k = 256 (ranks 38 to 349) 1637 -> 1512 us, H x H at
-// n = 16384 (many products of 5 to 40 columns) 3.44 -> 2.90 ms.
+// something, and a segment's pointers are kept in registers until it ends.
+// The MMA loop from shared memory alone reaches 36 of 37 TFLOP/s; what is lost
+// is the loader's instructions (nine per MMA before the three copy paths of
+// stage_operand and the per-layout MMA loops, under five now), during which the
+// warps of a CTA issue no MMAs.  H X at n = 32768, k = 256 (ranks 38 to 349):
+// 1640 us without any of this, 1512 us without MMAs on padding, 1370 us now
+// (28.7 TFLOP/s; cuBLAS DGEMM 35.5); H x H at n = 16384 (many products of 5 to
+// 40 columns) 3.44, 2.90, 2.47 ms.
 template <int BM, int BN, int BK>
 struct MmaSmem {
   static constexpr int LDKM = BM + 4;      // [k][m] layout
@@ -271,57 +276,76 @@ struct MmaSmem {
   static constexpr size_t bytes = sizeof(double) * STAGES * STAGE;
 };
 
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem, int src_bytes) {
+__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem));
+}
+// The same, or sixteen zero bytes (nothing is read then).
+__device__ __forceinline__ void cp_async16z(void *smem, const void *gmem, bool pred) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem),
-               "r"(src_bytes));
+               "r"(pred ? 16 : 0));
 }
 
 // One operand tile of ROWS lines (M or N side) x BK into stage memory, by
 // cp.async.  `src` is element (line 0, K index 0) of the stage; K-contiguous
 // operands go to [line][k], the others to [k][line].  Lines past `nlines` and
 // K values past `kin` are zero-filled.  A thread's copies differ by a constant
-// step in both memories, so a copy costs an addition, a comparison and the
-// copy itself.
+// step in both memories.  Three ways, uniform over the CTA: the whole tile by
+// plain 16-byte copies (an addition and the copy each), an edge at an even
+// line or K value by 16-byte copies that read all or nothing, any other by
+// 8-byte ones (a copy of a variable number of bytes compiles to some 70
+// instructions).
 template <int ROWS, int BK>
 __device__ __forceinline__ void stage_operand(double *dst, const double *src, int ld, bool kcontig,
                                               bool vec, int nlines, int kin) {
   const int tid = threadIdx.x;
+  const bool full = nlines >= ROWS && kin == BK;
   if (kcontig) {
     constexpr int CH = BK / 2, LS = kThreads / CH;   // 16-byte chunks per line, lines per pass
+    static_assert(ROWS % LS == 0, "whole passes");
     const int l0 = tid / CH, k = 2 * (tid % CH);
-    const int nk = min(2, max(0, kin - k));
     double *d = dst + l0 * (BK + 4) + k;
     const double *q = src + (long long)l0 * ld + k;
     const long long step = (long long)LS * ld;
+    if (vec && full) {
 #pragma unroll
-    for (int i = 0; i < (ROWS + LS - 1) / LS; ++i) {
-      if (ROWS % LS != 0 && l0 + i * LS >= ROWS) break;
-      const int take = l0 + i * LS < nlines ? nk : 0;
-      const double *from = take > 0 ? q + i * step : src;
-      if (vec) {
-        cp_async16(d + i * LS * (BK + 4), from, 8 * take);
-      } else {
-        cp_async8(d + i * LS * (BK + 4), from, take > 0);
-        cp_async8(d + i * LS * (BK + 4) + 1, take > 1 ? from + 1 : src, take > 1);
+      for (int i = 0; i < ROWS / LS; ++i, q += step) cp_async16(d + i * LS * (BK + 4), q);
+    } else if (vec && (kin & 1) == 0) {
+#pragma unroll
+      for (int i = 0; i < ROWS / LS; ++i, q += step) {
+        const bool in = k < kin && l0 + i * LS < nlines;
+        cp_async16z(d + i * LS * (BK + 4), in ? q : src, in);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < ROWS / LS; ++i, q += step) {
+        const bool in = k < kin && l0 + i * LS < nlines, in2 = in && k + 1 < kin;
+        cp_async8(d + i * LS * (BK + 4), in ? q : src, in);
+        cp_async8(d + i * LS * (BK + 4) + 1, in2 ? q + 1 : src, in2);
       }
     }
   } else {
     constexpr int CH = ROWS / 2, KS = kThreads / CH;   // chunks per K value, K values per pass
     const int line = 2 * (tid % CH), k0 = tid / CH;
-    const int nl = min(2, max(0, nlines - line));
     double *d = dst + k0 * (ROWS + 4) + line;
     const double *q = src + (long long)k0 * ld + line;
     const long long step = (long long)KS * ld;
+    if (vec && full) {
 #pragma unroll
-    for (int i = 0; i < BK / KS; ++i) {
-      const int take = k0 + i * KS < kin ? nl : 0;
-      const double *from = take > 0 ? q + i * step : src;
-      if (vec) {
-        cp_async16(d + i * KS * (ROWS + 4), from, 8 * take);
-      } else {
-        cp_async8(d + i * KS * (ROWS + 4), from, take > 0);
-        cp_async8(d + i * KS * (ROWS + 4) + 1, take > 1 ? from + 1 : src, take > 1);
+      for (int i = 0; i < BK / KS; ++i, q += step) cp_async16(d + i * KS * (ROWS + 4), q);
+    } else if (vec && ((nlines & 1) == 0 || nlines >= ROWS)) {
+#pragma unroll
+      for (int i = 0; i < BK / KS; ++i, q += step) {
+        const bool in = line < nlines && k0 + i * KS < kin;
+        cp_async16z(d + i * KS * (ROWS + 4), in ? q : src, in);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < BK / KS; ++i, q += step) {
+        const bool in = line < nlines && k0 + i * KS < kin, in2 = in && line + 1 < nlines;
+        cp_async8(d + i * KS * (ROWS + 4), in ? q : src, in);
+        cp_async8(d + i * KS * (ROWS + 4) + 1, in2 ? q + 1 : src, in2);
       }
     }
   }
@@ -349,6 +373,26 @@ __device__ __forceinline__ void stage_generated(double *dst, const KernelSpec &g
   }
 }
 
+// A whole stage's MMAs of one warp: ap, bp are the lane's first fragment
+// elements, the steps to the next line and K value known at compile time (one
+// copy of the loop per layout: every fragment load has a constant offset).
+template <int MT, int NT, int BK, int A_LINE, int A_K, int B_LINE, int B_K>
+__device__ __forceinline__ void stage_mmas(double (&acc)[MT][NT][2], const double *ap,
+                                           const double *bp) {
+#pragma unroll
+  for (int k4 = 0; k4 < BK / 4; ++k4) {
+    double a[MT], b[NT];
+#pragma unroll
+    for (int i = 0; i < MT; ++i) a[i] = ap[8 * i * A_LINE + 4 * k4 * A_K];
+#pragma unroll
+    for (int j = 0; j < NT; ++j) b[j] = bp[8 * j * B_LINE + 4 * k4 * B_K];
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+      for (int j = 0; j < NT; ++j) dmma884(acc[i][j], a[i], b[j]);
+  }
+}
+
 template <int BM, int BN, int WM, int WN, int BK>
 __global__ void __launch_bounds__(kThreads, 2)
 gemm_f64_mma_kernel(const GemmSeg *__restrict__ segs, const GemmProb *__restrict__ probs,
@@ -364,7 +408,22 @@ gemm_f64_mma_kernel(const GemmSeg *__restrict__ segs, const GemmProb *__restrict
   const GemmProb P = probs[tile.prob];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
-  const int wm0 = (warp / WARPS_N) * WM, wn0 = (warp % WARPS_N) * WN;
+  // Warps w and w + 4 share an SM sub-partition and its tensor core.  At an
+  // edge whole rows or columns of warps are idle, so warp rows (four of them)
+  // or columns go to different sub-partitions, and with two warp rows the
+  // second is turned by two.
+  int wrow, wcol;
+  if constexpr (WARPS_N == 2) {
+    wrow = warp & 3;
+    wcol = warp >> 2;
+  } else if constexpr (WARPS_N == 4) {
+    wrow = warp >> 2;
+    wcol = (warp + 2 * wrow) & 3;
+  } else {
+    wrow = warp / WARPS_N;
+    wcol = warp % WARPS_N;
+  }
+  const int wm0 = wrow * WM, wn0 = wcol * WN;
   const int seg_end = P.seg0 + P.nseg;
   // 8-row and 8-column MMA tiles of this warp that lie inside the problem
   const int mt_in = max(0, min(MT, (P.M - tile.m0 - wm0 + 7) / 8));
@@ -497,17 +556,11 @@ gemm_f64_mma_kernel(const GemmSeg *__restrict__ segs, const GemmProb *__restrict
     const double *bp = bs + (wn0 + g) * b_line_step + t * b_k_step;
     const int kin = min(BK, cit.le - cit.kk);   // K values of this stage
     if (whole && kin == BK) {
-#pragma unroll
-      for (int k4 = 0; k4 < BK / 4; ++k4) {
-        double a[MT], b[NT];
-#pragma unroll
-        for (int i = 0; i < MT; ++i) a[i] = ap[(8 * i) * a_line_step + 4 * k4 * a_k_step];
-#pragma unroll
-        for (int j = 0; j < NT; ++j) b[j] = bp[(8 * j) * b_line_step + 4 * k4 * b_k_step];
-#pragma unroll
-        for (int i = 0; i < MT; ++i)
-#pragma unroll
-          for (int j = 0; j < NT; ++j) dmma884(acc[i][j], a[i], b[j]);
+      switch (l) {
+        case 0: stage_mmas<MT, NT, BK, 1, SM::LDKM, 1, SM::LDKN>(acc, ap, bp); break;
+        case 1: stage_mmas<MT, NT, BK, SM::LDK, 1, 1, SM::LDKN>(acc, ap, bp); break;
+        case 2: stage_mmas<MT, NT, BK, 1, SM::LDKM, SM::LDK, 1>(acc, ap, bp); break;
+        default: stage_mmas<MT, NT, BK, SM::LDK, 1, SM::LDK, 1>(acc, ap, bp); break;
       }
     } else if (mt_in > 0 && nt_in > 0) {
       // edge of the problem or of a K range: only the MMA tiles and 4-deep
@@ -545,7 +598,7 @@ gemm_f64_mma_kernel(const GemmSeg *__restrict__ segs, const GemmProb *__restrict
         if (n >= P.N) continue;
         double *c = C + m + (long long)n * P.ldc;
         const double v = P.alpha * acc[i][j][h];
-        if (P.split > 1)
+        if (tile.atomic)
           atomicAdd(c, v);
         else
           *c = (P.beta == 0.0) ? v : v + P.beta * (*c);
@@ -554,21 +607,19 @@ gemm_f64_mma_kernel(const GemmSeg *__restrict__ segs, const GemmProb *__restrict
   }
 }
 
-// beta pre-pass for problems whose tiles accumulate with atomics
-__global__ void gemm_scale_c_kernel(const GemmProb *__restrict__ probs, int nprobs,
+// beta pre-pass for the (m, n) tiles that several tiles add to
+__global__ void gemm_scale_c_kernel(const GemmProb *__restrict__ probs,
+                                    const GemmTile *__restrict__ tiles, int bm, int bn,
                                     GemmBases bases) {
-  for (int p = blockIdx.y; p < nprobs; p += gridDim.y) {
-    const GemmProb P = probs[p];
-    if (P.split <= 1) continue;
-    double *C = base_ptr(bases, P.cbase) + P.c_off;
-    const long long total = (long long)P.M * P.N;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-         e += (long long)gridDim.x * blockDim.x) {
-      const long long m = e % P.M, n = e / P.M;
-      double *c = C + m + n * P.ldc;
-      *c = (P.beta == 0.0) ? 0.0 : P.beta * (*c);
+  const GemmTile T = tiles[blockIdx.x];
+  const GemmProb P = probs[T.prob];
+  double *C = base_ptr(bases, P.cbase) + P.c_off;
+  const int rows = min(bm, P.M - T.m0), cols = min(bn, P.N - T.n0);
+  for (int c = threadIdx.x >> 5; c < cols; c += blockDim.x >> 5)
+    for (int r = threadIdx.x & 31; r < rows; r += 32) {
+      double *p = C + T.m0 + r + (long long)(T.n0 + c) * P.ldc;
+      *p = (P.beta == 0.0) ? 0.0 : P.beta * (*p);
     }
-  }
 }
 
 template <int BM, int BN, int WM, int WN>
@@ -622,7 +673,7 @@ GemmPlan::~GemmPlan() {
     cudaFree(dev);
 }
 
-void gemm_plan_build(GemmPlan &plan, GemmBatch &batch, TileShape shape, bool allow_split,
+void gemm_plan_build(GemmPlan &plan, const GemmBatch &batch, TileShape shape, KSplit ksplit,
                      cudaStream_t stream, bool transient) {
   const auto t_start = std::chrono::steady_clock::now();
   struct Clock {
@@ -635,7 +686,7 @@ void gemm_plan_build(GemmPlan &plan, GemmBatch &batch, TileShape shape, bool all
   const int BM = tile_rows(shape);
   const int BN = tile_cols(shape);
   plan.shape = shape;
-  auto &probs = batch.probs;
+  const auto &probs = batch.probs;
   std::vector<long long> ktot(probs.size(), 0);
   long long base_tiles = 0;
   double work = 0.0;
@@ -649,15 +700,15 @@ void gemm_plan_build(GemmPlan &plan, GemmBatch &batch, TileShape shape, bool all
   }
   const long long target = 4LL * num_sms();
   // per problem: its K split and the K length of its tiles
-  plan.any_split = false;
   std::vector<long long> chunk_of(probs.size(), 0);
+  std::vector<int> split_of(probs.size(), 1);
   for (size_t p = 0; p < probs.size(); ++p) {
-    GemmProb &P = probs[p];
+    const GemmProb &P = probs[p];
     if (P.M <= 0 || P.N <= 0) continue;
     // Split K so that no tile carries much more than an even share of the
     // batch's work (the longest tile bounds the launch), and to fill the GPU.
     long long split = 1;
-    if (allow_split && ktot[p] > 2 * 256) {
+    if (ksplit == KSplit::All && ktot[p] > 2 * 256) {
       const double per_tile = work / (double)target;          // ideal work per tile
       const double mine = (double)std::max<long long>(ktot[p], 1);
       split = (long long)std::ceil(mine / std::max(per_tile, 512.0));
@@ -667,8 +718,7 @@ void gemm_plan_build(GemmPlan &plan, GemmBatch &batch, TileShape shape, bool all
     chunk = (chunk + kBK - 1) / kBK * kBK;
     if (chunk <= 0) chunk = kBK;
     split = std::max<long long>(1, (ktot[p] + chunk - 1) / chunk);
-    P.split = (int)split;
-    if (split > 1) plan.any_split = true;
+    split_of[p] = (int)split;
     chunk_of[p] = split == 1 ? ktot[p] : chunk;
   }
   // tiles of the problems with the longest K ranges first, for load balance
@@ -678,28 +728,66 @@ void gemm_plan_build(GemmPlan &plan, GemmBatch &batch, TileShape shape, bool all
   for (size_t p = 0; p < probs.size(); ++p) order[p] = (int)p;
   std::stable_sort(order.begin(), order.end(),
                    [&](int a, int b) { return chunk_of[a] > chunk_of[b]; });
-  std::vector<GemmTile> tiles;
+  std::vector<GemmTile> tiles, scale;
   tiles.reserve(base_tiles);
   for (int p : order) {
     const GemmProb &P = probs[p];
     if (P.M <= 0 || P.N <= 0) continue;
     const int mt = (P.M + BM - 1) / BM, nt = (P.N + BN - 1) / BN;
     const long long chunk = chunk_of[p];
+    const int split = split_of[p];
     for (int mi = 0; mi < mt; ++mi)
-      for (int ni = 0; ni < nt; ++ni)
-        for (long long si = 0; si < P.split; ++si) {
-          GemmTile t;
-          t.prob = p;
-          t.m0 = mi * BM;
-          t.n0 = ni * BN;
+      for (int ni = 0; ni < nt; ++ni) {
+        GemmTile t{p, mi * BM, ni * BN, 0, 0, split > 1 ? 1 : 0};
+        if (split > 1 && P.beta != 1.0) scale.push_back(t);
+        for (long long si = 0; si < split; ++si) {
           t.k0 = (int)(si * chunk);
-          t.k1 = (int)std::min<long long>(ktot[p], (si + 1) * chunk);
-          if (P.split == 1) t.k1 = (int)ktot[p];
+          t.k1 = split == 1 ? (int)ktot[p] : (int)std::min<long long>(ktot[p], (si + 1) * chunk);
           tiles.push_back(t);
         }
+      }
+  }
+  // A last wave that fills part of the GPU (two CTAs per SM) runs as long as a
+  // full one: its tiles are split along K into the number of parts, each at
+  // least 256 long, whose waves are shortest together (3% for a part's own
+  // start and end).  n = 32768, k = 256: 1024 output tiles of K about 1260,
+  // 3.46 waves, the last 136 in two parts; n = 16384: 512 tiles, 1.73 waves, the
+  // last 216 in four (689 -> 655 us for the whole product).
+  if (ksplit == KSplit::Tail) {
+    const long long slots = 2LL * num_sms(), rest = (long long)tiles.size() % slots;
+    if (rest > 0) {
+      std::vector<GemmTile> tail(tiles.end() - rest, tiles.end());
+      tiles.resize(tiles.size() - rest);
+      int parts = 1;
+      double best = 1.0;
+      for (int q = 2; q <= 8 && 256 * q <= tail.front().k1; ++q) {
+        const double t = (double)((rest * q + slots - 1) / slots) / q + 0.03 * q;
+        if (t < best) {
+          best = t;
+          parts = q;
+        }
+      }
+      for (GemmTile &t : tail) {
+        const long long mine = std::max<long long>(1, std::min<long long>(parts, t.k1 / 256));
+        const long long chunk = (t.k1 / mine + 31) / 32 * 32;
+        if (mine == 1) {
+          tiles.push_back(t);
+          continue;
+        }
+        t.atomic = 1;
+        if (probs[t.prob].beta != 1.0) scale.push_back(t);
+        const int kend = t.k1;
+        for (long long q = 0; q < mine; ++q) {
+          t.k0 = (int)std::min<long long>(kend, q * chunk);
+          t.k1 = q + 1 == mine ? kend : (int)std::min<long long>(kend, (q + 1) * chunk);
+          if (t.k0 < t.k1) tiles.push_back(t);
+        }
+      }
+    }
   }
   plan.ntiles = (int)tiles.size();
-  plan.nprobs = (int)probs.size();
+  plan.nscale = (int)scale.size();
+  tiles.insert(tiles.end(), scale.begin(), scale.end());
   const size_t bs = batch.segs.size() * sizeof(GemmSeg);
   const size_t bp = probs.size() * sizeof(GemmProb);
   const size_t bt = tiles.size() * sizeof(GemmTile);
@@ -732,9 +820,10 @@ void gemm_plan_build(GemmPlan &plan, GemmBatch &batch, TileShape shape, bool all
 
 void gemm_plan_run(const GemmPlan &plan, const GemmBases &bases, cudaStream_t stream) {
   if (plan.ntiles == 0) return;
-  if (plan.any_split) {
-    dim3 grid(64, std::min(plan.nprobs, 1024));
-    gemm_scale_c_kernel<<<grid, 256, 0, stream>>>(plan.probs, plan.nprobs, bases);
+  if (plan.nscale > 0) {
+    gemm_scale_c_kernel<<<plan.nscale, 256, 0, stream>>>(plan.probs, plan.tiles + plan.ntiles,
+                                                         tile_rows(plan.shape),
+                                                         tile_cols(plan.shape), bases);
     HB_LAUNCHED();
   }
   switch (plan.shape) {
@@ -742,14 +831,20 @@ void gemm_plan_run(const GemmPlan &plan, const GemmBases &bases, cudaStream_t st
     case TileShape::M64N128: launch_gemm<64, 128, 32, 32>(plan, bases, stream); break;
     case TileShape::M32N128: launch_gemm<32, 128, 32, 16>(plan, bases, stream); break;
     case TileShape::M32N256: launch_gemm<32, 256, 32, 32>(plan, bases, stream); break;
+    case TileShape::M64N64: launch_gemm<64, 64, 16, 32>(plan, bases, stream); break;
   }
 }
 
 void gemm_f64_run(GemmBatch &batch, const GemmBases &bases, TileShape shape, cudaStream_t stream,
                   bool allow_split) {
   if (batch.empty()) return;
+  if (shape == TileShape::M64N128) {
+    int nmax = 0;
+    for (const GemmProb &P : batch.probs) nmax = std::max(nmax, P.N);
+    if (nmax <= 64) shape = TileShape::M64N64;
+  }
   GemmPlan plan;
-  gemm_plan_build(plan, batch, shape, allow_split, stream, true);
+  gemm_plan_build(plan, batch, shape, allow_split ? KSplit::All : KSplit::None, stream, true);
   gemm_plan_run(plan, bases, stream);
 }
 

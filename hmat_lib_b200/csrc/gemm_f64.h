@@ -5,8 +5,8 @@
 // lets one output tile accumulate a leaf product and every level's low-rank
 // product in registers (one store per output element).  A problem may be
 // split along its concatenated K range into several tiles that add their
-// partial sums with FP64 atomics (C is then pre-scaled by beta in a separate
-// pass of the same launch sequence).
+// partial sums with FP64 atomics (their part of C is then pre-scaled by beta in
+// a separate pass of the same launch sequence).
 //
 // Every pointer is stored as (base slot, element offset) so that a plan --
 // the device copy of the descriptors -- can be reused with new buffers: the
@@ -45,7 +45,6 @@ struct GemmProb {
   int M, N;
   int seg0, nseg;
   int cbase;
-  int split;            // number of K-split tiles per (m, n) tile (1: plain store)
   double alpha, beta;
 };
 
@@ -53,16 +52,20 @@ struct GemmTile {
   int prob;
   int m0, n0;
   int k0, k1;           // range in the problem's concatenated K index
+  int atomic;           // 1: other tiles add to the same part of C
 };
 
 // Output tile per CTA.  The 32-row shapes serve skinny problems (a few rows:
-// the projections V^T X of low-rank blocks).
-enum class TileShape { M128N64 = 0, M64N128 = 1, M32N128 = 2, M32N256 = 3 };
+// the projections V^T X of low-rank blocks), the 64 x 64 shape batches of at
+// most 64 columns.
+enum class TileShape { M128N64 = 0, M64N128 = 1, M32N128 = 2, M32N256 = 3, M64N64 = 4 };
 inline int tile_rows(TileShape t) {
-  return t == TileShape::M128N64 ? 128 : t == TileShape::M64N128 ? 64 : 32;
+  return t == TileShape::M128N64 ? 128
+         : t == TileShape::M64N128 || t == TileShape::M64N64 ? 64 : 32;
 }
 inline int tile_cols(TileShape t) {
-  return t == TileShape::M128N64 ? 64 : t == TileShape::M32N256 ? 256 : 128;
+  return t == TileShape::M128N64 || t == TileShape::M64N64 ? 64
+         : t == TileShape::M32N256 ? 256 : 128;
 }
 
 struct GemmBatch {
@@ -71,7 +74,7 @@ struct GemmBatch {
 
   int add(int cbase, long long c_off, long long ldc, int M, int N, double alpha = 1.0,
           double beta = 0.0) {
-    probs.push_back(GemmProb{c_off, ldc, M, N, (int)segs.size(), 0, cbase, 1, alpha, beta});
+    probs.push_back(GemmProb{c_off, ldc, M, N, (int)segs.size(), 0, cbase, alpha, beta});
     return (int)probs.size() - 1;
   }
   // op(A) is M x K, op(B) is K x N.
@@ -94,28 +97,29 @@ struct GemmBatch {
 struct GemmPlan {
   TileShape shape = TileShape::M128N64;
   int ntiles = 0;
-  int nprobs = 0;
-  bool any_split = false;
+  int nscale = 0;               // (m, n) tiles that several tiles add to and beta != 1
   void *dev = nullptr;          // one allocation holding the three arrays
   bool transient = false;       // dev is stream-ordered (freed with cudaFreeAsync on `stream`)
   cudaStream_t stream = nullptr;
   GemmSeg *segs = nullptr;
   GemmProb *probs = nullptr;
-  GemmTile *tiles = nullptr;
+  GemmTile *tiles = nullptr;    // the tiles, then the nscale ones
   GemmPlan() = default;
   GemmPlan(const GemmPlan &) = delete;
   GemmPlan &operator=(const GemmPlan &) = delete;
   ~GemmPlan();
 };
 
-// Builds the tile list (splitting long K ranges when the batch would not
-// fill the GPU) and uploads it.  A transient plan lives in stream-ordered
+// How gemm_plan_build may split K ranges: not at all, the tiles of a launch's
+// last, partly filled wave, or any long range so that the batch fills the GPU.
+enum class KSplit { None, Tail, All };
+// Builds the tile list and uploads it.  A transient plan lives in stream-ordered
 // memory of `stream` and is released in stream order: no host
 // synchronisation.
-void gemm_plan_build(GemmPlan &plan, GemmBatch &batch, TileShape shape, bool allow_split,
+void gemm_plan_build(GemmPlan &plan, const GemmBatch &batch, TileShape shape, KSplit ksplit,
                      cudaStream_t stream, bool transient = false);
 
-// Launches a plan: the beta pre-pass for split problems, then the GEMM.
+// Launches a plan: the beta pre-pass for split tiles, then the GEMM.
 void gemm_plan_run(const GemmPlan &plan, const GemmBases &bases, cudaStream_t stream);
 
 // FP64 multiply-add work (2 M N K per problem) of every GEMM plan built on
@@ -129,7 +133,8 @@ double &plan_host_ms();
 // tensor-core (DMMA) kernel, 0 the DFMA kernel.
 int gemm_f64_engine();
 
-// One-shot convenience: plan, run, release (stream-ordered).
+// One-shot convenience: plan, run, release (stream-ordered).  A batch of at most
+// 64 columns asked for in 64 x 128 tiles gets 64 x 64 ones.
 void gemm_f64_run(GemmBatch &batch, const GemmBases &bases, TileShape shape, cudaStream_t stream,
                   bool allow_split = true);
 

@@ -498,9 +498,8 @@ GemmBatch leaf_batch(const HodlrFactor &f, int k, long long ldb, long long ldx) 
 }
 
 constexpr TileShape kShapeLeaves = TileShape::M128N64;
-constexpr TileShape kShapeVt = TileShape::M64N128;
-constexpr TileShape kShapeCz = TileShape::M64N128;
 constexpr TileShape kShapeWx = TileShape::M128N64;
+TileShape shape_vt(int k) { return k <= 64 ? TileShape::M64N64 : TileShape::M64N128; }
 
 // One-shot application (factorisation, where k is a level's rank).
 void apply_leaves_once(const HodlrFactor &f, const double *B, long long ldb, double *X,
@@ -516,8 +515,8 @@ void apply_level_once(const HodlrFactor &f, int l, double *X, int k, long long l
   double *T = dev_alloc(tot, s), *Z = dev_alloc(tot, s);
   const GemmBases b = solver_bases(f, X, nullptr, T, Z);
   LevelBatches L = level_batches(f, l, k, ldx);
-  gemm_f64_run(L.vt, b, kShapeVt, s);
-  gemm_f64_run(L.cz, b, kShapeCz, s);
+  gemm_f64_run(L.vt, b, shape_vt(k), s);
+  gemm_f64_run(L.cz, b, shape_vt(k), s);
   gemm_f64_run(L.wx, b, kShapeWx, s, false);
   dev_free(T, s);
   dev_free(Z, s);
@@ -545,7 +544,7 @@ HodlrFactor::~HodlrFactor() {
 namespace {
 
 void build_plan(GemmPlan &plan, GemmBatch &batch, TileShape shape, bool split, cudaStream_t s) {
-  if (!batch.empty()) gemm_plan_build(plan, batch, shape, split, s);
+  if (!batch.empty()) gemm_plan_build(plan, batch, shape, split ? KSplit::All : KSplit::Tail, s);
 }
 
 SolvePlan &solve_plan(HodlrFactor &f, int k, long long ldb, long long ldx, cudaStream_t s) {
@@ -564,8 +563,8 @@ SolvePlan &solve_plan(HodlrFactor &f, int k, long long ldb, long long ldx, cudaS
     P->vt.push_back(std::make_unique<GemmPlan>());
     P->cz.push_back(std::make_unique<GemmPlan>());
     P->wx.push_back(std::make_unique<GemmPlan>());
-    build_plan(*P->vt.back(), L.vt, kShapeVt, true, s);
-    build_plan(*P->cz.back(), L.cz, kShapeCz, true, s);     // K = q: split near the root
+    build_plan(*P->vt.back(), L.vt, shape_vt(k), true, s);
+    build_plan(*P->cz.back(), L.cz, shape_vt(k), true, s);     // K = q: split near the root
     build_plan(*P->wx.back(), L.wx, kShapeWx, false, s);
   }
   HB_CUDA(cudaMallocAsync((void **)&P->T, sizeof(double) * std::max<long long>(scratch, 1), s));
