@@ -127,8 +127,8 @@ constexpr int kFeatCols = 16;   // width of the feature sketch
 // ln(kernel length) and five log ratios of the sketch's singular values.
 std::vector<float> block_features(const std::vector<SketchBlock> &sk,
                                   const double *d_A, int aslot,
-                                  const KernelSpec &gen, unsigned long long seed,
-                                  cudaStream_t stream) {
+                                  const KernelSpec &gen, double kernel_length,
+                                  unsigned long long seed, cudaStream_t stream) {
   const int nsk = (int)sk.size();
   std::vector<float> f((size_t)nsk * kRankIn, 0.f);
   if (nsk == 0) return f;
@@ -212,10 +212,10 @@ std::vector<float> block_features(const std::vector<SketchBlock> &sk,
   }
   cudaFreeAsync(d_rank, stream);
   dev_free(w, stream);
-  // kernel length scale: option kernel_length, else (matrix-free build) the
+  // kernel length scale: option kernel_length, else (build from points) the
   // length of the kernel being compressed, else unknown (feature 0)
   double length = option("kernel_length", 0.0);
-  if (length <= 0.0 && aslot == (int)kGenSlot) length = gen.length;
+  if (length <= 0.0) length = kernel_length;
   for (int i = 0; i < nsk; ++i) {
     const SketchBlock &S = sk[i];
     float *row = &f[(size_t)i * kRankIn];
@@ -243,12 +243,13 @@ namespace {
 // twice its predicted one-shot width -- so that a build whose ranks are small never reserves (and
 // maps) scratch for wide sketches; a block that fills it moves its sketch
 // into scratch of twice the width while the device memory allows (grow())
-// and carries on.
+// and carries on.  `formed`: the input is a kernel matrix formed for this
+// build (build_batch).
 std::vector<std::shared_ptr<DeviceTree>> build_attempt(
     const std::vector<BuildInput> &in, double tol, cudaStream_t stream, int *svd_status,
-    BuildStats *stats, const KernelSpec *gen, std::chrono::steady_clock::time_point t0) {
+    BuildStats *stats, const KernelSpec *gen, const KernelSpec *formed,
+    std::chrono::steady_clock::time_point t0) {
   HB_REQUIRE(!in.empty(), INPUT_ERROR, "build: no tree to build");
-  HB_REQUIRE(!gen || in.size() == 1, INPUT_ERROR, "a matrix-free build takes one tree");
   *svd_status = SUCCESS;
   // Every off-diagonal block of every tree, flattened.  The inputs are
   // addressed as element offsets from the lowest input address, so one GEMM
@@ -319,7 +320,7 @@ std::vector<std::shared_ptr<DeviceTree>> build_attempt(
   // FP64 GEMMs.
   std::unique_ptr<SketchMixed> smix;
   std::vector<int> mix_of(sketched.size(), -1);
-  if (!gen && option("build_precision", 0.0) == 1.0) {
+  if (!gen && !formed && option("build_precision", 0.0) == 1.0) {
     std::vector<SketchMixedBlock> mb;
     for (size_t si = 0; si < sketched.size(); ++si) {
       const Blk &X = blk[sketched[si]];
@@ -365,7 +366,8 @@ std::vector<std::shared_ptr<DeviceTree>> build_attempt(
   for (SketchBlock &S : sk) S.first_w = std::min(w_first, S.cap);
   const auto tf0 = std::chrono::steady_clock::now();
   if (record && !sk.empty()) {
-    feats = block_features(sk, d_A, aslot, gspec, seed, stream);
+    feats = block_features(sk, d_A, aslot, gspec,
+                           gen ? gen->length : formed ? formed->length : 0.0, seed, stream);
     if (have_model) {
       const int nsk = (int)sk.size();
       float *dbuf = nullptr;
@@ -1030,7 +1032,38 @@ std::vector<std::shared_ptr<DeviceTree>> build_batch(const std::vector<BuildInpu
   const auto t0 = std::chrono::steady_clock::now();
   gemm_flops_counter() = 0.0;
   plan_host_ms() = 0.0;
-  return build_attempt(in, tol, stream, svd_status, stats, gen, t0);
+  HB_REQUIRE(!gen || in.size() == 1, INPUT_ERROR, "a matrix-free build takes one tree");
+  // A kernel matrix that fits a small share of the memory at hand (option
+  // kernel_form_frac) is formed once: the sketch rounds read each entry twice
+  // a round, and computing it (a square root, an exponential, a division) in
+  // the GEMM's loader costs several times the multiply-adds it feeds.  n = 8192,
+  // 3D, 25 rounds: 99 ms of rounds with generated operands, 70 with a formed matrix.
+  if (gen && !in[0].g.blocks.empty()) {
+    const int n = in[0].g.n;
+    const double bytes = 8.0 * (double)n * n;
+    if (bytes <= option("kernel_form_frac", 0.0625) * device_avail_bytes()) {
+      struct Matrix {
+        double *p;
+        cudaStream_t s;
+        ~Matrix() { dev_free(p, s); }
+      } a{nullptr, stream};
+      try {
+        a.p = dev_alloc((size_t)n * n, stream);
+      } catch (const Error &) {
+        // no contiguous piece of that size: entries are generated as below
+      }
+      if (a.p) {
+        constexpr int kCols = 64;
+        std::vector<GenBlock> panels;
+        for (int c = 0; c < n; c += kCols)
+          panels.push_back(GenBlock{0, c, n, std::min(kCols, n - c), a.p + (long long)c * n, n});
+        kernel_blocks(*gen, panels, stream);
+        return build_attempt({BuildInput{in[0].g, a.p, n}}, tol, stream, svd_status, stats,
+                             nullptr, gen, t0);
+      }
+    }
+  }
+  return build_attempt(in, tol, stream, svd_status, stats, gen, nullptr, t0);
 }
 
 std::shared_ptr<DeviceTree> build_from_dense(const Geometry &g, const double *d_A, long long lda,

@@ -89,6 +89,9 @@ const char *hodlr_b200_last_error(void);
  *       about eps ||A|| / sigma)
  *   jacobi_cluster_min_c (192): problems this wide or wider use a cluster of
  *       8 CTAs
+ *   kernel_form_frac (0.0625): a build from points forms its kernel matrix in
+ *       scratch when it takes at most this share of the device memory free or
+ *       held unused by the library's pools (0: never)
  *   bj_inner_sweeps (2): sweeps of the block Jacobi SVD's per-pair eigensolver
  *       at most (fewer: cheaper rounds, possibly more outer sweeps)
  *   jacobi_block_min_c (128): sketch cores this wide or wider are solved by
@@ -172,7 +175,9 @@ int hodlr_b200_hxh_dev(hodlr_b200_tree a, hodlr_b200_tree b, double svd_threshol
  * and kinds as for hodlr_b200_kernel_matrix_dev below) without forming it:
  * every entry the construction needs is computed on the device where it is
  * used, so memory holds only the points, the tree and the sketches (a dense
- * n = 65536 input would take 34 GB).  The tree equals the one
+ * n = 65536 input would take 34 GB).  A matrix that fits a sixteenth of the
+ * device memory at hand (option kernel_form_frac) is formed in scratch for the
+ * duration of the call instead.  The tree equals the one
  * hodlr_b200_build_dev makes from the generated dense matrix.  No
  * counterpart in hmat_lib, whose constructor takes the dense matrix
  * (dense_to_tree_hodlr, src/constructors.c:629).  Ownership and errors as for
