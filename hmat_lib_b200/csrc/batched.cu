@@ -13,8 +13,8 @@
 // A plan is made once per call signature (trees, pointers, sizes, op,
 // precision) and kept in a small cache.  When it is made, the autotuner times
 // every candidate configuration of each phase on the real operands (tile
-// shape 128 x 64 or 64 x 128, with or without splitting long K ranges across
-// tiles) and keeps the fastest; the chosen launches are then captured once
+// shape, with or without splitting long K ranges across tiles) and keeps the
+// fastest; the chosen launches are then captured once
 // into a CUDA graph that later calls replay.
 #include <list>
 #include <string>
@@ -91,7 +91,7 @@ bool same_signature(const BatchPlan &p, int op, int precision, int device,
 
 // Device time of `fn` on `s`: best of `reps` runs after one warm-up run.
 template <class F>
-float time_best(F fn, cudaStream_t s, int reps = 3) {
+float time_best(F fn, cudaStream_t s, int reps = 2) {
   cudaEvent_t a, b;
   HB_CUDA(cudaEventCreate(&a));
   HB_CUDA(cudaEventCreate(&b));
@@ -116,7 +116,11 @@ std::string shape_name(TileShape t) {
 }
 
 // Plans phase `phase` of the FP64 batch for every candidate configuration,
-// times them on the real operands, keeps the fastest.
+// times them on the real operands, keeps the fastest.  A shape whose columns
+// are at least half empty for every tree, and a split that splits nothing, are
+// not candidates: with 16 right-hand sides the 128- and 256-column tiles were
+// half of the 32 runs and most of their time (48 trees built and multiplied
+// once: 46 -> 27 ms).
 std::unique_ptr<GemmPlan> tune_phase(const GemmBatch &batch, int phase, ProdOp op, int kmax,
                                      BatchPlan &P, cudaStream_t s, bool autotune) {
   if (batch.empty()) return nullptr;
@@ -125,13 +129,18 @@ std::unique_ptr<GemmPlan> tune_phase(const GemmBatch &batch, int phase, ProdOp o
     bool split;
   };
   std::vector<Cand> cands;
-  const int forced = (int)option("batch_shape", -1.0);   // 0..3: one shape, no timing
-  if (forced >= 0 && forced <= 3) {
+  const int forced = (int)option("batch_shape", -1.0);   // 0..4: one shape, no timing
+  if (forced >= 0 && forced <= 4) {
     cands.push_back(Cand{(TileShape)forced, phase == 1});
   } else if (autotune) {
-    for (TileShape sh : {TileShape::M128N64, TileShape::M64N128, TileShape::M32N128,
-                         TileShape::M32N256})
+    int ncols = 1;
+    for (const GemmProb &p : batch.probs) ncols = std::max(ncols, p.N);
+    for (TileShape sh : {TileShape::M128N64, TileShape::M64N64, TileShape::M64N128,
+                         TileShape::M32N128, TileShape::M32N256}) {
+      if (sh == TileShape::M64N64 ? ncols > 64 : tile_cols(sh) > 64 && 2 * ncols <= tile_cols(sh))
+        continue;
       for (bool sp : {false, true}) cands.push_back(Cand{sh, sp});
+    }
   } else {
     cands.push_back(Cand{default_shape(op, kmax, phase), phase == 1});
   }
@@ -144,6 +153,7 @@ std::unique_ptr<GemmPlan> tune_phase(const GemmBatch &batch, int phase, ProdOp o
     auto plan = std::make_unique<GemmPlan>();
     gemm_plan_build(*plan, batch, c.shape, c.split ? KSplit::All : KSplit::None, s);
     if (plan->ntiles == 0) continue;
+    if (c.split && plan->nscale == 0 && cands.size() > 1) continue;   // nothing was split
     float ms = 0.f;
     if (cands.size() > 1) ms = time_best([&] { gemm_plan_run(*plan, b, s); }, s);
     if (!best || ms < best_ms) {

@@ -105,7 +105,7 @@ const char *hodlr_b200_last_error(void);
  *       (Y = A Omega, B^T = A^T Q) on the int8 tensor cores; orthonormalisation,
  *       core SVDs and truncation stay FP64
  *   autotune (1), batch_shape (-1), use_graphs (1), check_status (0): batched
- *       products time candidate tile shapes / force one (0-3) / replay a CUDA
+ *       products time candidate tile shapes / force one (0-4) / replay a CUDA
  *       graph / read the mixed kernels' status word after each call
  *   ozaki_schedule (1): int8 GEMM tile schedule, longest first (0 round-robin)
  *   ozaki_phase1_tiles_per_cta (2): K-split granularity of the projections
