@@ -260,7 +260,7 @@ gemm_f64_kernel(const GemmSeg *__restrict__ segs, const GemmProb *__restrict__ p
 // is the loader's instructions (nine per MMA before the three copy paths of
 // stage_operand and the per-layout MMA loops, under five now), during which the
 // warps of a CTA issue no MMAs.  H X at n = 32768, k = 256 (ranks 38 to 349):
-// 1640 us without any of this, 1512 us without MMAs on padding, 1370 us now
+// 1640 us without any of this, 1512 us without MMAs on padding, 1370 us so
 // (28.7 TFLOP/s; cuBLAS DGEMM 35.5); H x H at n = 16384 (many products of 5 to
 // 40 columns) 3.44, 2.90, 2.47 ms.
 template <int BM, int BN, int BK>
@@ -296,29 +296,28 @@ __device__ __forceinline__ void cp_async16z(void *smem, const void *gmem, bool p
 // line or K value by 16-byte copies that read all or nothing, any other by
 // 8-byte ones (a copy of a variable number of bytes compiles to some 70
 // instructions).
-template <int ROWS, int BK>
-__device__ __forceinline__ void stage_operand(double *dst, const double *src, int ld, bool kcontig,
-                                              bool vec, int nlines, int kin) {
-  const int tid = threadIdx.x;
+template <int ROWS, int BK, int THREADS>
+__device__ __forceinline__ void stage_operand(int tid, double *dst, const double *src, int ld,
+                                              bool kcontig, bool vec, int nlines, int kin) {
   const bool full = nlines >= ROWS && kin == BK;
   if (kcontig) {
-    constexpr int CH = BK / 2, LS = kThreads / CH;   // 16-byte chunks per line, lines per pass
+    constexpr int CH = BK / 2, LS = THREADS / CH;   // 16-byte chunks per line, lines per pass
     static_assert(ROWS % LS == 0, "whole passes");
     const int l0 = tid / CH, k = 2 * (tid % CH);
     double *d = dst + l0 * (BK + 4) + k;
     const double *q = src + (long long)l0 * ld + k;
     const long long step = (long long)LS * ld;
     if (vec && full) {
-#pragma unroll
+#pragma unroll(THREADS < kThreads ? 4 : 64)
       for (int i = 0; i < ROWS / LS; ++i, q += step) cp_async16(d + i * LS * (BK + 4), q);
     } else if (vec && (kin & 1) == 0) {
-#pragma unroll
+#pragma unroll(THREADS < kThreads ? 4 : 64)
       for (int i = 0; i < ROWS / LS; ++i, q += step) {
         const bool in = k < kin && l0 + i * LS < nlines;
         cp_async16z(d + i * LS * (BK + 4), in ? q : src, in);
       }
     } else {
-#pragma unroll
+#pragma unroll(THREADS < kThreads ? 4 : 64)
       for (int i = 0; i < ROWS / LS; ++i, q += step) {
         const bool in = k < kin && l0 + i * LS < nlines, in2 = in && k + 1 < kin;
         cp_async8(d + i * LS * (BK + 4), in ? q : src, in);
@@ -326,22 +325,23 @@ __device__ __forceinline__ void stage_operand(double *dst, const double *src, in
       }
     }
   } else {
-    constexpr int CH = ROWS / 2, KS = kThreads / CH;   // chunks per K value, K values per pass
+    constexpr int CH = ROWS / 2, KS = THREADS / CH;   // chunks per K value, K values per pass
+    static_assert(KS >= 1, "a line is no longer than a pass");
     const int line = 2 * (tid % CH), k0 = tid / CH;
     double *d = dst + k0 * (ROWS + 4) + line;
     const double *q = src + (long long)k0 * ld + line;
     const long long step = (long long)KS * ld;
     if (vec && full) {
-#pragma unroll
+#pragma unroll(THREADS < kThreads ? 4 : 64)
       for (int i = 0; i < BK / KS; ++i, q += step) cp_async16(d + i * KS * (ROWS + 4), q);
     } else if (vec && ((nlines & 1) == 0 || nlines >= ROWS)) {
-#pragma unroll
+#pragma unroll(THREADS < kThreads ? 4 : 64)
       for (int i = 0; i < BK / KS; ++i, q += step) {
         const bool in = line < nlines && k0 + i * KS < kin;
         cp_async16z(d + i * KS * (ROWS + 4), in ? q : src, in);
       }
     } else {
-#pragma unroll
+#pragma unroll(THREADS < kThreads ? 4 : 64)
       for (int i = 0; i < BK / KS; ++i, q += step) {
         const bool in = line < nlines && k0 + i * KS < kin, in2 = in && line + 1 < nlines;
         cp_async8(d + i * KS * (ROWS + 4), in ? q : src, in);
@@ -501,13 +501,15 @@ gemm_f64_mma_kernel(const GemmSeg *__restrict__ segs, const GemmProb *__restrict
     if (fl & 16u)
       stage_generated<BM, BK>(as, bases.gen, goff, ka, tile.m0, P.M - tile.m0, it.kk, kin);
     else
-      stage_operand<BM, BK>(as, pa + (ka ? (long long)it.kk : (long long)it.kk * lda), lda, ka,
-                            fl & 4u, P.M - tile.m0, kin);
+      stage_operand<BM, BK, kThreads>(tid, as,
+                                      pa + (ka ? (long long)it.kk : (long long)it.kk * lda), lda,
+                                      ka, fl & 4u, P.M - tile.m0, kin);
     if (fl & 32u)
       stage_generated<BN, BK>(bs, bases.gen, goff, kb, tile.n0, P.N - tile.n0, it.kk, kin);
     else
-      stage_operand<BN, BK>(bs, pb + (kb ? (long long)it.kk : (long long)it.kk * ldb), ldb, kb,
-                            fl & 8u, P.N - tile.n0, kin);
+      stage_operand<BN, BK, kThreads>(tid, bs,
+                                      pb + (kb ? (long long)it.kk : (long long)it.kk * ldb), ldb,
+                                      kb, fl & 8u, P.N - tile.n0, kin);
     return fl & 3u;
   };
   // the next K-block of the load side, opening its segment when it changes
@@ -607,6 +609,171 @@ gemm_f64_mma_kernel(const GemmSeg *__restrict__ segs, const GemmProb *__restrict
   }
 }
 
+// ---- the same product with loader warps ----------------------------------------------
+// Eight warps issue MMAs only, two more the copies: in
+// gemm_f64_mma_kernel every warp stops its MMAs for some 400 instructions a
+// stage, and the warps of a CTA do so together, which leaves the tensor cores
+// idle a fifth of the time.  Stages are handed over with named barriers (full:
+// the loaders arrive, the MMA warps wait; empty: the reverse); each carries its
+// operand layout and K length, a length of zero ends the tile.  Used for
+// plans without generated operands (whose entries all threads should compute).
+// H X at n = 32768, k = 256: 1370 -> 1253 us (tensor cores active 79 -> 84% of
+// the time); H^T X and X H at n = 10007, k = 33: 265 -> 209 us.
+constexpr int kWsLoaders = 64;
+constexpr int kWsThreads = kThreads + kWsLoaders;
+
+__device__ __forceinline__ void bar_sync(int id) {
+  asm volatile("bar.sync %0, %1;\n" ::"r"(id), "n"(kWsThreads) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(int id) {
+  asm volatile("bar.arrive %0, %1;\n" ::"r"(id), "n"(kWsThreads) : "memory");
+}
+
+template <int BM, int BN, int WM, int WN, int BK>
+__global__ void __launch_bounds__(kWsThreads, 2)
+gemm_f64_ws_kernel(const GemmSeg *__restrict__ segs, const GemmProb *__restrict__ probs,
+                   const GemmTile *__restrict__ tiles, GemmBases bases) {
+  using SM = MmaSmem<BM, BN, BK>;
+  constexpr int S = SM::STAGES;
+  static_assert(2 * S + 1 <= 16, "named barriers");
+  extern __shared__ __align__(16) double smem[];
+  __shared__ int meta[S];   // per stage: layout bits (1: A [m][k], 2: B [n][k]), K values << 2
+  const GemmTile tile = tiles[blockIdx.x];
+  const GemmProb P = probs[tile.prob];
+  auto full = [](int st) { return 1 + st; };
+  auto empty = [](int st) { return 1 + S + st; };
+
+  if (threadIdx.x >= kThreads) {
+    // ---------------- loaders ----------------
+    constexpr int kLag = S - 2;   // stages in flight behind the one being issued
+    const int tid = threadIdx.x - kThreads;
+    const int seg_end = P.seg0 + P.nseg;
+    const int nm = P.M - tile.m0, nn = P.N - tile.n0;
+    int kbase = 0, t = 0;
+    for (int si = P.seg0; si < seg_end; ++si) {
+      const GemmSeg G = segs[si];
+      int kk = max(tile.k0 - kbase, 0);
+      const int le = min(tile.k1 - kbase, G.K);
+      kbase += G.K;
+      if (kk >= le) continue;
+      const bool ka = G.ta == 1, kb = G.tb == 0;
+      const int lda = (int)G.lda, ldb = (int)G.ldb;
+      const double *pa = base_ptr(bases, G.abase) + G.a_off;
+      const double *pb = base_ptr(bases, G.bbase) + G.b_off;
+      // 16-byte copies: as in gemm_f64_mma_kernel
+      const bool va = ((lda | (ka ? kk : 0)) & 1) == 0 && ((unsigned long long)pa & 15) == 0;
+      const bool vb = ((ldb | (kb ? kk : 0)) & 1) == 0 && ((unsigned long long)pb & 15) == 0;
+      pa += ka ? (long long)tile.m0 * lda + kk : tile.m0 + (long long)kk * lda;
+      pb += kb ? (long long)tile.n0 * ldb + kk : tile.n0 + (long long)kk * ldb;
+      for (; kk < le; kk += BK, ++t) {
+        const int st = t % S, kin = min(BK, le - kk);
+        if (t >= S) bar_sync(empty(st));
+        double *as = smem + st * SM::STAGE;
+        stage_operand<BM, BK, kWsLoaders>(tid, as, pa, lda, ka, va, nm, kin);
+        stage_operand<BN, BK, kWsLoaders>(tid, as + SM::A_ELEMS, pb, ldb, kb, vb, nn, kin);
+        cp_async_commit();
+        if (tid == 0) meta[st] = (ka ? 1 : 0) | (kb ? 2 : 0) | (kin << 2);
+        if (t >= kLag) {
+          cp_async_wait<kLag>();
+          bar_arrive(full((t - kLag) % S));
+        }
+        pa += ka ? (long long)BK : (long long)BK * lda;
+        pb += kb ? (long long)BK : (long long)BK * ldb;
+      }
+    }
+    cp_async_wait<0>();
+    for (int u = max(0, t - kLag); u < t; ++u) bar_arrive(full(u % S));
+    // the end, then the stages still being read (no arrival is left over)
+    if (t >= S) bar_sync(empty(t % S));
+    if (tid == 0) meta[t % S] = 0;
+    __threadfence_block();
+    bar_arrive(full(t % S));
+    for (int u = max(0, t - S + 1); u < t; ++u) bar_sync(empty(u % S));
+    return;
+  }
+
+  // ---------------- MMA warps ----------------
+  constexpr int MT = WM / 8, NT = WN / 8, WARPS_N = BN / WN;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane >> 2, tq = lane & 3;
+  int wrow, wcol;   // warps to sub-partitions: as in gemm_f64_mma_kernel
+  if constexpr (WARPS_N == 2) {
+    wrow = warp & 3;
+    wcol = warp >> 2;
+  } else if constexpr (WARPS_N == 4) {
+    wrow = warp >> 2;
+    wcol = (warp + 2 * wrow) & 3;
+  } else {
+    wrow = warp / WARPS_N;
+    wcol = warp % WARPS_N;
+  }
+  const int wm0 = wrow * WM, wn0 = wcol * WN;
+  const int mt_in = max(0, min(MT, (P.M - tile.m0 - wm0 + 7) / 8));
+  const int nt_in = max(0, min(NT, (P.N - tile.n0 - wn0 + 7) / 8));
+  const bool whole = mt_in == MT && nt_in == NT;
+  double acc[MT][NT][2];
+#pragma unroll
+  for (int i = 0; i < MT; ++i)
+#pragma unroll
+    for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+
+  for (int st = 0;; st = st + 1 == S ? 0 : st + 1) {
+    bar_sync(full(st));
+    const int m = meta[st], kin = m >> 2;
+    if (kin == 0) break;
+    const double *as = smem + st * SM::STAGE;
+    const double *bs = as + SM::A_ELEMS;
+    const int a_line = (m & 1) ? SM::LDK : 1, a_k = (m & 1) ? 1 : SM::LDKM;
+    const int b_line = (m & 2) ? SM::LDK : 1, b_k = (m & 2) ? 1 : SM::LDKN;
+    const double *ap = as + (wm0 + g) * a_line + tq * a_k;
+    const double *bp = bs + (wn0 + g) * b_line + tq * b_k;
+    if (whole && kin == BK) {
+      switch (m & 3) {
+        case 0: stage_mmas<MT, NT, BK, 1, SM::LDKM, 1, SM::LDKN>(acc, ap, bp); break;
+        case 1: stage_mmas<MT, NT, BK, SM::LDK, 1, 1, SM::LDKN>(acc, ap, bp); break;
+        case 2: stage_mmas<MT, NT, BK, 1, SM::LDKM, SM::LDK, 1>(acc, ap, bp); break;
+        default: stage_mmas<MT, NT, BK, SM::LDK, 1, SM::LDK, 1>(acc, ap, bp); break;
+      }
+    } else if (mt_in > 0 && nt_in > 0) {
+      for (int k4 = 0; 4 * k4 < kin; ++k4) {
+        double b[NT];
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+          if (j < nt_in) b[j] = bp[(8 * j) * b_line + 4 * k4 * b_k];
+#pragma unroll
+        for (int i = 0; i < MT; ++i)
+          if (i < mt_in) {
+            const double a = ap[(8 * i) * a_line + 4 * k4 * a_k];
+#pragma unroll
+            for (int j = 0; j < NT; ++j)
+              if (j < nt_in) dmma884(acc[i][j], a, b[j]);
+          }
+      }
+    }
+    bar_arrive(empty(st));
+  }
+
+  double *C = base_ptr(bases, P.cbase) + P.c_off;
+#pragma unroll
+  for (int i = 0; i < MT; ++i) {
+    const int row = tile.m0 + wm0 + 8 * i + g;
+    if (row >= P.M) continue;
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int col = tile.n0 + wn0 + 8 * j + 2 * tq + h;
+        if (col >= P.N) continue;
+        double *c = C + row + (long long)col * P.ldc;
+        const double v = P.alpha * acc[i][j][h];
+        if (tile.atomic)
+          atomicAdd(c, v);
+        else
+          *c = (P.beta == 0.0) ? v : v + P.beta * (*c);
+      }
+  }
+}
+
 // beta pre-pass for the (m, n) tiles that several tiles add to
 __global__ void gemm_scale_c_kernel(const GemmProb *__restrict__ probs,
                                     const GemmTile *__restrict__ tiles, int bm, int bn,
@@ -637,6 +804,22 @@ void launch_gemm(const GemmPlan &plan, const GemmBases &bases, cudaStream_t stre
         plan.segs, plan.probs, plan.tiles, bases);
     HB_LAUNCHED();
     return;
+  }
+  if constexpr (BM <= 2 * kWsLoaders && BN <= 2 * kWsLoaders) {   // a chunk per loader and line
+    if (engine == 2 && !plan.generated) {
+      static bool configured = false;
+      if (!configured) {
+        HB_CUDA(cudaFuncSetAttribute(gemm_f64_ws_kernel<BM, BN, WM, WN, 32>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)MmaSmem<BM, BN, 32>::bytes));
+        configured = true;
+      }
+      gemm_f64_ws_kernel<BM, BN, WM, WN, 32>
+          <<<plan.ntiles, kWsThreads, MmaSmem<BM, BN, 32>::bytes, stream>>>(plan.segs, plan.probs,
+                                                                          plan.tiles, bases);
+      HB_LAUNCHED();
+      return;
+    }
   }
   if (engine == 2) {
     static bool configured = false;
@@ -787,6 +970,9 @@ void gemm_plan_build(GemmPlan &plan, const GemmBatch &batch, TileShape shape, KS
   }
   plan.ntiles = (int)tiles.size();
   plan.nscale = (int)scale.size();
+  plan.generated = false;
+  for (const GemmSeg &g : batch.segs)
+    plan.generated = plan.generated || g.abase == kGenSlot || g.bbase == kGenSlot;
   tiles.insert(tiles.end(), scale.begin(), scale.end());
   const size_t bs = batch.segs.size() * sizeof(GemmSeg);
   const size_t bp = probs.size() * sizeof(GemmProb);

@@ -99,6 +99,7 @@ struct GemmPlan {
   int ntiles = 0;
   int nscale = 0;               // (m, n) tiles that several tiles add to and beta != 1
   void *dev = nullptr;          // one allocation holding the three arrays
+  bool generated = false;       // some operand is a generated kernel matrix
   bool transient = false;       // dev is stream-ordered (freed with cudaFreeAsync on `stream`)
   cudaStream_t stream = nullptr;
   GemmSeg *segs = nullptr;
