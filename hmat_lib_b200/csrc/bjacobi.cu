@@ -13,15 +13,16 @@
 //   2. if some column pair of G is coupled above the convergence test, every
 //      CTA runs sweeps of cyclic two-sided Jacobi on G, G = W diag W^T (the
 //      same arithmetic in every CTA, so the same W), and sorts the diagonal in
-//      descending order;
+//      descending order; pairs inside a block once a sweep, else pairs across;
 //   3. X[:, pair] = X[:, pair] W and V[:, pair] = V[:, pair] W over its rows
 //      (mma m8n8k4 again), in place, a 32-row tile at a time.
 // Phases 1 and 3 read 32 x 64 tiles through a ring of asynchronous copies and
 // are bound by the FP64 tensor cores (2.6 x 64 x 64 multiply-adds per row and
 // pair); phase 2 by the latency of its 63 steps a sweep, which is why a step
 // has one barrier and its angle comes from single precision (see rotation()).
-// Core stage (254 cores of up to 704 columns, n = 32768 2D): 61 -> 33 ms; 62
-// cores of up to 1600 columns (n = 8192 3D): 179 -> 79 ms.
+// Core stage (254 cores of up to 704 columns, n = 32768 2D): 61 -> 28 ms; 62
+// cores of up to 1600 columns (n = 8192 3D): 179 -> 74 ms (33 and 79 with all
+// 63 steps in every round).
 // Rotations act on the columns themselves (no re-factorisation of a pair), so
 // small columns keep their relative accuracy; the rotation is applied only
 // when the pair needs it, so the late sweeps are mostly Gram passes.
@@ -56,8 +57,8 @@ constexpr int kPT = 32 * (kPW + 1);   // threads: one more warp computes the rot
 constexpr int kHalf = kPair / 2; // column pairs of a step
 // Sweeps of a pair's eigensolver at most (option bj_inner_sweeps).  A pair need
 // not be finished: its rotation is orthogonal all the same, and the outer
-// sweeps finish the job.  Core stage with 30 / 4 / 3 / 2 / 1: 38 / 36 / 35 / 33 /
-// 33 ms at n = 32768 (2D), 100 / 97 / 89 / 79 / 87 ms at n = 8192 (3D).
+// sweeps finish the job.  Core stage with 4 / 3 / 2 / 1: 32 / 30 / 28 / 33 ms at
+// n = 32768 (2D), 82 / 78 / 74 / 92 ms at n = 8192 (3D).
 constexpr int kInner = 2;
 constexpr int kT = 32;           // transpose tile, rows of a staged tile
 constexpr int kLdT = kT + 4;     // leading dimension of a staged tile (column by column)
@@ -122,7 +123,7 @@ struct BjDev {
 
 // Shared memory of the pair kernel.  gp: this CTA's partial Gram (tiles I <= J),
 // later W with sorted columns, element (i, j) at i + j kLd.  pl: the pair's Gram
-// by position (see place_of), two buffers of four planes [K][M], K <= M: the
+// by place, two buffers of four planes [K][M], K <= M: the
 // products of K's first / second column with M's first / second.
 struct PairSmem {
   double gp[kPair * kLd];
@@ -132,25 +133,39 @@ struct PairSmem {
   int perm[kPair];
 };
 
-// Where column x of the pair sits at step 0 of the round-robin over 64
-// columns: pair k holds columns k and 63 - k (pair 0: 0 and 63), first / second.
-__device__ __forceinline__ void place_of(int x, int &k, int &second) {
-  second = x >= kHalf;
-  k = x < kHalf ? x : x == kPair - 1 ? 0 : kPair - 1 - x;
-}
-__device__ __forceinline__ int column_at(int k, int second) {
-  return !second ? k : k == 0 ? kPair - 1 : kPair - 1 - k;
-}
-// One step of the round-robin moves every column to its next place (the
-// second column of pair 0 stays); after 63 steps all are back.
-__device__ __forceinline__ void next_place(int &k, int &second) {
-  if (!second) {
+// At the start of a sweep pair k holds column k of the first block and column
+// k of the second (first / second place).
+__device__ __forceinline__ int column_at(int k, int second) { return k + second * kHalf; }
+// One step moves every column to its next place.  All pairs of the 64 columns
+// (`all`): the round-robin (the second column of pair 0 stays), back after 63
+// steps.  Pairs across the two blocks only: the second columns move on by one,
+// back after 32 steps.
+__device__ __forceinline__ void next_place(int &k, int &second, bool all) {
+  if (!all) {
+    if (second) k = (k + 1) % kHalf;
+  } else if (!second) {
     second = k == 0;
     k = k == 0 ? 1 : k - 1;
   } else if (k == kHalf - 1) {
     second = 0;
   } else if (k > 0) {
     ++k;
+  }
+}
+// The place whose column comes to place (k, second) in a step.
+__device__ __forceinline__ void prev_place(int &k, int &second, bool all) {
+  if (!all) {
+    if (second) k = (k + kHalf - 1) % kHalf;
+  } else if (!second) {
+    if (k == kHalf - 1)
+      second = 1;
+    else
+      ++k;
+  } else if (k == 1) {
+    k = 0;
+    second = 0;
+  } else if (k > 1) {
+    --k;
   }
 }
 // Where pair k's rotation is kept: the four lanes of a row of W read pairs
@@ -346,10 +361,7 @@ bj_pair_kernel(const BjDev *__restrict__ probs, const int2 *__restrict__ slots, 
     if (i == j) {
       S.dg[i] = s;
     } else {
-      int ki, si, kj, sj;
-      place_of(i, ki, si);
-      place_of(j, kj, sj);
-      (&S.pl[0][0][0][0])[plane_offset(ki, si, kj, sj)] = s;
+      (&S.pl[0][0][0][0])[plane_offset(i % kHalf, i / kHalf, j % kHalf, j / kHalf)] = s;
     }
   }
   // after this barrier no CTA reads another's gp any more
@@ -365,6 +377,11 @@ bj_pair_kernel(const BjDev *__restrict__ probs, const int2 *__restrict__ slots, 
   // computes the next step's 32 rotations: lane k applies the step to the one
   // block that holds the next product of pair k itself.  So a step has one
   // barrier and lasts as long as that chain (a block, an angle).
+  // Pairs inside a block are tested and rotated once a sweep, in its first
+  // round (the block with the bye there: in the second); otherwise the 32
+  // steps of pairs across the blocks do, half the 63 of all pairs.
+  const int r_sweep = (int)(g_round % (P.players - 1));
+  const bool all = r_sweep == 0 || (r_sweep == 1 && a == 0);
   const bool solver = warp == kPW;
   constexpr int kBlocks = kHalf * (kHalf - 1) / 2;   // off-diagonal blocks K < M
   constexpr int kPlane = kHalf * kHalf;
@@ -381,8 +398,8 @@ bj_pair_kernel(const BjDev *__restrict__ probs, const int2 *__restrict__ slots, 
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       int k = bk[u], sk = q >> 1, m = bm[u], sm = q & 1;
-      next_place(k, sk);
-      next_place(m, sm);
+      next_place(k, sk, all);
+      next_place(m, sm, all);
       to[u][q] = plane_offset(k, sk, m, sm);
     }
   }
@@ -394,12 +411,13 @@ bj_pair_kernel(const BjDev *__restrict__ probs, const int2 *__restrict__ slots, 
   int to_pair = 0, nk = 0, nm = 0, nq = 0;
   {
     int k = lane, sk = 0, m = lane, sm = 1;
-    next_place(k, sk);
-    next_place(m, sm);
+    next_place(k, sk, all);
+    next_place(m, sm, all);
     to_pair = plane_offset(k, sk, m, sm);
     // the places whose columns come to (lane, first) and (lane, second)
-    const int ka = lane == kHalf - 1 ? lane : lane + 1, sa = lane == kHalf - 1;
-    const int kb = lane == 0 || lane == 1 ? 0 : lane - 1, sb = lane != 1;
+    int ka = lane, sa = 0, kb = lane, sb = 1;
+    prev_place(ka, sa, all);
+    prev_place(kb, sb, all);
     nk = min(ka, kb);
     nm = max(ka, kb);
     nq = ka < kb ? 2 * sa + sb : 2 * sb + sa;
@@ -413,7 +431,8 @@ bj_pair_kernel(const BjDev *__restrict__ probs, const int2 *__restrict__ slots, 
   }
   __syncthreads();
   int par = 0;
-  // whether some column pair of the current G must be rotated (uniform)
+  // whether some column pair of the current G that this round tests must be
+  // rotated (uniform)
   auto unconverged = [&]() -> bool {
     const double *pl = &S.pl[par][0][0][0];
     bool w = false;
@@ -425,8 +444,8 @@ bj_pair_kernel(const BjDev *__restrict__ probs, const int2 *__restrict__ slots, 
         if (bk[u] >= 0) {
 #pragma unroll
           for (int q = 0; q < 4; ++q)
-            w = w || needs_rotation(S.dg[bk[u] + (q >> 1) * kHalf], S.dg[bm[u] + (q & 1) * kHalf],
-                                    pl[from[u] + q * kPlane], P.theta2, fro2, conv2);
+            w = w || ((all || q == 1 || q == 2) && needs_rotation(S.dg[bk[u] + (q >> 1) * kHalf], S.dg[bm[u] + (q & 1) * kHalf],
+                                    pl[from[u] + q * kPlane], P.theta2, fro2, conv2));
         }
     }
     return __syncthreads_or(w) != 0;
@@ -459,7 +478,7 @@ bj_pair_kernel(const BjDev *__restrict__ probs, const int2 *__restrict__ slots, 
   if (solver) decide(S.pl[par][1][lane][lane], par);
   __syncthreads();
   for (int sweep = 0; sweep < inner_max; ++sweep) {
-    for (int step = 0; step < kPair - 1; ++step) {
+    for (int step = all ? kPair - 1 : kHalf; step > 0; --step) {
       const double *src = &S.pl[par][0][0][0];
       double *dst = &S.pl[par ^ 1][0][0][0];
       if (solver) {
@@ -471,11 +490,16 @@ bj_pair_kernel(const BjDev *__restrict__ probs, const int2 *__restrict__ slots, 
         const double z = (nq & 1) ? M.y : M.x, w = (nq & 1) ? M.x : -M.y;
         const double g = z * (x * b00 + y * b10) + w * (x * b01 + y * b11);
         const double n0 = d0 - moved, n1 = d1 + moved;
-        const double up = __shfl_down_sync(0xffffffffu, n0, 1);
-        const double dn = __shfl_up_sync(0xffffffffu, n1, 1);
-        const double first = __shfl_sync(0xffffffffu, n0, 0);
-        d0 = lane == kHalf - 1 ? n1 : up;
-        d1 = lane == 0 ? n1 : lane == 1 ? first : dn;
+        const double dn = __shfl_sync(0xffffffffu, n1, (lane + kHalf - 1) % kHalf);
+        if (all) {
+          const double up = __shfl_down_sync(0xffffffffu, n0, 1);
+          const double first = __shfl_sync(0xffffffffu, n0, 0);
+          d0 = lane == kHalf - 1 ? n1 : up;
+          d1 = lane == 0 ? n1 : lane == 1 ? first : dn;
+        } else {
+          d0 = n0;
+          d1 = dn;
+        }
         decide(g, par ^ 1);
       } else {
 #pragma unroll
@@ -499,18 +523,24 @@ bj_pair_kernel(const BjDev *__restrict__ probs, const int2 *__restrict__ slots, 
           wa[u] = cs.x * x - cs.y * y;
           wb[u] = cs.y * x + cs.x * y;
         }
-        const double an = __shfl_down_sync(0xffffffffu, wa[0], 1);
-        const double bn = __shfl_up_sync(0xffffffffu, wb[7], 1);
-        const double a0 = wa[0], b7 = wb[7], b0 = wb[0];
+        const double bn = __shfl_sync(0xffffffffu, wb[7], (lane & ~3) | ((lane + 3) & 3));
+        if (all) {
+          const double an = __shfl_down_sync(0xffffffffu, wa[0], 1);
+          const double a0 = wa[0], b7 = wb[7], b0 = wb[0];
 #pragma unroll
-        for (int u = 0; u < 7; ++u) wa[u] = wa[u + 1];
-        wa[7] = tq == 3 ? b7 : an;
+          for (int u = 0; u < 7; ++u) wa[u] = wa[u + 1];
+          wa[7] = tq == 3 ? b7 : an;
 #pragma unroll
-        for (int u = 7; u > 0; --u) wb[u] = wb[u - 1];
-        if (tq == 0) {
-          wb[0] = b0;
-          wb[1] = a0;
+          for (int u = 7; u > 0; --u) wb[u] = wb[u - 1];
+          if (tq == 0) {
+            wb[0] = b0;
+            wb[1] = a0;
+          } else {
+            wb[0] = bn;
+          }
         } else {
+#pragma unroll
+          for (int u = 7; u > 0; --u) wb[u] = wb[u - 1];
           wb[0] = bn;
         }
       }
