@@ -74,25 +74,51 @@ T *upload_vec(const std::vector<T> &v, cudaStream_t s) {
   return d;
 }
 
-// dst[i + j ldd] = src[j + i lds] for i, j < n (32 x 32 tiles through shared
-// memory, one padding column against bank conflicts)
-__global__ void bj_transpose_kernel(const double *__restrict__ src, long long lds, int n,
-                                    double *__restrict__ dst, long long ldd) {
+// One problem's start and end.
+struct BjIo {
+  const double *A;   // the core's transpose (L x L, ld lda)
+  long long lda;
+  double *X, *V;     // Lp x Lp
+  int L, Lp;
+  int rank;          // end: columns wanted
+  const int *perm;   // end: where they are, in order
+  double *U, *Vout;  // end: L x rank each, ld L
+};
+
+// X = A^T with zero padding, V = I (32 x 32 tiles through shared memory, one
+// padding column against bank conflicts): all of both is written.
+__global__ void bj_start_kernel(const BjIo *__restrict__ probs) {
+  const BjIo P = probs[blockIdx.y];
   __shared__ double tile[kT][kT + 1];
-  const int i0 = blockIdx.x * kT, j0 = blockIdx.y * kT;
   const int tx = threadIdx.x, ty = threadIdx.y;   // 32 x 8 threads
-  // tile[jj][ii] = src[(j0 + ii) + (i0 + jj) lds]: coalesced along ii
-  for (int jj = ty; jj < kT; jj += 8)
-    if (i0 + jj < n && j0 + tx < n) tile[jj][tx] = src[(j0 + tx) + (long long)(i0 + jj) * lds];
-  __syncthreads();
-  // dst[(i0 + ii) + (j0 + jj) ldd] = src[(j0 + jj) + (i0 + ii) lds] = tile[ii][jj]
-  for (int jj = ty; jj < kT; jj += 8)
-    if (i0 + tx < n && j0 + jj < n) dst[(i0 + tx) + (long long)(j0 + jj) * ldd] = tile[tx][jj];
+  const int nt = P.Lp / kT;
+  for (int t = blockIdx.x; t < nt * nt; t += gridDim.x) {
+    const int i0 = t % nt * kT, j0 = t / nt * kT;
+    // tile[jj][ii] = A[(j0 + ii) + (i0 + jj) lda]: coalesced along ii
+    for (int jj = ty; jj < kT; jj += 8)
+      tile[jj][tx] =
+          i0 + jj < P.L && j0 + tx < P.L ? P.A[(j0 + tx) + (long long)(i0 + jj) * P.lda] : 0.0;
+    __syncthreads();
+    // X[(i0 + ii) + (j0 + jj) Lp] = A[(j0 + jj) + (i0 + ii) lda] = tile[ii][jj]
+    for (int jj = ty; jj < kT; jj += 8) {
+      const long long o = (i0 + tx) + (long long)(j0 + jj) * P.Lp;
+      P.X[o] = tile[tx][jj];
+      P.V[o] = i0 + tx == j0 + jj ? 1.0 : 0.0;
+    }
+    __syncthreads();
+  }
 }
 
-__global__ void bj_identity_kernel(double *__restrict__ v, long long ld, int n) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    v[i + (long long)i * ld] = 1.0;
+// The wanted columns of X and V in order.
+__global__ void bj_gather_kernel(const BjIo *__restrict__ probs) {
+  const BjIo P = probs[blockIdx.y];
+  for (int c = blockIdx.x; c < P.rank; c += gridDim.x) {
+    const long long from = (long long)P.perm[c] * P.Lp, to = (long long)c * P.L;
+    for (int r = threadIdx.x; r < P.L; r += blockDim.x) {
+      P.U[to + r] = P.X[from + r];
+      P.Vout[to + r] = P.V[from + r];
+    }
+  }
 }
 
 // Blocks (a, b), a < b, of pair k in round r of a round-robin over `players` (even).
@@ -118,7 +144,7 @@ struct BjDev {
   double theta2;   // columns of squared norm at or below this are not rotated (times gscale)
   double fro;      // ||A||_F, the scale of the norm-relative test (times sqrt(gscale))
   double conv;     // convergence threshold of a column pair
-  int *rot;        // set when a pair of the problem rotated in the current sweep
+  int *rot;        // 1 + the last round in which a pair of the problem rotated
 };
 
 // Shared memory of the pair kernel.  gp: this CTA's partial Gram (tiles I <= J),
@@ -579,7 +605,7 @@ bj_pair_kernel(const BjDev *__restrict__ probs, const int2 *__restrict__ slots, 
       S.gp[wrow + S.perm[column_at(8 * tq + u, 1)] * kLd] = wb[u];
     }
   }
-  if (crank == 0 && tid == 0) *P.rot = 1;
+  if (crank == 0 && tid == 0) *P.rot = (int)g_round + 1;
   __syncthreads();
 
   // ---- 3. the rotation of this CTA's rows of X and V, in place, a 32-row
@@ -675,21 +701,30 @@ void block_jacobi_svd(const std::vector<BjProb> &probs, double tol, int max_swee
   std::vector<long long> noff(np);   // squared column norms of X
   for (int p = 0; p < np; ++p) noff[p] = take(wk[p].Lp);
   double *w = dev_alloc(total, s);
-  HB_CUDA(cudaMemsetAsync(w, 0, sizeof(double) * total, s));
-  int *d_rot = nullptr;   // per problem: a pair rotated in this sweep
+  int *d_rot = nullptr;   // per problem: 1 + the last round that rotated a pair
   HB_CUDA(cudaMallocAsync((void **)&d_rot, sizeof(int) * np, s));
   HB_CUDA(cudaMemsetAsync(d_rot, 0, sizeof(int) * np, s));
   // ---- X = A^T, V = I, thresholds -------------------------------------------------------
   std::vector<NormDesc> nd;
+  std::vector<BjIo> io;
   for (int p = 0; p < np; ++p) {
     const Work &W = wk[p];
-    dim3 grid((W.L + kT - 1) / kT, (W.L + kT - 1) / kT);
-    bj_transpose_kernel<<<grid, dim3(kT, 8), 0, s>>>(probs[p].A, probs[p].lda, W.L, w + W.x, W.Lp);
-    HB_LAUNCHED();
-    bj_identity_kernel<<<(W.Lp + 255) / 256, 256, 0, s>>>(w + W.v, W.Lp, W.Lp);
-    HB_LAUNCHED();
+    io.push_back(BjIo{probs[p].A, probs[p].lda, w + W.x, w + W.v, W.L, W.Lp, 0, nullptr,
+                      probs[p].U, probs[p].V});
     nd.push_back(NormDesc{w + W.x, W.Lp, W.L, W.Lp, w + noff[p]});
   }
+  // `io` in pieces of a grid's height
+  auto for_problems = [&](auto launch) {
+    BjIo *d = upload_vec(io, s);
+    for (int off = 0; off < np; off += 65535) {
+      launch(d + off, std::min(65535, np - off));
+      HB_LAUNCHED();
+    }
+    cudaFreeAsync(d, s);
+  };
+  for_problems([&](const BjIo *d, int n) {
+    bj_start_kernel<<<dim3(64, (unsigned)n), dim3(kT, 8), 0, s>>>(d);
+  });
   column_norms2(nd, s);
   // a column pair of length L recomputed by a 64-term sum is orthogonal to
   // about sqrt(L) eps
@@ -791,15 +826,13 @@ void block_jacobi_svd(const std::vector<BjProb> &probs, double tol, int max_swee
       Work &W = wk[p];
       if (!W.active || (g + 1) % (W.players - 1) != 0) continue;
       ++W.sweep;
-      if (!rot[p]) {
+      if (rot[p] <= g + 1 - (W.players - 1)) {   // none since the sweep began
         W.active = false;
         W.converged = true;
         changed = true;
       } else if (W.sweep >= max_sweeps) {
         W.active = false;
         changed = true;
-      } else {
-        HB_CUDA(cudaMemsetAsync(d_rot + p, 0, sizeof(int), s));
       }
     }
     if (changed) make_slots();
@@ -812,7 +845,7 @@ void block_jacobi_svd(const std::vector<BjProb> &probs, double tol, int max_swee
   for (int p = 0; p < np; ++p) nd.push_back(NormDesc{w + wk[p].x, wk[p].Lp, wk[p].L, wk[p].Lp,
                                                      w + noff[p]});
   column_norms2(nd, s);
-  std::vector<CopyDesc> gather;
+  std::vector<int> perms;
   std::vector<std::vector<double>> sig(np);
   std::vector<int> ranks(np), sweeps(np);
   read_norms();
@@ -831,16 +864,22 @@ void block_jacobi_svd(const std::vector<BjProb> &probs, double tol, int max_swee
       while (r < W.L && sig[p][r] >= tol * s0) ++r;
     ranks[p] = r;
     sweeps[p] = W.converged ? W.sweep : max_sweeps + 1;
-    for (int c = 0; c < W.L; ++c) {
-      gather.push_back(CopyDesc{w + W.x + (long long)perm[c] * W.Lp, W.Lp,
-                                probs[p].U + (long long)c * W.L, W.L, W.L, 1});
-      gather.push_back(CopyDesc{w + W.v + (long long)perm[c] * W.Lp, W.Lp,
-                                probs[p].V + (long long)c * W.L, W.L, W.L, 1});
-    }
+    io[p].rank = r;
+    perms.insert(perms.end(), perm.begin(), perm.begin() + r);
   }
-  CopyDesc *dg = upload_vec(gather, s);
-  copy2d_batched(dg, (int)gather.size(), s);
-  cudaFreeAsync(dg, s);
+  int *d_perm = upload_vec(perms, s);
+  {
+    int at = 0, widest = 1;
+    for (int p = 0; p < np; ++p) {
+      io[p].perm = d_perm + at;
+      at += ranks[p];
+      widest = std::max(widest, ranks[p]);
+    }
+    for_problems([&](const BjIo *d, int n) {
+      bj_gather_kernel<<<dim3((unsigned)std::min(widest, 64), (unsigned)n), 256, 0, s>>>(d);
+    });
+  }
+  cudaFreeAsync(d_perm, s);
   // singular values (one upload, scattered by one copy launch), ranks and
   // sweeps (one launch)
   bool failed = false;
@@ -853,18 +892,16 @@ void block_jacobi_svd(const std::vector<BjProb> &probs, double tol, int max_swee
     }
     double *ds = upload_vec(hs, s);
     std::vector<CopyDesc> sc;
-    std::vector<BjIntOut> io;
+    std::vector<BjIntOut> ints;
     for (int p = 0; p < np; ++p) {
       sc.push_back(CopyDesc{ds + so[p], wk[p].L, probs[p].sigma, wk[p].L, wk[p].L, 1});
-      io.push_back(BjIntOut{probs[p].rank, probs[p].sweeps, ranks[p], sweeps[p]});
+      ints.push_back(BjIntOut{probs[p].rank, probs[p].sweeps, ranks[p], sweeps[p]});
       failed = failed || !wk[p].converged;
     }
-    CopyDesc *dsc = upload_vec(sc, s);
-    copy2d_batched(dsc, (int)sc.size(), s);
-    BjIntOut *dio = upload_vec(io, s);
+    copy2d_batched(sc, s);
+    BjIntOut *dio = upload_vec(ints, s);
     bj_int_out_kernel<<<(np + 127) / 128, 128, 0, s>>>(dio, np);
     HB_LAUNCHED();
-    cudaFreeAsync(dsc, s);
     cudaFreeAsync(dio, s);
     cudaFreeAsync(ds, s);
   }

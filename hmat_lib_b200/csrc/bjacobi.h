@@ -15,8 +15,9 @@ struct BjProb {
   const double *A;
   long long lda;
   int L;
-  double *U;       // out: L x L (ld L), left vectors times sigma, descending sigma
-  double *V;       // out: L x L (ld L), right vectors
+  double *U;       // out: L x rank (ld L), left vectors times sigma, descending sigma;
+                   //   room for L columns
+  double *V;       // out: L x rank (ld L), right vectors; room for L columns
   double *sigma;   // out: L singular values, descending
   int *rank;       // out (device int): hmat_lib's relative truncation rank
   int *sweeps;     // out (device int, optional): sweeps used; max_sweeps + 1 if not converged

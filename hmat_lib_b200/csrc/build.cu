@@ -106,11 +106,7 @@ void gather_to_host(std::vector<CopyDesc> descs, int stride, double *host, cudaS
     d.cols = 1;
     live.push_back(d);
   }
-  if (!live.empty()) {
-    CopyDesc *dd = upload_vec(live, s);
-    copy2d_batched(dd, (int)live.size(), s);
-    cudaFreeAsync(dd, s);
-  }
+  copy2d_batched(live, s);
   HB_CUDA(cudaMemcpyAsync(host, stage, sizeof(double) * nrow * stride, cudaMemcpyDeviceToHost, s));
   HB_CUDA(cudaStreamSynchronize(s));
   dev_free(stage, s);
@@ -666,11 +662,7 @@ std::vector<std::shared_ptr<DeviceTree>> build_attempt(
           }
           gemm_f64_run(gc, bases, TileShape::M64N128, stream);
           gemm_f64_run(gu, bases, TileShape::M128N64, stream, false);
-          if (!acc.empty()) {
-            CopyDesc *d = upload_vec(acc, stream);
-            add2d_batched(d, (int)acc.size(), 1.0, stream);
-            cudaFreeAsync(d, stream);
-          }
+          add2d_batched(acc, stream);
         }
         std::vector<TsqrProb> tp;
         for (int i : pa) {
@@ -738,9 +730,7 @@ std::vector<std::shared_ptr<DeviceTree>> build_attempt(
         cp.push_back(CopyDesc{work + S.bt + (long long)S.ell * S.n, S.n,
                               work + S.p + (long long)S.ell * S.n, S.n, S.n, wb[i]});
       }
-      CopyDesc *d = upload_vec(cp, stream);
-      copy2d_batched(d, (int)cp.size(), stream);
-      cudaFreeAsync(d, stream);
+      copy2d_batched(cp, stream);
     }
     // 6. P / R_B update
     orthonormalise(false);
@@ -924,11 +914,7 @@ std::vector<std::shared_ptr<DeviceTree>> build_attempt(
     copies.push_back(CopyDesc{eprobs[p].U, B.m, dt.arena + B.u_off, B.m, B.m, B.s});
     copies.push_back(CopyDesc{eprobs[p].V, B.n, dt.arena + B.v_off, B.n, B.n, B.s});
   }
-  if (!copies.empty()) {
-    CopyDesc *d = upload_vec(copies, stream);
-    copy2d_batched(d, (int)copies.size(), stream);
-    cudaFreeAsync(d, stream);
-  }
+  copy2d_batched(copies, stream);
   if (!sk.empty()) {
     // U = Q[:, :ell] (U_R Sigma)[:, :s],  V = P[:, :ell] V_R[:, :s]; the arenas
     // are addressed from the lowest arena address

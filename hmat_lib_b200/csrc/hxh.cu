@@ -31,22 +31,6 @@ namespace {
 
 enum Slot { kA = 0, kB = 1, kWork = 2, kOut = 3 };
 
-template <class T>
-T *upload_vec(const std::vector<T> &v, cudaStream_t s) {
-  T *d = nullptr;
-  HB_CUDA(cudaMallocAsync((void **)&d, sizeof(T) * std::max<size_t>(v.size(), 1), s));
-  if (!v.empty())
-    h2d_async(d, v.data(), sizeof(T) * v.size(), s);
-  return d;
-}
-
-void run_copies(const std::vector<CopyDesc> &c, cudaStream_t s) {
-  if (c.empty()) return;
-  CopyDesc *d = upload_vec(c, s);
-  copy2d_batched(d, (int)c.size(), s);
-  cudaFreeAsync(d, s);
-}
-
 // Blocked Householder QR of Y (m x S), Q written over Y, R (S x S, zeroed by
 // the caller) accumulated: 32-column panels, each orthogonalised against the
 // previous columns twice (coefficients added into R) and then factored by
@@ -88,11 +72,7 @@ void block_qr(const std::vector<BlockQr> &probs, double *base, cudaStream_t s) {
       }
       gemm_f64_run(gc, gb, TileShape::M64N128, s);
       gemm_f64_run(gu, gb, TileShape::M128N64, s, false);
-      if (!acc.empty()) {
-        CopyDesc *d = upload_vec(acc, s);
-        add2d_batched(d, (int)acc.size(), 1.0, s);
-        cudaFreeAsync(d, s);
-      }
+      add2d_batched(acc, s);
     }
     std::vector<TsqrProb> tp;
     for (const BlockQr *p : pa) {
@@ -253,7 +233,7 @@ void recomp_finish(const std::vector<RecompJob> &jobs, const std::vector<int> &r
       gf.seg(pv, kWork, j.v, j.n, 0, kWork, j.jo_v, j.S, 0, j.S);
     }
   }
-  run_copies(cp, s);
+  copy2d_batched(cp, s);
   gemm_f64_run(gf, gb, TileShape::M128N64, s, false);
 }
 
@@ -400,7 +380,7 @@ std::shared_ptr<DeviceTree> hxh_multiply(DeviceTree &A, DeviceTree &B, double to
         if (ao.s > 0)
           cp.push_back(CopyDesc{A.arena + ao.v_off, ao.n, work + xpd[d] + ao.c0, n, ao.n, ao.s});
       }
-    run_copies(cp, s);
+    copy2d_batched(cp, s);
     if (smax_b[d] > 0) {
       if (mixed)
         product_mixed_op(A, ProdOp::N, work + xd[d], smax_b[d], n, work + yd[d], n, s, d + 1);
@@ -447,7 +427,7 @@ std::shared_ptr<DeviceTree> hxh_multiply(DeviceTree &A, DeviceTree &B, double to
         col += t.cols;
       }
     }
-    run_copies(cp, s);
+    copy2d_batched(cp, s);
     gemm_f64_run(gv, gb, TileShape::M128N64, s, false);
   }
 
@@ -492,7 +472,7 @@ std::shared_ptr<DeviceTree> hxh_multiply(DeviceTree &A, DeviceTree &B, double to
     const int m = go.leaf_m[i];
     if (m) cp.push_back(CopyDesc{work + leaf_out[i], m, out->arena + out->leaves[i].off, m, m, m});
   }
-  run_copies(cp, s);
+  copy2d_batched(cp, s);
   std::vector<long long> uo(nb), vo(nb);
   for (int b = 0; b < nb; ++b) {
     uo[b] = out->g.blocks[b].u_off;

@@ -822,24 +822,32 @@ jacobi_qrp_kernel(const JacobiProb *__restrict__ probs, JacobiParams prm, int *s
   }
 }
 
+// dst (+)= src for every descriptor: CTAs take columns, threads rows (no
+// division per element).
+template <bool kAdd>
 __global__ void copy2d_kernel(const CopyDesc *__restrict__ descs) {
   const CopyDesc D = descs[blockIdx.y];
-  const long long total = (long long)D.rows * D.cols;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    const long long r = e % D.rows, c = e / D.rows;
-    D.dst[r + c * D.ldd] = D.src[r + c * D.lds];
+  for (int c = blockIdx.x; c < D.cols; c += gridDim.x) {
+    const double *src = D.src + (long long)c * D.lds;
+    double *dst = D.dst + (long long)c * D.ldd;
+    for (int r = threadIdx.x; r < D.rows; r += blockDim.x) dst[r] = kAdd ? dst[r] + src[r] : src[r];
   }
 }
 
-__global__ void add2d_kernel(const CopyDesc *__restrict__ descs, double alpha) {
-  const CopyDesc D = descs[blockIdx.y];
-  const long long total = (long long)D.rows * D.cols;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    const long long r = e % D.rows, c = e / D.rows;
-    D.dst[r + c * D.ldd] += alpha * D.src[r + c * D.lds];
+template <bool kAdd>
+void run_copies2d(const std::vector<CopyDesc> &descs, cudaStream_t stream) {
+  if (descs.empty()) return;
+  int cols = 1;
+  for (const CopyDesc &d : descs) cols = std::max(cols, d.cols);
+  CopyDesc *d = nullptr;
+  HB_CUDA(cudaMallocAsync((void **)&d, sizeof(CopyDesc) * descs.size(), stream));
+  h2d_async(d, descs.data(), sizeof(CopyDesc) * descs.size(), stream);
+  for (size_t off = 0; off < descs.size(); off += 65535) {
+    dim3 grid((unsigned)std::min(cols, 32), (unsigned)std::min<size_t>(65535, descs.size() - off));
+    copy2d_kernel<kAdd><<<grid, 256, 0, stream>>>(d + off);
+    HB_LAUNCHED();
   }
+  cudaFreeAsync(d, stream);
 }
 
 }  // namespace
@@ -920,24 +928,12 @@ void jacobi_svd_batched(const std::vector<JacobiProb> &probs, const JacobiParams
   cudaFreeAsync(d, stream);
 }
 
-void copy2d_batched(const CopyDesc *d_descs, int n, cudaStream_t stream) {
-  if (n <= 0) return;
-  for (int off = 0; off < n; off += 65535) {
-    dim3 grid(32, std::min(65535, n - off));
-    copy2d_kernel<<<grid, 256, 0, stream>>>(d_descs + off);
-    HB_LAUNCHED();
-  }
+void copy2d_batched(const std::vector<CopyDesc> &descs, cudaStream_t stream) {
+  run_copies2d<false>(descs, stream);
 }
 
-}  // namespace hb
-
-namespace hb {
-void add2d_batched(const CopyDesc *d_descs, int n, double alpha, cudaStream_t stream) {
-  if (n <= 0) return;
-  for (int off = 0; off < n; off += 65535) {
-    dim3 grid(32, std::min(65535, n - off));
-    add2d_kernel<<<grid, 256, 0, stream>>>(d_descs + off, alpha);
-    HB_LAUNCHED();
-  }
+void add2d_batched(const std::vector<CopyDesc> &descs, cudaStream_t stream) {
+  run_copies2d<true>(descs, stream);
 }
+
 }  // namespace hb

@@ -72,9 +72,8 @@ struct CopyDesc {
   int rows, cols;
 };
 
-void copy2d_batched(const CopyDesc *d_descs, int n, cudaStream_t stream);
-
-// dst += alpha * src for every descriptor (same shape rules as CopyDesc).
-void add2d_batched(const CopyDesc *d_descs, int n, double alpha, cudaStream_t stream);
+// dst = src, dst += src for every descriptor (uploaded stream-ordered).
+void copy2d_batched(const std::vector<CopyDesc> &descs, cudaStream_t stream);
+void add2d_batched(const std::vector<CopyDesc> &descs, cudaStream_t stream);
 
 }  // namespace hb

@@ -549,8 +549,7 @@ DeviceTree &transposed_tree(DeviceTree &t, cudaStream_t s) {
     cp.push_back(CopyDesc{t.arena + o.u_off, o.m, tt->arena + B.v_off, B.n, B.n, B.s});
   }
   if (!cp.empty()) {
-    CopyDesc *d = upload(cp, s);
-    copy2d_batched(d, (int)cp.size(), s);
+    copy2d_batched(cp, s);
     // rebalance every block's columns
     long long tot = 0;
     std::vector<long long> off(gt.nblock(), 0);
@@ -578,7 +577,6 @@ DeviceTree &transposed_tree(DeviceTree &t, cudaStream_t s) {
       HB_LAUNCHED();
     }
     HB_CUDA(cudaStreamSynchronize(s));
-    cudaFree(d);
     cudaFree(dbd);
     cudaFree(norms);
   }

@@ -645,9 +645,7 @@ std::unique_ptr<HodlrFactor> hodlr_factorize(std::shared_ptr<DeviceTree> tp, cud
         const BlockDesc &B = g.blocks[block_index(l, j, c)];
         if (B.s) cp.push_back(CopyDesc{t.arena + B.u_off, B.m, tmp + B.r0, n, B.m, B.s});
       }
-    CopyDesc *dcp = upload_tmp(cp, s);
-    copy2d_batched(dcp, (int)cp.size(), s);
-    cudaFreeAsync(dcp, s);
+    copy2d_batched(cp, s);
     apply_leaves_once(*f, tmp, n, Wl, n, w, s);
     for (int lev = h - 1; lev > l; --lev) apply_level_once(*f, lev, Wl, w, n, s);
 
