@@ -108,15 +108,22 @@ cudaMemPool_t scratch_pool() {
   return pool;
 }
 
+namespace {
+constexpr size_t kLarge = size_t(32) << 20;
+// `bytes` of a large allocation rounded up to an eighth of a power of two.
+size_t large_size(size_t bytes) {
+  size_t step = kLarge / 8;
+  while (step * 16 <= bytes) step *= 2;
+  return (bytes + step - 1) / step * step;
+}
+}  // namespace
+
 double *dev_alloc(size_t elems, cudaStream_t stream) {
   keep_pool_memory();
-  constexpr size_t kLarge = size_t(32) << 20;
   size_t bytes = std::max<size_t>(elems, 1) * sizeof(double);
   void *p = nullptr;
   if (bytes >= kLarge) {
-    size_t step = kLarge / 8;
-    while (step * 16 <= bytes) step *= 2;
-    bytes = (bytes + step - 1) / step * step;
+    bytes = large_size(bytes);
     const cudaMemPool_t pool = scratch_pool();
     cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, pool, stream);
     if (e == cudaErrorMemoryAllocation) {
@@ -240,8 +247,11 @@ std::unique_ptr<DeviceTree> dtree_create(const Geometry &g_in, cudaStream_t stre
   // cudaMalloc of the arena had to map fresh pages there.  cudaFree releases
   // these allocations like any other.
   keep_pool_memory();
-  HB_CUDA(cudaMallocAsync((void **)&t->arena, std::max<long long>(off, 1) * sizeof(double),
-                          stream));
+  // (large arenas in rounded sizes, so that a tree of nearly the same ranks
+  // finds the place of one that was freed)
+  size_t bytes = std::max<long long>(off, 1) * sizeof(double);
+  if (bytes >= kLarge) bytes = large_size(bytes);
+  HB_CUDA(cudaMallocAsync((void **)&t->arena, bytes, stream));
   HB_CUDA(cudaMallocAsync((void **)&t->d_leaves,
                           std::max<size_t>(t->leaves.size(), 1) * sizeof(LeafDesc), stream));
   HB_CUDA(cudaMallocAsync((void **)&t->d_blocks,
