@@ -8,8 +8,8 @@
 //
 //  * exact: min(m, n) <= exact_max -> one-sided Jacobi SVD of the block;
 //  * sketched: adaptive blocked randomized range finder.  Each round draws a
-//    Gaussian test matrix Om, forms Y = A Om - Q (B Om) with one pass over
-//    the block, orthonormalises Y panel by panel against the basis Q (block
+//    random test matrix Om (sketch.h), forms Y = A Om - Q (B Om) with one pass
+//    over the block, orthonormalises Y panel by panel against the basis Q (block
 //    classical Gram-Schmidt applied twice, then TSQR), and appends
 //    B^T = A^T Q_new with a second pass.  The columns of B^T are in turn
 //    orthonormalised into P with their coefficients collected in R_B, so
@@ -27,6 +27,7 @@
 #include "build.h"
 #include "jacobi.h"
 #include "rank_mlp.h"
+#include "sketch.h"
 #include "sketch_mixed.h"
 #include "tsqr.h"
 #include "workload.h"
@@ -62,6 +63,7 @@ struct SketchBlock {
   int pred = -1;         // predicted rank (-1: none)
   bool one_shot = false; // first round sized by the predictor, judged at tol
   bool fell_back = false;
+  bool hadamard = false; // A Om by sketch_multiply (sketch.h)
   int mix = -1;          // index in the int8 sketch products (-1: FP64 GEMMs)
 };
 
@@ -351,6 +353,7 @@ std::vector<std::shared_ptr<DeviceTree>> build_attempt(
     S.cap = caps[si];
     S.a_off = blk[b].a0;
     S.mix = mix_of[si];
+    S.hadamard = S.mix < 0 && B.n >= kSketchMinCols;
     sk.push_back(S);
   }
   // ---- learned sizing of the first sketch ---------------------------------------------
@@ -424,6 +427,7 @@ std::vector<std::shared_ptr<DeviceTree>> build_attempt(
     S.c = take((long long)S.cap * kPanel);
     S.rn = take((long long)kPanel * kPanel + kPanel + wb);
   }
+  const long long mixer = take(64 * 64);
   const double ms_features =
       std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - tf0).count();
   const double eta_learned = option("learned_eta", 1.0);
@@ -435,6 +439,12 @@ std::vector<std::shared_ptr<DeviceTree>> build_attempt(
   bases.p[kWork] = work;
   for (int i = 2; i < kGemmBases; ++i) bases.p[i] = work;
   if (!sk.empty()) HB_CUDA(cudaMemsetAsync(work, 0, scratch * sizeof(double), stream));
+  for (const SketchBlock &S : sk)
+    if (S.hadamard) {
+      const std::vector<double> M = sketch_mixer(seed);
+      h2d_async(work + mixer, M.data(), sizeof(double) * M.size(), stream);
+      break;
+    }
   // A block at its cap whose memory-bounded cap is larger: Q, B^T, P and R_B
   // (with its first ell columns) and the round buffers sized by the cap move
   // to a fresh allocation of twice the width, addressed by offsets from
@@ -581,27 +591,42 @@ std::vector<std::shared_ptr<DeviceTree>> build_attempt(
               act.end());
     if (act.empty()) break;
 
-    // 1. Gaussian test matrices
+    // 1. test matrices: in full for the products that read them as matrices
+    auto test_id = [&](const SketchBlock &S) {
+      return ((unsigned long long)S.bid << 24) + (unsigned long long)rounds;
+    };
     std::vector<RandDesc> rd;
-    for (int i : act)
-      rd.push_back(RandDesc{work + sk[i].om, sk[i].n, sk[i].n, wb[i],
-                            ((unsigned long long)sk[i].bid << 24) + (unsigned long long)rounds});
+    std::vector<SketchFill> fd;
+    for (int i : act) {
+      const SketchBlock &S = sk[i];
+      if (!S.hadamard)
+        rd.push_back(RandDesc{work + S.om, S.n, S.n, wb[i], test_id(S)});
+      else if (S.ell > 0)
+        fd.push_back(SketchFill{work + S.om, S.n, S.n, wb[i], test_id(S)});
+    }
     gaussian_fill(rd, seed, stream);
+    sketch_fill(fd, work + mixer, seed, stream);
 
     // 2. Y = A Om written into the new columns of Q; 3. Y -= Q (B Om)
     {
       GemmBatch g1;
+      std::vector<SketchDesc> h1;
       std::vector<SketchMixed::Call> m1;
       for (int i : act) {
         const SketchBlock &S = sk[i];
+        double *y = work + S.q + (long long)S.ell * S.m;   // zero until now
         if (S.mix >= 0) {
-          m1.push_back(SketchMixed::Call{S.mix, work + S.om, S.n, wb[i],
-                                         work + S.q + (long long)S.ell * S.m, S.m});
-          continue;
+          m1.push_back(SketchMixed::Call{S.mix, work + S.om, S.n, wb[i], y, S.m});
+        } else if (S.hadamard) {
+          const BlockDesc &B = blk[S.b].B;
+          h1.push_back(SketchDesc{gen ? nullptr : d_A + S.a_off, S.lda, B.r0, B.c0, S.m, S.n,
+                                  wb[i], y, S.m, test_id(S)});
+        } else {
+          int pr = g1.add(kWork, S.q + (long long)S.ell * S.m, S.m, S.m, wb[i]);
+          g1.seg(pr, aslot, S.a_off, S.lda, 0, kWork, S.om, S.n, 0, S.n);
         }
-        int pr = g1.add(kWork, S.q + (long long)S.ell * S.m, S.m, S.m, wb[i]);
-        g1.seg(pr, aslot, S.a_off, S.lda, 0, kWork, S.om, S.n, 0, S.n);
       }
+      sketch_multiply(h1, work + mixer, gen, seed, stream);
       gemm_f64_run(g1, bases, TileShape::M128N64, stream);
       if (smix) smix->multiply(false, m1, stream);
       // ||A om_c||^2: the scale against which a projected column counts as noise
