@@ -1109,7 +1109,7 @@ def main():
         "fp64": {"value": value_fp64, "unit": "GB/s", "ms_per_step": r64["ms"],
                  "gflops": flops_step / (r64["ms"] * 1e-3) / 1e9,
                  "e2e": bytes_step / e2e_s_fp64 / 1e9,
-                 "roofline": {"bound": "fp64", "kernel": f"gemm_f64_mma_kernel ({dom64})",
+                 "roofline": {"bound": "fp64", "kernel": f"gemm_f64_ws_kernel ({dom64})",
                               "achieved": achieved64, "peak": peak64, "unit": "TFLOP/s",
                               "frac": achieved64 / peak64,
                               "traffic": traffic_ratio64[dom64] * bytes64[dom64],

@@ -1048,7 +1048,8 @@ std::vector<std::shared_ptr<DeviceTree>> build_batch(const std::vector<BuildInpu
   // kernel_form_frac) is formed once: the sketch rounds read each entry twice
   // a round, and computing it (a square root, an exponential, a division) in
   // the GEMM's loader costs several times the multiply-adds it feeds.  n = 8192,
-  // 3D, 25 rounds: 99 ms of rounds with generated operands, 70 with a formed matrix.
+  // 3D, 25 rounds: 99 ms of rounds with generated operands, 70 with a formed
+  // matrix (66 now).
   if (gen && !in[0].g.blocks.empty()) {
     const int n = in[0].g.n;
     const double bytes = 8.0 * (double)n * n;

@@ -262,7 +262,8 @@ gemm_f64_kernel(const GemmSeg *__restrict__ segs, const GemmProb *__restrict__ p
 // warps of a CTA issue no MMAs.  H X at n = 32768, k = 256 (ranks 38 to 349):
 // 1640 us without any of this, 1512 us without MMAs on padding, 1370 us so
 // (28.7 TFLOP/s; cuBLAS DGEMM 35.5); H x H at n = 16384 (many products of 5 to
-// 40 columns) 3.44, 2.90, 2.47 ms.
+// 40 columns) 3.44, 2.90, 2.47 ms.  With loader warps beside the MMA warps
+// (gemm_f64_ws_kernel) 1250 us (31.5 TFLOP/s in the larger launch) and 2.25 ms.
 template <int BM, int BN, int BK>
 struct MmaSmem {
   static constexpr int LDKM = BM + 4;      // [k][m] layout

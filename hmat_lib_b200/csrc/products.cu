@@ -103,7 +103,8 @@ long long product_w_layout(const DeviceTree &t, int k, std::vector<long long> &w
 // Tile shape of a product phase: option product_shape1 / product_shape2
 // (0-4: 128x64, 64x128, 32x128, 32x256, 64x64), else by op and k: up to 64
 // right-hand sides take 64 x 64 tiles (more of them, three stages deep, and no
-// idle half; H^T X and X H at n = 10007, k = 33: 349 -> 265 us).
+// idle half; H^T X and X H at n = 10007, k = 33: 349 -> 265 us;
+// 207 with the GEMM's loader warps).
 TileShape default_shape(ProdOp op, int k, int phase) {
   const int forced =
       (int)(phase == 1 ? option("product_shape1", -1.0) : option("product_shape2", -1.0));
