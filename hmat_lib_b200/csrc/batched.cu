@@ -49,8 +49,11 @@ struct BatchPlan {
   cudaGraphExec_t exec = nullptr;
   long long graph_launches = 0;
   std::string tuned;
+  // a plan runs as soon as it is made, and on any stream after that
+  std::atomic<bool> in_flight{true};
 
   ~BatchPlan() {
+    wait_in_flight(in_flight, device);
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
     ph1.reset();
@@ -227,6 +230,7 @@ void batched_product(const std::vector<std::shared_ptr<DeviceTree>> &trees, Prod
   if (prec == Precision::MIXED)
     HB_REQUIRE(op == ProdOp::N, INPUT_ERROR, "mixed precision is available for Y = H X (op N)");
 
+  for (const auto &t : trees) t->in_flight = true;
   std::lock_guard<std::mutex> lk(g_batch_mutex);
   BatchPlan *P = nullptr;
   for (auto it = g_batch_cache.begin(); it != g_batch_cache.end(); ++it)

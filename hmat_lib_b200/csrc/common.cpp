@@ -41,6 +41,14 @@ int num_sms() {
   return cached;
 }
 
+void wait_in_flight(std::atomic<bool> &in_flight, int device) {
+  if (!in_flight.exchange(false)) return;
+  int current = device;
+  if (cudaGetDevice(&current) == cudaSuccess && current != device) cudaSetDevice(device);
+  if (cudaDeviceSynchronize() != cudaSuccess) (void)cudaGetLastError();
+  if (current != device) cudaSetDevice(current);
+}
+
 double option(const char *name, double dflt) {
   std::lock_guard<std::mutex> lk(g_opt_mutex);
   auto it = opts().find(name);

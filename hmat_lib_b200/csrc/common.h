@@ -3,6 +3,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <atomic>
 #include <cstdint>
 #include <cstdio>
 #include <string>
@@ -67,6 +68,12 @@ long long launches();
   } while (0)
 
 int num_sms();
+
+// Waits for all work on `device` if `in_flight` is set, and clears it: the first
+// step of every destructor whose memory queued work may still use.  cudaFree of
+// cudaMalloc memory waits for the device by itself; of stream-ordered memory it
+// hands the bytes to the next allocation at once.
+void wait_in_flight(std::atomic<bool> &in_flight, int device);
 
 // Runtime knobs (hodlr_b200_set_option).
 double option(const char *name, double dflt);

@@ -482,6 +482,7 @@ std::shared_ptr<DeviceTree> hxh_multiply(DeviceTree &A, DeviceTree &B, double to
   HB_CUDA(cudaStreamSynchronize(s));
   dev_free(work, s);
   HB_CUDA(cudaStreamSynchronize(s));
+  out->in_flight = false;
   return out;
 }
 

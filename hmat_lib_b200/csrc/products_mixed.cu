@@ -588,6 +588,7 @@ DeviceTree &transposed_tree(DeviceTree &t, cudaStream_t s) {
 
 void product_mixed_op(DeviceTree &t, ProdOp op, const double *X, int k, long long ldx, double *Y,
                       long long ldy, cudaStream_t s, int min_depth) {
+  t.in_flight = true;
   if (op == ProdOp::N) {
     product_mixed(t, X, k, ldx, Y, ldy, s, min_depth);
     return;

@@ -150,6 +150,9 @@ int hodlr_b200_build_batched_dev(int count, const int *heights, const int *ns,
                                  const double *const *d_matrices, const int *lds,
                                  double svd_threshold, void *stream, hodlr_b200_tree *out,
                                  int *ierr);
+/* Waits for the device first if a product or solve that uses the tree may
+ * still be queued, so a tree can be freed right after such a call; the same
+ * holds for hodlr_b200_factor_free and hodlr_b200_batched_release. */
 void hodlr_b200_tree_free(hodlr_b200_tree t);
 /* Fills an allocated, empty host tree of the same height with copies of the
  * device factors (library allocator; free with free_tree_data). */
