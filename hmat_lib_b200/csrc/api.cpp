@@ -729,7 +729,7 @@ struct DevFloats {
   float *p = nullptr;
   cudaStream_t s;
   DevFloats(const float *host, size_t n, cudaStream_t st) : s(st) {
-    HB_CUDA(cudaMallocAsync((void **)&p, sizeof(float) * std::max<size_t>(n, 1), s));
+    pool_alloc(&p, sizeof(float) * std::max<size_t>(n, 1), s);
     if (host && n)
       HB_CUDA(cudaMemcpyAsync(p, host, sizeof(float) * n, cudaMemcpyHostToDevice, s));
   }

@@ -182,7 +182,7 @@ void build_fp64(BatchPlan &P, const std::vector<std::shared_ptr<DeviceTree>> &tr
     w_base[i] = w_total;
     w_total += product_w_layout(*trees[i], sig[i].k, w_off[i]);
   }
-  HB_CUDA(cudaMalloc(&P.w, std::max<long long>(w_total, 1) * sizeof(double)));
+  device_alloc(&P.w, std::max<long long>(w_total, 1) * sizeof(double));
   const double *base = P.w;
   for (size_t i = 0; i < n; ++i)
     for (const double *p : {(const double *)trees[i]->arena, sig[i].X, (const double *)sig[i].Y})

@@ -70,7 +70,7 @@ constexpr int kMaxCluster = 8;
 template <class T>
 T *upload_vec(const std::vector<T> &v, cudaStream_t s) {
   T *d = nullptr;
-  HB_CUDA(cudaMallocAsync((void **)&d, sizeof(T) * std::max<size_t>(v.size(), 1), s));
+  pool_alloc(&d, sizeof(T) * std::max<size_t>(v.size(), 1), s);
   if (!v.empty())
     h2d_async(d, v.data(), sizeof(T) * v.size(), s);
   return d;
@@ -704,7 +704,7 @@ void block_jacobi_svd(const std::vector<BjProb> &probs, double tol, int max_swee
   for (int p = 0; p < np; ++p) noff[p] = take(wk[p].Lp);
   double *w = dev_alloc(total, s);
   int *d_rot = nullptr;   // per problem: 1 + the last round that rotated a pair
-  HB_CUDA(cudaMallocAsync((void **)&d_rot, sizeof(int) * np, s));
+  pool_alloc(&d_rot, sizeof(int) * np, s);
   HB_CUDA(cudaMemsetAsync(d_rot, 0, sizeof(int) * np, s));
   // ---- X = A^T, V = I, thresholds -------------------------------------------------------
   std::vector<NormDesc> nd;

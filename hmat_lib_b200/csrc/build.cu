@@ -41,7 +41,7 @@ enum GB { kA = 0, kWork = 1, kArena = 2 };
 template <class T>
 T *upload_vec(const std::vector<T> &v, cudaStream_t s) {
   T *d = nullptr;
-  HB_CUDA(cudaMallocAsync((void **)&d, sizeof(T) * std::max<size_t>(v.size(), 1), s));
+  pool_alloc(&d, sizeof(T) * std::max<size_t>(v.size(), 1), s);
   if (!v.empty())
     h2d_async(d, v.data(), sizeof(T) * v.size(), s);
   return d;
@@ -67,29 +67,44 @@ struct SketchBlock {
   int mix = -1;          // index in the int8 sketch products (-1: FP64 GEMMs)
 };
 
-// Device memory free or held unused by the device's default stream-ordered
-// pool or the library's scratch pool (bytes).
-double device_avail_bytes() {
-  size_t free_b = 0, total_b = 0;
-  HB_CUDA(cudaMemGetInfo(&free_b, &total_b));
-  double avail = (double)free_b;
-  int dev = 0;
-  cudaMemPool_t pools[2] = {nullptr, scratch_pool()};
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetDefaultMemPool(&pools[0], dev) != cudaSuccess)
-    pools[0] = nullptr;
-  for (cudaMemPool_t pool : pools) {
-    if (!pool) continue;
-    uint64_t reserved = 0, used = 0;
-    if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) ==
-            cudaSuccess &&
-        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess &&
-        reserved > used)
-      avail += (double)(reserved - used);
+// What large scratch can still get (bytes): device memory that is free or held
+// unused by the scratch pool.  What the default pool holds unused (arenas of
+// freed trees) is out of that pool's reach until it is given back to the device,
+// which fits() does where it decides.  Asked once and then kept up by take().
+class ScratchBudget {
+ public:
+  bool fits(double need) {
+    if (avail_ < 0.0) ask();
+    if (need > avail_ && need <= avail_ + kept_) {
+      HB_CUDA(cudaMemPoolTrimTo(default_pool_, 0));
+      ask();
+    }
+    return need <= avail_;
   }
-  (void)cudaGetLastError();
-  return avail;
-}
+  void take(double bytes) { avail_ = std::max(0.0, avail_ - bytes); }
+  void forget() { avail_ = -1.0; }
+  double total() const { return avail_ + kept_; }
+
+ private:
+  double avail_ = -1.0, kept_ = 0.0;
+  cudaMemPool_t default_pool_ = nullptr;
+
+  static double unused(cudaMemPool_t pool) {
+    uint64_t reserved = 0, used = 0;
+    HB_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved));
+    HB_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
+    return reserved > used ? (double)(reserved - used) : 0.0;
+  }
+  void ask() {
+    int dev = 0;
+    HB_CUDA(cudaGetDevice(&dev));
+    HB_CUDA(cudaDeviceGetDefaultMemPool(&default_pool_, dev));
+    size_t free_b = 0, total_b = 0;
+    HB_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    avail_ = (double)free_b + unused(scratch_pool());
+    kept_ = unused(default_pool_);
+  }
+};
 
 // Reads descs[i] (a column of up to `stride` doubles each, dst unused) into
 // row i of `host` (rows of `stride` doubles): one gather launch into
@@ -151,7 +166,7 @@ std::vector<float> block_features(const std::vector<SketchBlock> &sk,
   double *w = dev_alloc(total, stream);
   HB_CUDA(cudaMemsetAsync(w, 0, sizeof(double) * total, stream));
   int *d_rank = nullptr;
-  HB_CUDA(cudaMallocAsync((void **)&d_rank, sizeof(int) * (nsk + 1), stream));
+  pool_alloc(&d_rank, sizeof(int) * (nsk + 1), stream);
   HB_CUDA(cudaMemsetAsync(d_rank, 0, sizeof(int) * (nsk + 1), stream));
   std::vector<RandDesc> rd;
   for (int i = 0; i < nsk; ++i)
@@ -370,8 +385,7 @@ std::vector<std::shared_ptr<DeviceTree>> build_attempt(
     if (have_model) {
       const int nsk = (int)sk.size();
       float *dbuf = nullptr;
-      HB_CUDA(cudaMallocAsync((void **)&dbuf, sizeof(float) * (kRankParams + nsk * (kRankIn + 1)),
-                              stream));
+      pool_alloc(&dbuf, sizeof(float) * (kRankParams + nsk * (kRankIn + 1)), stream);
       HB_CUDA(cudaMemcpyAsync(dbuf, model.data(), sizeof(float) * kRankParams,
                               cudaMemcpyHostToDevice, stream));
       HB_CUDA(cudaMemcpyAsync(dbuf + kRankParams, feats.data(), sizeof(float) * nsk * kRankIn,
@@ -452,7 +466,7 @@ std::vector<std::shared_ptr<DeviceTree>> build_attempt(
   std::vector<double *> grown;
   const double mem_frac = option("sketch_mem_frac", 0.6);
   double limited_avail = -1.0;   // device memory seen by the first growth that did not fit
-  double round_avail = -1.0;     // device memory left to this round's growths (-1: not asked yet)
+  ScratchBudget budget;          // of this round's growths
   auto grow = [&](SketchBlock &S, int limit) {
     const long long wbw = std::max(S.first_w, w_next);
     const long long m = S.m, n = S.n, e = S.ell;
@@ -466,27 +480,26 @@ std::vector<std::shared_ptr<DeviceTree>> build_attempt(
     };
     // twice the width, else smaller steps, whichever fits the memory budget
     // together with the block's core SVD (about five c2^2 doubles)
-    if (round_avail < 0.0) round_avail = cap_opt > 0 ? 1e300 : device_avail_bytes();
-    const double avail = round_avail;
     int c2 = 0;
     long long parts[5];
     for (int cand : {2 * S.cap, S.cap + S.cap / 2, S.cap + 256, S.cap + kPanel}) {
       const int c = std::min(limit, std::max(cand, S.cap + kPanel) / kPanel * kPanel);
       if (c <= S.cap) continue;
-      if (8.0 * ((double)layout(c, parts) + 5.0 * (double)c * c) <= mem_frac * avail) {
+      const double need = 8.0 * ((double)layout(c, parts) + 5.0 * (double)c * c);
+      if (cap_opt > 0 || (mem_frac > 0.0 && budget.fits(need / mem_frac))) {
         c2 = c;
         break;
       }
     }
     if (c2 == 0) {
-      if (limited_avail < 0.0) limited_avail = avail;
+      if (limited_avail < 0.0) limited_avail = std::max(0.0, budget.total());
       return;
     }
     const long long total = layout(c2, parts);
     const long long sq = parts[0], sb = parts[1], sr = parts[2], st = parts[3];
     double *g = dev_alloc(total, stream);
     grown.push_back(g);
-    round_avail = std::max(0.0, round_avail - 8.0 * (double)total);
+    if (cap_opt <= 0) budget.take((double)scratch_bytes(total));
     HB_CUDA(cudaMemsetAsync(g, 0, sizeof(double) * total, stream));
     const long long base = (long long)(g - work);
     const long long q = base, bt = q + sq, pp = bt + sb, rb = pp + sb, t = rb + sr, c = t + st;
@@ -514,7 +527,7 @@ std::vector<std::shared_ptr<DeviceTree>> build_attempt(
   // used by every Jacobi problem in the same order
   int *d_int = nullptr;
   const int n_int = (int)exact.size() + (int)sk.size() + 1;
-  HB_CUDA(cudaMallocAsync((void **)&d_int, sizeof(int) * 2 * n_int, stream));
+  pool_alloc(&d_int, sizeof(int) * 2 * n_int, stream);
   HB_CUDA(cudaMemsetAsync(d_int, 0, sizeof(int) * 2 * n_int, stream));
   int *d_status = d_int + n_int - 1;
   int *d_sweeps = d_int + n_int;
@@ -577,7 +590,7 @@ std::vector<std::shared_ptr<DeviceTree>> build_attempt(
       if (!sk[i].done) act.push_back((int)i);
     if (act.empty()) break;
     std::vector<int> wb(sk.size(), 0);
-    round_avail = -1.0;
+    budget.forget();
     for (int i : act) {
       const int wr = rounds == 0 ? sk[i].first_w : w_next;
       if (sk[i].ell >= sk[i].cap && sk[i].cap < memcap[i]) grow(sk[i], memcap[i]);
@@ -1053,8 +1066,8 @@ std::vector<std::shared_ptr<DeviceTree>> build_batch(const std::vector<BuildInpu
   // matrix (66 now).
   if (gen && !in[0].g.blocks.empty()) {
     const int n = in[0].g.n;
-    const double bytes = 8.0 * (double)n * n;
-    if (bytes <= option("kernel_form_frac", 0.0625) * device_avail_bytes()) {
+    const double bytes = 8.0 * (double)n * n, frac = option("kernel_form_frac", 0.0625);
+    if (frac > 0.0 && ScratchBudget().fits(bytes / frac)) {
       struct Matrix {
         double *p;
         cudaStream_t s;

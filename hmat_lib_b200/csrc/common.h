@@ -69,6 +69,20 @@ long long launches();
 
 int num_sms();
 
+// Device memory: stream-ordered from the device's default pool, or by cudaMalloc.
+// When the device is out of memory, both first give back to it what the library's
+// pools hold unused (dtree.cu).
+void *pool_alloc(size_t bytes, cudaStream_t stream);
+void *device_alloc(size_t bytes);
+template <class T>
+void pool_alloc(T **p, size_t bytes, cudaStream_t stream) {
+  *p = static_cast<T *>(pool_alloc(bytes, stream));
+}
+template <class T>
+void device_alloc(T **p, size_t bytes) {
+  *p = static_cast<T *>(device_alloc(bytes));
+}
+
 // Waits for all work on `device` if `in_flight` is set, and clears it: the first
 // step of every destructor whose memory queued work may still use.  cudaFree of
 // cudaMalloc memory waits for the device by itself; of stream-ordered memory it

@@ -85,8 +85,9 @@ void keep_pool_memory() {
 // of a row of n = 32768 builds (170 ms of work each then, 115 now).  Here everything is free
 // again when a call ends, and sizes are rounded up to an eighth of a power of
 // two, so the next call finds the same blocks.  The pool keeps at most half of
-// the device's memory mapped (nothing with option pool_keep = 0), and gives all
-// of it back when an allocation would fail otherwise.
+// the device's memory mapped (nothing with option pool_keep = 0).  What one pool
+// keeps the other cannot use: an allocation that fails makes both give it back
+// (allocate()).
 cudaMemPool_t scratch_pool() {
   static std::mutex mu;
   static std::map<int, cudaMemPool_t> pools;
@@ -119,26 +120,54 @@ size_t large_size(size_t bytes) {
 }
 }  // namespace
 
+namespace {
+// Runs `alloc` (false).  When the device is out of memory, waits for its work,
+// so that everything freed is free, gives back what the default and the scratch
+// pool hold unused, and runs alloc(true), the last try, without rounding.
+template <class F>
+void allocate(F alloc) {
+  cudaError_t e = alloc(false);
+  if (e == cudaErrorMemoryAllocation) {
+    (void)cudaGetLastError();
+    int dev = 0;
+    cudaMemPool_t pool = nullptr;
+    if (cudaDeviceSynchronize() != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetDefaultMemPool(&pool, dev) != cudaSuccess ||
+        cudaMemPoolTrimTo(pool, 0) != cudaSuccess || cudaMemPoolTrimTo(scratch_pool(), 0) != cudaSuccess)
+      (void)cudaGetLastError();
+    e = alloc(true);
+  }
+  HB_CUDA(e);
+}
+}  // namespace
+
+size_t scratch_bytes(size_t elems) {
+  const size_t bytes = std::max<size_t>(elems, 1) * sizeof(double);
+  return bytes >= kLarge ? large_size(bytes) : bytes;
+}
+
 double *dev_alloc(size_t elems, cudaStream_t stream) {
   keep_pool_memory();
-  size_t bytes = std::max<size_t>(elems, 1) * sizeof(double);
+  const size_t bytes = std::max<size_t>(elems, 1) * sizeof(double);
+  if (bytes < kLarge) return (double *)pool_alloc(bytes, stream);
   void *p = nullptr;
-  if (bytes >= kLarge) {
-    bytes = large_size(bytes);
-    const cudaMemPool_t pool = scratch_pool();
-    cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, pool, stream);
-    if (e == cudaErrorMemoryAllocation) {
-      // memory that other work has released but not returned
-      (void)cudaGetLastError();
-      HB_CUDA(cudaStreamSynchronize(stream));
-      HB_CUDA(cudaMemPoolTrimTo(pool, 0));
-      e = cudaMallocFromPoolAsync(&p, std::max<size_t>(elems, 1) * sizeof(double), pool, stream);
-    }
-    HB_CUDA(e);
-    return (double *)p;
-  }
-  HB_CUDA(cudaMallocAsync(&p, bytes, stream));
+  const cudaMemPool_t pool = scratch_pool();
+  allocate([&](bool exact) {
+    return cudaMallocFromPoolAsync(&p, exact ? bytes : large_size(bytes), pool, stream);
+  });
   return (double *)p;
+}
+
+void *pool_alloc(size_t bytes, cudaStream_t stream) {
+  void *p = nullptr;
+  allocate([&](bool) { return cudaMallocAsync(&p, bytes, stream); });
+  return p;
+}
+
+void *device_alloc(size_t bytes) {
+  void *p = nullptr;
+  allocate([&](bool) { return cudaMalloc(&p, bytes); });
+  return p;
 }
 
 void dev_free(void *p, cudaStream_t stream) {
@@ -249,14 +278,14 @@ std::unique_ptr<DeviceTree> dtree_create(const Geometry &g_in, cudaStream_t stre
   // these allocations like any other.
   keep_pool_memory();
   // (large arenas in rounded sizes, so that a tree of nearly the same ranks
-  // finds the place of one that was freed)
-  size_t bytes = std::max<long long>(off, 1) * sizeof(double);
-  if (bytes >= kLarge) bytes = large_size(bytes);
-  HB_CUDA(cudaMallocAsync((void **)&t->arena, bytes, stream));
-  HB_CUDA(cudaMallocAsync((void **)&t->d_leaves,
-                          std::max<size_t>(t->leaves.size(), 1) * sizeof(LeafDesc), stream));
-  HB_CUDA(cudaMallocAsync((void **)&t->d_blocks,
-                          std::max<size_t>(g.blocks.size(), 1) * sizeof(BlockDesc), stream));
+  // finds the place of one that was freed, unless only the exact size fits)
+  allocate([&](bool exact) {
+    return cudaMallocAsync((void **)&t->arena,
+                           exact ? std::max<long long>(off, 1) * sizeof(double) : scratch_bytes(off),
+                           stream);
+  });
+  pool_alloc(&t->d_leaves, std::max<size_t>(t->leaves.size(), 1) * sizeof(LeafDesc), stream);
+  pool_alloc(&t->d_blocks, std::max<size_t>(g.blocks.size(), 1) * sizeof(BlockDesc), stream);
   HB_CUDA(cudaMemcpyAsync(t->d_leaves, t->leaves.data(), t->leaves.size() * sizeof(LeafDesc),
                           cudaMemcpyHostToDevice, stream));
   if (!g.blocks.empty())

@@ -92,6 +92,7 @@ cudaStream_t lib_stream();
 // pool (once per device; option pool_keep).
 void keep_pool_memory();
 double *dev_alloc(size_t elems, cudaStream_t stream);
+size_t scratch_bytes(size_t elems);   // that dev_alloc takes for `elems` doubles
 // The pool that large scratch comes from.
 cudaMemPool_t scratch_pool();
 void dev_free(void *p, cudaStream_t stream);

@@ -990,7 +990,7 @@ void gemm_plan_build(GemmPlan &plan, const GemmBatch &batch, TileShape shape, KS
   plan.stream = stream;
   // stream-ordered in both cases (a cudaMalloc stops the device); a kept plan
   // is ready for any stream after the synchronisation below
-  HB_CUDA(cudaMallocAsync(&plan.dev, total, stream));
+  pool_alloc(&plan.dev, total, stream);
   char *base = (char *)plan.dev;
   plan.segs = (GemmSeg *)base;
   plan.probs = (GemmProb *)(base + align_up(bs, 256));

@@ -158,7 +158,7 @@ std::vector<int> recomp_run(const std::vector<RecompJob> &jobs, double *work, do
   }
   std::vector<JacobiProb> jp;
   int *d_int = nullptr;
-  HB_CUDA(cudaMallocAsync((void **)&d_int, sizeof(int) * (nj + 1), s));
+  pool_alloc(&d_int, sizeof(int) * (nj + 1), s);
   HB_CUDA(cudaMemsetAsync(d_int, 0, sizeof(int) * (nj + 1), s));
   for (int i = 0; i < nj; ++i) {
     const RecompJob &j = jobs[i];

@@ -840,7 +840,7 @@ void run_copies2d(const std::vector<CopyDesc> &descs, cudaStream_t stream) {
   int cols = 1;
   for (const CopyDesc &d : descs) cols = std::max(cols, d.cols);
   CopyDesc *d = nullptr;
-  HB_CUDA(cudaMallocAsync((void **)&d, sizeof(CopyDesc) * descs.size(), stream));
+  pool_alloc(&d, sizeof(CopyDesc) * descs.size(), stream);
   h2d_async(d, descs.data(), sizeof(CopyDesc) * descs.size(), stream);
   for (size_t off = 0; off < descs.size(); off += 65535) {
     dim3 grid((unsigned)std::min(cols, 32), (unsigned)std::min<size_t>(65535, descs.size() - off));
@@ -915,7 +915,7 @@ void jacobi_svd_batched(const std::vector<JacobiProb> &probs, const JacobiParams
       list.push_back(p);
     }
   JacobiProb *d = nullptr;
-  HB_CUDA(cudaMallocAsync((void **)&d, sizeof(JacobiProb) * list.size(), stream));
+  pool_alloc(&d, sizeof(JacobiProb) * list.size(), stream);
   h2d_async(d, list.data(), sizeof(JacobiProb) * list.size(), stream);
   if (nsmall > 0) {
     if (small_r <= 128)

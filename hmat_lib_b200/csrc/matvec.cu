@@ -194,8 +194,8 @@ void matvec_f64(DeviceTree &t, const double *x, double *y, cudaStream_t s) {
       std::copy(woff.begin(), woff.end(), (int *)host.data());
       std::copy(items.begin(), items.end(), (MvItem *)(host.data() + wb));
       if (!t.mv_w)
-        HB_CUDA(cudaMalloc((void **)&t.mv_w, sizeof(double) * std::max<long long>(total, 1)));
-      HB_CUDA(cudaMalloc((void **)&t.mv_woff, host.size()));
+        device_alloc(&t.mv_w, sizeof(double) * std::max<long long>(total, 1));
+      device_alloc(&t.mv_woff, host.size());
       t.mv_items = (MvItem *)((char *)t.mv_woff + wb);
       HB_CUDA(cudaMemcpyAsync(t.mv_woff, host.data(), host.size(), cudaMemcpyHostToDevice, s));
       HB_CUDA(cudaStreamSynchronize(s));

@@ -701,7 +701,7 @@ MaxBatch ozaki_max_batch(std::vector<MaxJob> jobs, cudaStream_t stream) {
   }
   b.n = (int)jobs.size();
   if (b.n) {
-    HB_CUDA(cudaMalloc((void **)&b.d, sizeof(MaxJob) * jobs.size()));
+    device_alloc(&b.d, sizeof(MaxJob) * jobs.size());
     HB_CUDA(cudaMemcpyAsync(b.d, jobs.data(), sizeof(MaxJob) * jobs.size(), cudaMemcpyHostToDevice,
                             stream));
   }
@@ -721,7 +721,7 @@ SliceBatch ozaki_slice_batch(std::vector<SliceJob> jobs, cudaStream_t stream) {
   }
   b.n = (int)jobs.size();
   if (b.n) {
-    HB_CUDA(cudaMalloc((void **)&b.d, sizeof(SliceJob) * jobs.size()));
+    device_alloc(&b.d, sizeof(SliceJob) * jobs.size());
     HB_CUDA(cudaMemcpyAsync(b.d, jobs.data(), sizeof(SliceJob) * jobs.size(),
                             cudaMemcpyHostToDevice, stream));
   }

@@ -130,8 +130,7 @@ ProductPlan &product_plan(DeviceTree &t, ProdOp op, int k, long long ldx, long l
   std::vector<long long> w_off;
   const long long w_total = product_w_layout(t, k, w_off);
   plan->w_elems = w_total;
-  HB_CUDA(cudaMallocAsync((void **)&plan->w, std::max<long long>(w_total, 1) * sizeof(double),
-                          stream));
+  pool_alloc(&plan->w, std::max<long long>(w_total, 1) * sizeof(double), stream);
   GemmBatch p1, p2;
   append_product(p1, p2, t, op, k, ldx, ldy, ProductSlots{kArena, kX, kY, kW, 0, 0, 0, 0}, w_off,
                  min_depth);

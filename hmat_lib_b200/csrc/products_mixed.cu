@@ -36,7 +36,7 @@ long long cdiv(long long a, long long b) { return (a + b - 1) / b; }
 template <class T>
 T *upload(const std::vector<T> &v, cudaStream_t s) {
   T *d = nullptr;
-  HB_CUDA(cudaMalloc((void **)&d, sizeof(T) * std::max<size_t>(v.size(), 1)));
+  device_alloc(&d, sizeof(T) * std::max<size_t>(v.size(), 1));
   if (!v.empty())
     HB_CUDA(cudaMemcpyAsync(d, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, s));
   return d;
@@ -45,7 +45,7 @@ T *upload(const std::vector<T> &v, cudaStream_t s) {
 template <class T>
 T *dalloc(long long count) {
   T *d = nullptr;
-  HB_CUDA(cudaMalloc((void **)&d, sizeof(T) * std::max<long long>(count, 1)));
+  device_alloc(&d, sizeof(T) * std::max<long long>(count, 1));
   return d;
 }
 
@@ -558,7 +558,7 @@ DeviceTree &transposed_tree(DeviceTree &t, cudaStream_t s) {
       tot += 2LL * tt->g.blocks[b].s;
     }
     double *norms = nullptr;
-    HB_CUDA(cudaMalloc((void **)&norms, sizeof(double) * std::max(tot, 1LL)));
+    device_alloc(&norms, sizeof(double) * std::max(tot, 1LL));
     std::vector<NormDesc> nd;
     std::vector<BalanceDesc> bd;
     for (int b = 0; b < gt.nblock(); ++b) {

@@ -220,7 +220,7 @@ __global__ void adam_kernel(float *params, const float *grad, float *m, float *v
 
 struct DevF {
   float *p = nullptr;
-  explicit DevF(size_t n) { HB_CUDA(cudaMalloc((void **)&p, sizeof(float) * std::max<size_t>(n, 1))); }
+  explicit DevF(size_t n) { device_alloc(&p, sizeof(float) * std::max<size_t>(n, 1)); }
   ~DevF() {
     if (p) cudaFree(p);
   }
@@ -252,7 +252,7 @@ void rank_mlp_gradient(const float *d_params, const float *d_x, const float *d_t
     configured = true;
   }
   float *partial = nullptr;
-  HB_CUDA(cudaMallocAsync((void **)&partial, sizeof(float) * nblocks * (kRankParams + 1), stream));
+  pool_alloc(&partial, sizeof(float) * nblocks * (kRankParams + 1), stream);
   gradient_kernel<<<nblocks, kGradThreads, smem, stream>>>(d_params, d_x, d_t, n, partial);
   HB_LAUNCHED();
   reduce_partials_kernel<<<(kRankParams + 256) / 256, 256, 0, stream>>>(partial, nblocks, d_grad,

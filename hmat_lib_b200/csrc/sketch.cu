@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(kGroup) sketch_fill_kernel(const FillJob *__re
 template <class T>
 T *upload(const std::vector<T> &v, cudaStream_t s) {
   T *d = nullptr;
-  HB_CUDA(cudaMallocAsync((void **)&d, sizeof(T) * v.size(), s));
+  pool_alloc(&d, sizeof(T) * v.size(), s);
   h2d_async(d, v.data(), sizeof(T) * v.size(), s);
   return d;
 }

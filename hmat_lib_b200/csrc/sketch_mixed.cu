@@ -14,7 +14,7 @@ int pad16(int x) { return (x + 15) / 16 * 16; }
 template <class T>
 T *upload(const std::vector<T> &v, cudaStream_t s, std::vector<void *> &keep) {
   T *d = nullptr;
-  HB_CUDA(cudaMalloc((void **)&d, sizeof(T) * std::max<size_t>(v.size(), 1)));
+  device_alloc(&d, sizeof(T) * std::max<size_t>(v.size(), 1));
   keep.push_back(d);
   if (!v.empty())
     h2d_async(d, v.data(), sizeof(T) * v.size(), s);
@@ -49,12 +49,12 @@ SketchMixed::SketchMixed(const std::vector<SketchMixedBlock> &blocks, cudaStream
   // stream-ordered (the device's pool, kept mapped): a synchronous cudaMalloc
   // of the slices (gigabytes) competed with the pool for physical memory
   keep_pool_memory();
-  HB_CUDA(cudaMallocAsync((void **)&slices_, std::max<long long>(bytes, 1), s));
-  HB_CUDA(cudaMallocAsync((void **)&exps_, sizeof(int) * std::max<long long>(nexp, 1), s));
-  HB_CUDA(cudaMallocAsync((void **)&status_, sizeof(int), s));
+  pool_alloc(&slices_, std::max<long long>(bytes, 1), s);
+  pool_alloc(&exps_, sizeof(int) * std::max<long long>(nexp, 1), s);
+  pool_alloc(&status_, sizeof(int), s);
   HB_CUDA(cudaMemsetAsync(status_, 0, sizeof(int), s));
   unsigned long long *maxabs = nullptr;
-  HB_CUDA(cudaMallocAsync((void **)&maxabs, sizeof(unsigned long long) * std::max(nexp, 1LL), s));
+  pool_alloc(&maxabs, sizeof(unsigned long long) * std::max(nexp, 1LL), s);
   HB_CUDA(cudaMemsetAsync(maxabs, 0, sizeof(unsigned long long) * std::max(nexp, 1LL), s));
   std::vector<MaxJob> mj;
   std::vector<SliceJob> rows, cols;
@@ -112,9 +112,9 @@ void SketchMixed::multiply(bool transA, const std::vector<Call> &calls, cudaStre
   uint8_t *xsl = nullptr;
   unsigned long long *xmax = nullptr;
   int *xexp = nullptr;
-  HB_CUDA(cudaMallocAsync((void **)&xsl, std::max(sbytes, 1LL), s));
-  HB_CUDA(cudaMallocAsync((void **)&xmax, sizeof(unsigned long long) * std::max(nw_total, 1LL), s));
-  HB_CUDA(cudaMallocAsync((void **)&xexp, sizeof(int) * std::max(nw_total, 1LL), s));
+  pool_alloc(&xsl, std::max(sbytes, 1LL), s);
+  pool_alloc(&xmax, sizeof(unsigned long long) * std::max(nw_total, 1LL), s);
+  pool_alloc(&xexp, sizeof(int) * std::max(nw_total, 1LL), s);
   HB_CUDA(cudaMemsetAsync(xmax, 0, sizeof(unsigned long long) * std::max(nw_total, 1LL), s));
   std::vector<MaxJob> mj;
   std::vector<SliceJob> sj;

@@ -351,7 +351,7 @@ __global__ void eye_kernel(const EyeDesc *__restrict__ d) {
 template <class T>
 T *upload_tmp(const std::vector<T> &v, cudaStream_t s) {
   T *d = nullptr;
-  HB_CUDA(cudaMallocAsync((void **)&d, sizeof(T) * std::max<size_t>(v.size(), 1), s));
+  pool_alloc(&d, sizeof(T) * std::max<size_t>(v.size(), 1), s);
   if (!v.empty())
     h2d_async(d, v.data(), sizeof(T) * v.size(), s);
   return d;
@@ -568,8 +568,8 @@ SolvePlan &solve_plan(HodlrFactor &f, int k, long long ldb, long long ldx, cudaS
     build_plan(*P->cz.back(), L.cz, shape_vt(k), true, s);     // K = q: split near the root
     build_plan(*P->wx.back(), L.wx, kShapeWx, false, s);
   }
-  HB_CUDA(cudaMallocAsync((void **)&P->T, sizeof(double) * std::max<long long>(scratch, 1), s));
-  HB_CUDA(cudaMallocAsync((void **)&P->Z, sizeof(double) * std::max<long long>(scratch, 1), s));
+  pool_alloc(&P->T, sizeof(double) * std::max<long long>(scratch, 1), s);
+  pool_alloc(&P->Z, sizeof(double) * std::max<long long>(scratch, 1), s);
   HB_CUDA(cudaStreamSynchronize(s));
   auto &ref = *P;
   f.plans[key] = std::move(P);
@@ -613,10 +613,10 @@ std::unique_ptr<HodlrFactor> hodlr_factorize(std::shared_ptr<DeviceTree> tp, cud
       f->q[node_index(d, j)] = q;
       total += align_up((long long)q * q);
     }
-  HB_CUDA(cudaMallocAsync((void **)&f->buf, sizeof(double) * std::max<long long>(total, 1), s));
+  pool_alloc(&f->buf, sizeof(double) * std::max<long long>(total, 1), s);
   HB_CUDA(cudaMemsetAsync(f->buf, 0, sizeof(double) * std::max<long long>(total, 1), s));
   int *d_status = nullptr;
-  HB_CUDA(cudaMallocAsync((void **)&d_status, sizeof(int), s));
+  pool_alloc(&d_status, sizeof(int), s);
   HB_CUDA(cudaMemsetAsync(d_status, 0, sizeof(int), s));
 
   // ---- leaf inverses -----------------------------------------------------------------

@@ -296,7 +296,7 @@ __global__ void colnorm_kernel(const NormDesc *__restrict__ descs) {
 template <class T>
 T *upload(const std::vector<T> &v, cudaStream_t s) {
   T *d = nullptr;
-  HB_CUDA(cudaMallocAsync((void **)&d, sizeof(T) * std::max<size_t>(v.size(), 1), s));
+  pool_alloc(&d, sizeof(T) * std::max<size_t>(v.size(), 1), s);
   h2d_async(d, v.data(), sizeof(T) * v.size(), s);
   return d;
 }
@@ -391,7 +391,7 @@ std::unique_ptr<TsqrPlan, TsqrPlanDeleter> tsqr_plan(const std::vector<TsqrProb>
     }
   }
   lo[probs.size()] = (int)lev.size();
-  if (scratch) HB_CUDA(cudaMallocAsync((void **)&plan->buf, scratch * sizeof(double), s));
+  if (scratch) pool_alloc(&plan->buf, scratch * sizeof(double), s);
   int max_levels = 0;
   for (size_t p = 0; p < probs.size(); ++p) {
     Level *L = lev.data() + lo[p];

@@ -80,7 +80,7 @@ namespace hb {
 void kernel_blocks(const KernelSpec &K, const std::vector<GenBlock> &blocks, cudaStream_t stream) {
   if (blocks.empty()) return;
   GenBlock *d = nullptr;
-  HB_CUDA(cudaMallocAsync((void **)&d, sizeof(GenBlock) * blocks.size(), stream));
+  pool_alloc(&d, sizeof(GenBlock) * blocks.size(), stream);
   HB_CUDA(cudaMemcpyAsync(d, blocks.data(), sizeof(GenBlock) * blocks.size(),
                           cudaMemcpyHostToDevice, stream));
   for (size_t off = 0; off < blocks.size(); off += 65535) {

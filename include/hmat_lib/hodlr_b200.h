@@ -55,8 +55,10 @@ const char *hodlr_b200_last_error(void);
  *   pool_keep (1): freed tree arenas and small stream-ordered scratch stay
  *       mapped in the device's default memory pool (release threshold
  *       unlimited), scratch of 32 MiB or more in a pool of the library's own
- *       (up to half of the device's memory); set 0 before the library's first
- *       call on a device to leave the default pool alone and keep no scratch
+ *       (up to half of the device's memory); both give back what they hold
+ *       unused when an allocation would fail otherwise; set 0 before the
+ *       library's first call on a device to leave the default pool alone and
+ *       keep no scratch
  *   learned_ranks (0): size each sketch from the rank model (fallback to
  *       adaptive growth per block)
  *   learned_margin (0.1), learned_extra (40), learned_eta (1.0): one-shot width
@@ -160,6 +162,8 @@ int hodlr_b200_tree_to_host(hodlr_b200_tree t, struct TreeHODLR *hodlr, int *ier
 /* Device handle of a host tree (uploading it if needed); release with
  * hodlr_b200_tree_free. */
 hodlr_b200_tree hodlr_b200_tree_from_host(const struct TreeHODLR *hodlr, int *ierr);
+/* arena_bytes: what leaves and factors take; the allocation behind them is up
+ * to an eighth larger from 32 MiB on, where the memory allows it. */
 int hodlr_b200_tree_info(hodlr_b200_tree t, int *height, int *n, int *max_rank,
                          long long *storage_doubles, long long *arena_bytes);
 /* Ranks in block order b = 2 * (2^d - 1 + j) + (c - 1); returns the count. */
