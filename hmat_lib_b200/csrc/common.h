@@ -83,6 +83,25 @@ void device_alloc(T **p, size_t bytes) {
   *p = static_cast<T *>(device_alloc(bytes));
 }
 
+// Lets a kernel take more than 48 KB of dynamic shared memory.  The attribute
+// belongs to the current device, so it is set once on each; any thread may call.
+class SmemOptIn {
+ public:
+  template <class Kernel>
+  void operator()(Kernel kernel, size_t bytes) {
+    int dev = 0;
+    HB_CUDA(cudaGetDevice(&dev));
+    const uint64_t bit = dev < 64 ? uint64_t(1) << dev : 0;
+    if (done_.load(std::memory_order_acquire) & bit) return;
+    HB_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void *>(kernel),
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    done_.fetch_or(bit, std::memory_order_release);
+  }
+
+ private:
+  std::atomic<uint64_t> done_{0};
+};
+
 // Waits for all work on `device` if `in_flight` is set, and clears it: the first
 // step of every destructor whose memory queued work may still use.  cudaFree of
 // cudaMalloc memory waits for the device by itself; of stream-ordered memory it

@@ -794,13 +794,9 @@ template <int BM, int BN, int WM, int WN>
 void launch_gemm(const GemmPlan &plan, const GemmBases &bases, cudaStream_t stream) {
   const int engine = gemm_f64_engine();
   if (engine == 1) {
-    static bool configured = false;
+    static SmemOptIn opt_in;
     const size_t smem = MmaSmem<BM, BN, 16>::bytes;
-    if (!configured) {
-      HB_CUDA(cudaFuncSetAttribute(gemm_f64_mma_kernel<BM, BN, WM, WN, 16>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      configured = true;
-    }
+    opt_in(gemm_f64_mma_kernel<BM, BN, WM, WN, 16>, smem);
     gemm_f64_mma_kernel<BM, BN, WM, WN, 16><<<plan.ntiles, kThreads, smem, stream>>>(
         plan.segs, plan.probs, plan.tiles, bases);
     HB_LAUNCHED();
@@ -808,40 +804,27 @@ void launch_gemm(const GemmPlan &plan, const GemmBases &bases, cudaStream_t stre
   }
   if constexpr (BM <= 2 * kWsLoaders && BN <= 2 * kWsLoaders) {   // a chunk per loader and line
     if (engine == 2 && !plan.generated) {
-      static bool configured = false;
-      if (!configured) {
-        HB_CUDA(cudaFuncSetAttribute(gemm_f64_ws_kernel<BM, BN, WM, WN, 32>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)MmaSmem<BM, BN, 32>::bytes));
-        configured = true;
-      }
-      gemm_f64_ws_kernel<BM, BN, WM, WN, 32>
-          <<<plan.ntiles, kWsThreads, MmaSmem<BM, BN, 32>::bytes, stream>>>(plan.segs, plan.probs,
-                                                                          plan.tiles, bases);
+      static SmemOptIn opt_in;
+      const size_t smem = MmaSmem<BM, BN, 32>::bytes;
+      opt_in(gemm_f64_ws_kernel<BM, BN, WM, WN, 32>, smem);
+      gemm_f64_ws_kernel<BM, BN, WM, WN, 32><<<plan.ntiles, kWsThreads, smem, stream>>>(
+          plan.segs, plan.probs, plan.tiles, bases);
       HB_LAUNCHED();
       return;
     }
   }
   if (engine == 2) {
-    static bool configured = false;
+    static SmemOptIn opt_in;
     const size_t smem = MmaSmem<BM, BN, 32>::bytes;
-    if (!configured) {
-      HB_CUDA(cudaFuncSetAttribute(gemm_f64_mma_kernel<BM, BN, WM, WN, 32>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      configured = true;
-    }
+    opt_in(gemm_f64_mma_kernel<BM, BN, WM, WN, 32>, smem);
     gemm_f64_mma_kernel<BM, BN, WM, WN, 32><<<plan.ntiles, kThreads, smem, stream>>>(
         plan.segs, plan.probs, plan.tiles, bases);
     HB_LAUNCHED();
     return;
   }
-  static bool configured = false;
+  static SmemOptIn opt_in;
   const size_t smem = Smem<BM, BN>::bytes;
-  if (!configured) {
-    HB_CUDA(cudaFuncSetAttribute(gemm_f64_kernel<BM, BN>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = true;
-  }
+  opt_in(gemm_f64_kernel<BM, BN>, smem);
   gemm_f64_kernel<BM, BN><<<plan.ntiles, kThreads, smem, stream>>>(plan.segs, plan.probs,
                                                                    plan.tiles, bases);
   HB_LAUNCHED();

@@ -670,12 +670,8 @@ std::vector<int> ozaki_schedule(std::vector<OzTile> &tiles, const std::vector<Oz
 void ozaki_gemm(const OzSeg *d_segs, const OzTile *d_tiles, const int *d_starts, int grid,
                 double *cbase, int *d_status, cudaStream_t stream) {
   if (grid <= 0) return;
-  static bool configured = false;
-  if (!configured) {
-    HB_CUDA(cudaFuncSetAttribute(ozaki_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kSmem));
-    configured = true;
-  }
+  static SmemOptIn opt_in;
+  opt_in(ozaki_gemm_kernel, kSmem);
   // bulk copies per operand block (1, 2, 4 or 8 lanes; every chunk stays a
   // multiple of 16 bytes since B blocks are multiples of 384 bytes)
   int split = (int)option("ozaki_copy_split", 1.0);

@@ -245,12 +245,8 @@ void rank_mlp_gradient(const float *d_params, const float *d_x, const float *d_t
   const int nblocks = (n + kSamplesPerBlock - 1) / kSamplesPerBlock;
   const size_t smem = sizeof(float) * (kRankParams + kGradWarps * (kRankParams + 1) +
                                       kGradWarps * 32 * (kRankIn + 4 * kRankH + 2));
-  static bool configured = false;
-  if (!configured) {
-    HB_CUDA(cudaFuncSetAttribute(gradient_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
-    configured = true;
-  }
+  static SmemOptIn opt_in;
+  opt_in(gradient_kernel, smem);
   float *partial = nullptr;
   pool_alloc(&partial, sizeof(float) * nblocks * (kRankParams + 1), stream);
   gradient_kernel<<<nblocks, kGradThreads, smem, stream>>>(d_params, d_x, d_t, n, partial);
