@@ -220,21 +220,24 @@ __device__ __forceinline__ int plane_offset(int k, int sk, int m, int sm) {
 // when it must be rotated.  Columns at or below theta are neither rotated nor
 // tested (all of them together hold at most sqrt(L) theta = 1e-3 tol ||A||_F
 // / sqrt(L) of the matrix: no kept singular value moves by more than 0.1% of
-// the truncation threshold).  A coupling at rounding level of the problem's
-// own scale counts as converged: a column recomputed from others carries an
-// error of about eps ||A|| times its weight, which no rotation removes.
-// All squared: no square root on the eigensolver's critical path (entries are
-// of order one, so the squares of columns above theta do not vanish).
+// the truncation threshold).  The cosine is taken against ||A||_F in place of
+// the smaller column: a coupling at rounding level of the problem's own scale
+// counts as converged, because a column recomputed from others carries an error
+// of about eps ||A|| times its weight, which no rotation removes.  Against the
+// smaller column itself, sweeps at a tolerance of zero chase that error and never
+// end.  All squared: no square root on the eigensolver's critical path (entries
+// are of order one, so the squares of columns above theta do not vanish).
 __device__ __forceinline__ bool needs_rotation(double al, double be, double ga, double theta2,
                                                double fro2, double conv2) {
-  return al > theta2 && be > theta2 && ga * ga > conv2 * fmin(al * be, fro2 * fmax(al, be));
+  return al > theta2 && be > theta2 && ga * ga > conv2 * (fro2 * fmax(al, be));
 }
 
 // tan, cos of the rotation that zeroes the product g of two columns whose
 // squared norms differ by d = |x_b|^2 - |x_a|^2.  Any angle keeps W orthogonal
 // as long as c^2 (1 + t^2) = 1; the angle itself only has to make the product
 // small, so t comes from single precision (the product left is about 1e-7 of
-// g) and c is then corrected to double precision for that t: with y close to
+// g; needs_rotation() passes only 2 |g| > 1e-13 max(|x_a|^2, |x_b|^2), far inside
+// a float's range, so a pair that must turn does) and c is then corrected to double precision for that t: with y close to
 // (1 + t^2)^-1/2 and r = 1 - (1 + t^2) y^2, c = y (1 - r)^-1/2, whose binomial
 // series to second order is exact beyond 1e-18 at r = 1e-6.  A double-precision
 // square root, division and reciprocal square root in a row were about half

@@ -58,6 +58,28 @@ def test_block_solver_matches_scalar_solver(n, h, kind, length):
     t_blk.free()
 
 
+@pytest.mark.parametrize("n,dim,h,kind,length", [(1024, 1, 2, "gaussian", 0.3),
+                                                 (2049, 3, 2, "exponential", 0.2),
+                                                 (3001, 3, 2, "matern32", 0.1)])
+def test_threshold_zero_converges(n, dim, h, kind, length):
+    """With svd_threshold = 0 every column is tested, down to rounding level:
+    the sweeps end all the same, and the tree is exact up to the sketch's own
+    stop (1e-14 of the block's norm per column: sqrt(n) 1e-14 in all, doubled
+    over the levels)."""
+    import torch
+    pts = W.points_1d_sorted(n, 3) if dim == 1 else W.points_morton(n, dim, 3)
+    a = torch.from_numpy(np.ascontiguousarray(W.kernel_matrix(pts, kind, length, 1e-2))).cuda()
+    torch.cuda.synchronize()
+    t = DeviceTree.build(a.data_ptr(), n, n, h, 0.0)
+    e = torch.eye(n, dtype=torch.float64, device="cuda")
+    y = torch.zeros_like(e)
+    torch.cuda.synchronize()
+    t.matmat(e.data_ptr(), n, n, y.data_ptr(), n)
+    torch.cuda.synchronize()
+    assert float((y - a).norm() / a.norm()) <= 2.0 * np.sqrt(n) * 1e-14
+    t.free()
+
+
 def test_block_solver_against_reference_ranks():
     """The n = 8192 3D exponential workload (hmat_lib's ranks in
     tests/golden/ref_exp3d_n8192.npz), matrix-free, every sketched core on
