@@ -729,7 +729,8 @@ std::vector<std::shared_ptr<DeviceTree>> build_attempt(
           for (size_t a = 0; a < pa.size(); ++a) {
             const SketchBlock &S = sk[pa[a]];
             cd.push_back(CleanDesc{tp[a].Y, tp[a].ldy, tp[a].m, tp[a].w, tp[a].R, tp[a].ldr,
-                                   work + S.rn + kPanel * kPanel + kPanel + q * kPanel});
+                                   work + S.rn + kPanel * kPanel + kPanel + q * kPanel,
+                                   S.ell + q * kPanel > 0});
           }
           panel_clean(cd, option("sketch_clean_rel", 1e-13), stream);
         }

@@ -301,13 +301,31 @@ T *upload(const std::vector<T> &v, cudaStream_t s) {
   return d;
 }
 
+constexpr double kCleanOrth = 1e-5;   // see panel_clean()
+
 __global__ void panel_clean_kernel(const CleanDesc *__restrict__ descs, double rel) {
   const CleanDesc D = descs[blockIdx.y];
-  double scale2 = 0.0;
-  for (int c = 0; c < D.w; ++c) scale2 = fmax(scale2, D.prenorm2[c]);
-  const double thr = rel * sqrt(scale2);
-  for (int c = 0; c < D.w; ++c) {
-    if (fabs(D.R[c + (long long)c * D.ldr]) > thr) continue;
+  static_assert(kPanel == 32, "a lane per column");
+  __shared__ unsigned drop;
+  if (threadIdx.x < 32) {
+    const int c = threadIdx.x;
+    const double *R = D.R + (long long)c * D.ldr;
+    double scale2 = c < D.w ? D.prenorm2[c] : 0.0, top = 0.0, diag = 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      scale2 = fmax(scale2, __shfl_xor_sync(0xffffffffu, scale2, o));
+    if (c < D.w) {
+      for (int i = 0; i < c; ++i) top = fmax(top, fabs(R[i]));
+      diag = fabs(R[c]);
+    }
+    const bool zero = c < D.w && (!(diag > rel * sqrt(scale2)) ||
+                                  (D.later && diag <= kCleanOrth * top));
+    const unsigned mask = __ballot_sync(0xffffffffu, zero);
+    if (c == 0) drop = mask;
+  }
+  __syncthreads();
+  for (unsigned m = drop; m; m &= m - 1) {
+    const int c = __ffs(m) - 1;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < D.rows; i += gridDim.x * blockDim.x)
       D.Q[i + (long long)c * D.ldq] = 0.0;
   }

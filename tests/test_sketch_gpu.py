@@ -81,3 +81,26 @@ def test_full_rank_blocks(n):
     ranks, got = _build(a, n, 0, 1e-9)
     assert list(ranks) == [n // 2, n // 2]
     assert np.linalg.norm(got - a) <= 1e-11 * np.linalg.norm(a)
+
+
+@pytest.mark.parametrize("n,h,band", [(1024, 1, 64), (1024, 1, 129), (4096, 2, 64), (4096, 2, 129)])
+def test_steep_end_of_the_singular_values(n, h, band):
+    """Random banded matrices: a block is a triangular corner, whose singular
+    values fall off a cliff inside a panel (to 1e-12 and below within a few
+    columns).  Columns of the basis at that level are not orthogonal to the
+    rest and must not stay in it.  What the truncation drops is at most
+    sqrt(band) 1e-8 of a block's norm, far less of the matrix's."""
+    import torch
+    r = np.random.default_rng(band)
+    i = np.arange(n)
+    a = np.where(np.abs(i[:, None] - i[None, :]) <= band, r.standard_normal((n, n)), 0.0)
+    d = torch.from_numpy(np.ascontiguousarray(a.T)).cuda()      # column-major
+    torch.cuda.synchronize()
+    t = DeviceTree.build(d.data_ptr(), n, n, h, 1e-8)
+    e = torch.eye(n, dtype=torch.float64, device="cuda")
+    y = torch.zeros_like(e)
+    torch.cuda.synchronize()
+    t.matmat(e.data_ptr(), n, n, y.data_ptr(), n)
+    torch.cuda.synchronize()
+    assert float((y - d).norm() / d.norm()) <= 1e-8
+    t.free()
