@@ -67,19 +67,21 @@ struct SketchBlock {
   int mix = -1;          // index in the int8 sketch products (-1: FP64 GEMMs)
 };
 
-// What large scratch can still get (bytes): device memory that is free or held
-// unused by the scratch pool.  What the default pool holds unused (arenas of
-// freed trees) is out of that pool's reach until it is given back to the device,
-// which fits() does where it decides.  Asked once and then kept up by take().
+// The device memory that is left for large scratch (bytes): free, held unused by
+// the scratch pool, or held unused by the default pool (arenas of freed trees),
+// which the scratch pool can get only once it is given back to the device.
+// Asked once and then kept up by take().
 class ScratchBudget {
  public:
-  bool fits(double need) {
+  // Whether `bytes` are at most `share` of what is left and can be had: what the
+  // default pool keeps is given back only if they do not fit without it.
+  bool fits(double bytes, double share) {
     if (avail_ < 0.0) ask();
-    if (need > avail_ && need <= avail_ + kept_) {
+    if (bytes > avail_ && bytes <= share * total()) {
       HB_CUDA(cudaMemPoolTrimTo(default_pool_, 0));
       ask();
     }
-    return need <= avail_;
+    return bytes <= avail_ && bytes <= share * total();
   }
   void take(double bytes) { avail_ = std::max(0.0, avail_ - bytes); }
   void forget() { avail_ = -1.0; }
@@ -486,7 +488,7 @@ std::vector<std::shared_ptr<DeviceTree>> build_attempt(
       const int c = std::min(limit, std::max(cand, S.cap + kPanel) / kPanel * kPanel);
       if (c <= S.cap) continue;
       const double need = 8.0 * ((double)layout(c, parts) + 5.0 * (double)c * c);
-      if (cap_opt > 0 || (mem_frac > 0.0 && budget.fits(need / mem_frac))) {
+      if (cap_opt > 0 || budget.fits(need, mem_frac)) {
         c2 = c;
         break;
       }
@@ -1067,8 +1069,7 @@ std::vector<std::shared_ptr<DeviceTree>> build_batch(const std::vector<BuildInpu
   // matrix (66 now).
   if (gen && !in[0].g.blocks.empty()) {
     const int n = in[0].g.n;
-    const double bytes = 8.0 * (double)n * n, frac = option("kernel_form_frac", 0.0625);
-    if (frac > 0.0 && ScratchBudget().fits(bytes / frac)) {
+    if (ScratchBudget().fits(8.0 * (double)n * n, option("kernel_form_frac", 0.0625))) {
       struct Matrix {
         double *p;
         cudaStream_t s;

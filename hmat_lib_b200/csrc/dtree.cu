@@ -118,14 +118,12 @@ size_t large_size(size_t bytes) {
   while (step * 16 <= bytes) step *= 2;
   return (bytes + step - 1) / step * step;
 }
-}  // namespace
 
-namespace {
 // Runs `alloc` (false).  When the device is out of memory, waits for its work,
 // so that everything freed is free, gives back what the default and the scratch
 // pool hold unused, and runs alloc(true), the last try, without rounding.
 template <class F>
-void allocate(F alloc) {
+void allocate(size_t bytes, F alloc) {
   cudaError_t e = alloc(false);
   if (e == cudaErrorMemoryAllocation) {
     (void)cudaGetLastError();
@@ -137,7 +135,11 @@ void allocate(F alloc) {
       (void)cudaGetLastError();
     e = alloc(true);
   }
-  HB_CUDA(e);
+  if (e != cudaSuccess) {
+    (void)cudaGetLastError();
+    throw Error{ALLOCATION_FAILURE, "device allocation of " + std::to_string(bytes) +
+                                        " bytes: " + cudaGetErrorString(e)};
+  }
 }
 }  // namespace
 
@@ -152,7 +154,7 @@ double *dev_alloc(size_t elems, cudaStream_t stream) {
   if (bytes < kLarge) return (double *)pool_alloc(bytes, stream);
   void *p = nullptr;
   const cudaMemPool_t pool = scratch_pool();
-  allocate([&](bool exact) {
+  allocate(bytes, [&](bool exact) {
     return cudaMallocFromPoolAsync(&p, exact ? bytes : large_size(bytes), pool, stream);
   });
   return (double *)p;
@@ -160,13 +162,13 @@ double *dev_alloc(size_t elems, cudaStream_t stream) {
 
 void *pool_alloc(size_t bytes, cudaStream_t stream) {
   void *p = nullptr;
-  allocate([&](bool) { return cudaMallocAsync(&p, bytes, stream); });
+  allocate(bytes, [&](bool) { return cudaMallocAsync(&p, bytes, stream); });
   return p;
 }
 
 void *device_alloc(size_t bytes) {
   void *p = nullptr;
-  allocate([&](bool) { return cudaMalloc(&p, bytes); });
+  allocate(bytes, [&](bool) { return cudaMalloc(&p, bytes); });
   return p;
 }
 
@@ -279,10 +281,9 @@ std::unique_ptr<DeviceTree> dtree_create(const Geometry &g_in, cudaStream_t stre
   keep_pool_memory();
   // (large arenas in rounded sizes, so that a tree of nearly the same ranks
   // finds the place of one that was freed, unless only the exact size fits)
-  allocate([&](bool exact) {
-    return cudaMallocAsync((void **)&t->arena,
-                           exact ? std::max<long long>(off, 1) * sizeof(double) : scratch_bytes(off),
-                           stream);
+  const size_t bytes = std::max<long long>(off, 1) * sizeof(double);
+  allocate(bytes, [&](bool exact) {
+    return cudaMallocAsync((void **)&t->arena, exact ? bytes : scratch_bytes(off), stream);
   });
   pool_alloc(&t->d_leaves, std::max<size_t>(t->leaves.size(), 1) * sizeof(LeafDesc), stream);
   pool_alloc(&t->d_blocks, std::max<size_t>(g.blocks.size(), 1) * sizeof(BlockDesc), stream);

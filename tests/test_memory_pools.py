@@ -95,6 +95,30 @@ def test_calls_get_what_scratch_left(fake, call):
         t.free()
 
 
+def _build_points():
+    p = np.zeros(2048)
+    return DeviceTree.build_kernel(p.ctypes.data, 2048, 1, 0, 0.1, 1.0, 4, 1e-8, stream=64)
+
+
+def test_formed_matrix_leaves_the_default_pool_alone_if_it_fits(fake):
+    with F.loaded(*fake) as lib:
+        F.device_tree(1, 2048, 1).free()
+        kept = lib.fake_pool_bytes(0, 1)
+        _build_points().free()                      # 32 MiB of 4 GiB
+        assert lib.fake_pool_bytes(1, 1) >= 32 * MB
+        assert lib.fake_pool_bytes(0, 1) >= kept
+
+
+def test_formed_matrix_gets_what_freed_trees_left(fake):
+    with F.loaded(*fake) as lib:
+        lib.hodlr_b200_set_option(b"kernel_form_frac", 0.6)
+        F.device_tree(1, 3072, 1).free()
+        lib.fake_set_capacity(lib.fake_pool_bytes(0, 1) + 20 * MB)
+        _build_points().free()                      # 32 MiB, 20 of them free
+        assert lib.fake_pool_bytes(1, 1) >= 32 * MB
+        assert lib.fake_pool_bytes(0, 1) < 144 * MB
+
+
 def test_arena_falls_back_to_its_exact_size(fake):
     with F.loaded(*fake) as lib:
         exact = 8 * (2 * 2048 * 2048 + 2 * 2 * 2048)
