@@ -279,15 +279,16 @@ std::vector<double> sketch_mixer(unsigned long long seed) {
 void sketch_multiply(const std::vector<SketchDesc> &descs, const double *M,
                      const KernelSpec *gen, unsigned long long seed, cudaStream_t stream) {
   // A row tile's columns are split so that the launch has about six items for
-  // each of the 296 resident CTAs (a launch of the last rounds has few row
+  // each of the resident CTAs, two an SM (a launch of the last rounds has few row
   // tiles, of wide blocks), but no item has less than 8 column groups: an
   // item's partial sums are 32 KB of atomics against 32 KB of A per group.
-  constexpr int kResident = 2 * 148, kWaves = 6, kMinGroups = 8;
+  constexpr int kWaves = 6, kMinGroups = 8;
+  const long long resident = 2LL * num_sms();
   long long tiles = 0;
   for (const SketchDesc &D : descs)
     tiles += (long long)((D.m + kRows - 1) / kRows) * ((D.n + kGroup - 1) / kGroup) *
              ((D.w + kGroup - 1) / kGroup);
-  const int per = (int)std::max<long long>(kMinGroups, tiles / (kResident * kWaves));
+  const int per = (int)std::max<long long>(kMinGroups, tiles / (resident * kWaves));
   std::vector<Job> jobs;
   long long items = 0;
   auto launch = [&]() {
