@@ -201,7 +201,8 @@ def build_roofline(stats, seconds, storage, peak_tflops, peak_gbs, matrix_free=F
     """Build against both roofs: its algorithmic bytes (the input read once,
     8 n^2, unless matrix-free, plus the factors written once, 8 W) over the
     wall time against the measured HBM bandwidth, and the FP64 GEMM work it
-    issued over the wall time against the FP64 GEMM peak measured in the run."""
+    issued (without the Hadamard sketch products, which are additions) over the
+    wall time against the FP64 GEMM peak measured in the run."""
     nbytes = (0.0 if matrix_free else 8.0 * stats["input_elems"]) + 8.0 * storage
     tflops = stats["gemm_flops"] / seconds / 1e12
     return {"algorithmic_bytes": nbytes, "GB/s": nbytes / seconds / 1e9,
@@ -1033,9 +1034,9 @@ def main():
     dom64 = "phase1" if r64["p1"] >= r64["p2"] else "phase2"
     dom64_ms = r64["p1"] if dom64 == "phase1" else r64["p2"]
     achieved64 = 2.0 * k * el[dom64] / (dom64_ms * 1e-3) / 1e12
-    # DRAM traffic / algorithmic bytes of the FP64 phases, measured by ncu on
-    # the n = 16384 instance of this workload family
-    traffic_ratio64 = {"phase1": 1.24, "phase2": 1.11}
+    # DRAM traffic / algorithmic bytes of the FP64 phases (gemm_f64_ws_kernel),
+    # measured by ncu on the n = 16384 instance of this workload family
+    traffic_ratio64 = {"phase1": 1.21, "phase2": 1.09}
     bytes64 = {"phase1": 8.0 * sn + 8.0 * n * k, "phase2": 8.0 * (leaves_el + sn) + 16.0 * n * k}
     cpu = None
     if world == 1 and not args.no_cpu_baseline:
@@ -1113,8 +1114,8 @@ def main():
                               "achieved": achieved64, "peak": peak64, "unit": "TFLOP/s",
                               "frac": achieved64 / peak64,
                               "traffic": traffic_ratio64[dom64] * bytes64[dom64],
-                              "traffic_source": "ncu DRAM bytes / algorithmic bytes at "
-                                                "n = 16384, times the bytes at this n",
+                              "traffic_source": "ncu DRAM bytes / algorithmic bytes of this "
+                                                "kernel at n = 16384, times the bytes at this n",
                               "algorithmic_bytes": bytes64[dom64],
                               "peak_source": "cuBLAS DGEMM 8192^3 measured in this run",
                               "phase_ms": {"phase1": r64["p1"], "phase2": r64["p2"]}},

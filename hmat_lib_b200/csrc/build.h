@@ -24,7 +24,8 @@ struct BuildStats {
   double ms_finish = 0.0;      // arena, leaf copies, U = Q U_R S, V = P V_R
   int learned_fallbacks = 0;   // one-shot sketches that failed the error check
   double ms_features = 0.0;    // rank-model features and prediction (host clock)
-  double gemm_flops = 0.0;     // FP64 GEMM work of the build (2 M N K summed)
+  double gemm_flops = 0.0;     // FP64 GEMM work of the build (2 M N K summed; without the
+                               //   Hadamard sketch products, half of it before they came)
   double input_elems = 0.0;    // entries of the input matrices (n^2 per tree)
   double ms_host_setup = 0.0;  // host clock from the call to the first stage event
   double ms_host_total = 0.0;  // host clock from the call to the return
@@ -46,9 +47,10 @@ const std::vector<float> &last_build_features();
 // Compresses every off-diagonal block of the n x n matrix d_A (ld lda, device)
 // following the block sizes of `g` (ranks ignored) with hmat_lib's relative
 // truncation rule at `tol`.  `svd_status` receives SUCCESS or SVD_FAILURE.
-// With `gen` set, the matrix is the kernel matrix it defines and is never
-// formed: every entry the build needs is computed where it is used (d_A and
-// lda are then ignored).
+// With `gen` set, the matrix is the kernel matrix it defines (d_A and lda are then
+// ignored): formed in scratch when it is a small share of the device memory at
+// hand (option kernel_form_frac), otherwise every entry the build needs is
+// computed where it is used.
 std::shared_ptr<DeviceTree> build_from_dense(const Geometry &g, const double *d_A, long long lda,
                                              double tol, cudaStream_t stream, int *svd_status,
                                              BuildStats *stats = nullptr,

@@ -82,7 +82,7 @@ void keep_pool_memory() {
 // device.  Trees and plans outlive a call, so in the default pool they land in
 // the holes that a build's gigabytes of scratch leave, and the next build maps
 // fresh memory: cudaMallocAsync calls of 30 to 1000 ms in every third or fourth
-// of a row of n = 32768 builds (170 ms of work each then, 115 now).  Here everything is free
+// of a row of n = 32768 builds (170 ms of work each then, 109 now).  Here everything is free
 // again when a call ends, and sizes are rounded up to an eighth of a power of
 // two, so the next call finds the same blocks.  The pool keeps at most half of
 // the device's memory mapped (nothing with option pool_keep = 0).  What one pool

@@ -1,7 +1,9 @@
 // FP64 variable-batched segmented GEMM for sm_100a.
 //
-// Two kernels (option gemm_f64_engine): the FP64 tensor-core (DMMA) kernel
-// (default, below), and a CUDA-core DFMA kernel: 256 threads, a BM x BN output tile per CTA
+// Three kernels (option gemm_f64_engine): on the FP64 tensor cores (DMMA) one with
+// loader warps beside the MMA warps (default, last below) and one whose warps do
+// both (generated operands, 256-column tiles, 16-deep stages), and a CUDA-core
+// DFMA kernel: 256 threads, a BM x BN output tile per CTA
 // (128 x 64, 64 x 128, 64 x 64, 32 x 128 or 32 x 256), K advanced 16 at a time through a two-stage
 // cp.async pipeline (8-byte copies with zero fill, so any leading dimension
 // and any offset work), 32 accumulators per thread, operands read from shared
@@ -918,8 +920,9 @@ void gemm_plan_build(GemmPlan &plan, const GemmBatch &batch, TileShape shape, KS
   // full one: its tiles are split along K into the number of parts, each at
   // least 256 long, whose waves are shortest together (3% for a part's own
   // start and end).  n = 32768, k = 256: 1024 output tiles of K about 1260,
-  // 3.46 waves, the last 136 in two parts; n = 16384: 512 tiles, 1.73 waves, the
-  // last 216 in four (689 -> 655 us for the whole product).
+  // 3.46 waves, the last 136 in two parts; a tree of n = 16384 whose ranks add to
+  // 1000: 512 tiles, 1.73 waves, the last 216 in four (689 -> 655 us for the whole
+  // product).  From three parts on the order of their sums is open.
   if (ksplit == KSplit::Tail) {
     const long long slots = 2LL * num_sms(), rest = (long long)tiles.size() % slots;
     if (rest > 0) {

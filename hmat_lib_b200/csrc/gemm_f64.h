@@ -124,14 +124,15 @@ void gemm_plan_build(GemmPlan &plan, const GemmBatch &batch, TileShape shape, KS
 void gemm_plan_run(const GemmPlan &plan, const GemmBases &bases, cudaStream_t stream);
 
 // FP64 multiply-add work (2 M N K per problem) of every GEMM plan built on
-// the calling thread since the counter was last reset (build statistics).
+// the calling thread since the counter was last reset (build statistics).  The
+// Hadamard sketch products (sketch.h) are no GEMM and not in it.
 double &gemm_flops_counter();
 // Host milliseconds spent making GEMM and TSQR plans on this thread (reset by
 // the caller).
 double &plan_host_ms();
 
-// Which kernel runs the FP64 products (option gemm_f64_engine): 1 the FP64
-// tensor-core (DMMA) kernel, 0 the DFMA kernel.
+// Which kernels run the FP64 products (option gemm_f64_engine): 2 (default) and 1
+// the FP64 tensor-core (DMMA) ones with K stages of 32 and 16, 0 the DFMA kernel.
 int gemm_f64_engine();
 
 // One-shot convenience: plan, run, release (stream-ordered).  A batch of at most

@@ -104,7 +104,10 @@ long long product_w_layout(const DeviceTree &t, int k, std::vector<long long> &w
 // (0-4: 128x64, 64x128, 32x128, 32x256, 64x64), else by op and k: up to 64
 // right-hand sides take 64 x 64 tiles (more of them, three stages deep, and no
 // idle half; H^T X and X H at n = 10007, k = 33: 349 -> 265 us;
-// 207 with the GEMM's loader warps).
+// 204 with the GEMM's loader warps).  Against the wider shapes over eight trees
+// (n = 700 to 32768, 1D to 3D), k = 2 to 64 and every op: 0.58 to 0.98 of their
+// time, 0.76 in the median, but for X H at 16 to 48 columns of the trees of the
+// largest ranks (1.00 to 1.03).
 TileShape default_shape(ProdOp op, int k, int phase) {
   const int forced =
       (int)(phase == 1 ? option("product_shape1", -1.0) : option("product_shape2", -1.0));

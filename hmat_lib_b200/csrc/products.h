@@ -14,14 +14,17 @@ enum class ProdOp : int {
 };
 
 enum class Precision : int {
-  FP64 = 0,     // DFMA throughout
+  FP64 = 0,     // on the FP64 tensor cores
   MIXED = 1,    // split-precision tensor-core products (products_mixed.cu)
 };
 
 // Two launches per product: phase 1 projects the input onto every block's
 // factor (W_b = V_b^T X_b, split along the long dimension with atomics);
-// phase 2 writes each output row band once, accumulating the leaf product and
-// one U_b W_b term per level in registers.
+// phase 2 accumulates the leaf product and one U_b W_b term per level of an
+// output tile in registers and writes it once, but for the tiles of a last,
+// partly filled wave, whose K range is split among several tiles that add to
+// zeroed output (two more launches zero what atomics add to).  Sums of three or
+// more parts may differ in their last bits from run to run.
 struct ProductPlan {
   ProdOp op = ProdOp::N;
   int k = 0;

@@ -37,7 +37,11 @@ enum { HODLR_B200_CUDA_ERROR = 100 };
 
 enum HodlrB200Precision {
   HODLR_B200_FP64 = 0,   /* FP64 products (FP64 tensor cores) */
-  HODLR_B200_MIXED = 1   /* split-precision tensor-core products with FP64 result */
+  HODLR_B200_MIXED = 1   /* split-precision tensor-core products with FP64 result:
+                          * less exact (about 42 bits) and faster where a product is
+                          * bound by FP64 arithmetic (128 columns or more, ranks in
+                          * the tens and hundreds); slower on small products and on
+                          * low-rank 1D trees, batches of them included */
 };
 
 const char *hodlr_b200_version(void);
@@ -80,7 +84,8 @@ const char *hodlr_b200_last_error(void);
  *       each growth of its scratch (plus its core SVD) fits this share of the
  *       device memory free or held unused by the stream-ordered pool
  *   sketch_seed (20240607): seed of the random test matrices
- *   sketch_clean_rel (1e-13): rounding level below which a new panel is zeroed
+ *   sketch_clean_rel (1e-13): rounding level below which a column of a new
+ *       panel is zeroed
  *   exact_max (128): blocks with min(m, n) up to this are compressed by an
  *       exact Jacobi SVD
  *   jacobi_max_sweeps (60): Jacobi sweep bound (SVD_FAILURE past it)
