@@ -9,6 +9,7 @@ import glob
 import os
 import shutil
 import subprocess
+from concurrent.futures import ThreadPoolExecutor
 
 import numpy as np
 
@@ -20,10 +21,16 @@ CUDA = os.path.dirname(os.path.dirname(build.NVCC))
 
 
 def link(directory) -> str:
-    """Builds the library against the stand-in runtime; its path."""
-    build.build()
-    objects = [os.path.join(build.BUILD, os.path.basename(s) + ".o") for s in build._sources()]
-    objects.append(os.path.join(build.BUILD, "source_hash.cpp.o"))
+    """Builds the library against the stand-in runtime; its path.  Objects that
+    are missing or old are compiled, but the library itself, which this process
+    may have loaded, is left alone."""
+    os.makedirs(build.BUILD, exist_ok=True)
+    header = build._newest_header()
+    with ThreadPoolExecutor(max_workers=8) as ex:
+        made = list(ex.map(lambda s: build._compile(s, False, header), build._sources()))
+    made.append(build._hash_object(False))
+    assert not [e for _, e in made if e], made
+    objects = [o for o, _ in made]
     out = os.path.join(str(directory), "libhodlr_fake.so")
     cmd = ["g++", "-shared", "-fPIC", "-O1", "-std=c++17", "-I", os.path.join(CUDA, "include"),
            os.path.join(HERE, "fake_cudart.cpp"), *objects, "-Wl,-Bsymbolic", "-lpthread", "-o", out]
