@@ -126,6 +126,7 @@ struct Events {
 void host_product(DeviceTree &t, ProdOp op, const double *X, long long xr, long long xc,
                   long long ldx, double *Y, long long ldy) {
   cudaStream_t s = lib_stream();
+  InFlight use{t.last_use};
   DevBuf dx(xr * xc, s), dy(xr * xc, s);
   // option "matmat_precision" = 1 routes H X, H^T X and X H through the int8
   // tensor-core path (about 42 bits); the default keeps FP64 throughout
@@ -146,6 +147,7 @@ void host_product(DeviceTree &t, ProdOp op, const double *X, long long xr, long 
     product(dx.p, dy.p, (int)(op == ProdOp::L ? xr : xc));
     d2h(Y, ldy, dy.p, xr, xc, s);
     HB_CUDA(cudaStreamSynchronize(s));
+    use.done = true;
     return;
   }
   cudaStream_t si = copy_stream(0), so = copy_stream(1);
@@ -179,6 +181,7 @@ void host_product(DeviceTree &t, ProdOp op, const double *X, long long xr, long 
   HB_CUDA(cudaEventRecord(copied_out, so));
   HB_CUDA(cudaStreamWaitEvent(s, copied_out, 0));
   HB_CUDA(cudaStreamSynchronize(s));
+  use.done = true;
 }
 
 std::shared_ptr<DeviceTree> subtree_device(const HODLRInternalNode *internal, int height,
@@ -612,6 +615,7 @@ int hodlr_b200_matmat_dev(hodlr_b200_tree t, int op, int precision, const double
     const long long rows = (op == HODLR_B200_OP_L) ? k : t->p->g.n;
     HB_REQUIRE(k >= 0 && ldx >= std::max(1LL, rows) && ldy >= std::max(1LL, rows), INPUT_ERROR,
                "leading dimension below the number of rows");
+    const InFlight use{t->p->last_use};
     if (precision == HODLR_B200_MIXED) {
       product_mixed_op(*t->p, (ProdOp)op, d_x, k, ldx, d_y, ldy, as_stream(stream));
       return SUCCESS;

@@ -49,11 +49,10 @@ struct BatchPlan {
   cudaGraphExec_t exec = nullptr;
   long long graph_launches = 0;
   std::string tuned;
-  // a plan runs as soon as it is made, and on any stream after that
-  std::atomic<bool> in_flight{true};
+  LastUse last_use;
 
   ~BatchPlan() {
-    wait_in_flight(in_flight, device);
+    last_use.wait(device);
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
     ph1.reset();
@@ -230,7 +229,12 @@ void batched_product(const std::vector<std::shared_ptr<DeviceTree>> &trees, Prod
   if (prec == Precision::MIXED)
     HB_REQUIRE(op == ProdOp::N, INPUT_ERROR, "mixed precision is available for Y = H X (op N)");
 
-  for (const auto &t : trees) t->in_flight = true;
+  struct Uses {
+    const std::vector<std::shared_ptr<DeviceTree>> &trees;
+    ~Uses() {
+      for (const auto &t : trees) t->last_use.touch();
+    }
+  } uses{trees};
   std::lock_guard<std::mutex> lk(g_batch_mutex);
   BatchPlan *P = nullptr;
   for (auto it = g_batch_cache.begin(); it != g_batch_cache.end(); ++it)
@@ -281,6 +285,7 @@ void batched_product(const std::vector<std::shared_ptr<DeviceTree>> &trees, Prod
     while (g_batch_cache.size() > kBatchCacheSize) g_batch_cache.pop_back();
     P = g_batch_cache.front().get();
   }
+  const InFlight use{P->last_use};   // ends before the lock: the plan may be evicted then
   PhaseTimer timer(stream);
   if (P->exec && !timing) {
     HB_CUDA(cudaGraphLaunch(P->exec, stream));

@@ -990,7 +990,7 @@ std::vector<std::shared_ptr<DeviceTree>> build_attempt(
   dev_free(work, stream);
   for (double *g : grown) dev_free(g, stream);
   HB_CUDA(cudaStreamSynchronize(stream));
-  for (auto &dt : dts) dt->in_flight = false;
+  for (auto &dt : dts) dt->last_use.settled();
   if (smix && smix->status(stream) != SUCCESS) {
     *svd_status = SVD_FAILURE;
     set_last_error("an int8 sketch product gave up waiting on a barrier");

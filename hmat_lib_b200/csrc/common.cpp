@@ -41,11 +41,28 @@ int num_sms() {
   return cached;
 }
 
-void wait_in_flight(std::atomic<bool> &in_flight, int device) {
-  if (!in_flight.exchange(false)) return;
+namespace {
+std::atomic<uint64_t> g_uses{0};
+constexpr int kWaitDevices = 64;
+std::atomic<uint64_t> g_waited[kWaitDevices];   // every use up to this one is done
+}  // namespace
+
+void LastUse::touch() { at_ = g_uses.fetch_add(1) + 1; }
+
+void LastUse::wait(int device) {
+  const uint64_t at = at_.exchange(0);
+  const bool known = device >= 0 && device < kWaitDevices;
+  if (at == 0 || (known && at <= g_waited[device].load())) return;
   int current = device;
   if (cudaGetDevice(&current) == cudaSuccess && current != device) cudaSetDevice(device);
-  if (cudaDeviceSynchronize() != cudaSuccess) (void)cudaGetLastError();
+  const uint64_t now = g_uses.load();
+  if (cudaDeviceSynchronize() != cudaSuccess) {
+    (void)cudaGetLastError();
+  } else if (known) {
+    uint64_t old = g_waited[device].load();
+    while (old < now && !g_waited[device].compare_exchange_weak(old, now)) {
+    }
+  }
   if (current != device) cudaSetDevice(current);
 }
 

@@ -102,11 +102,31 @@ class SmemOptIn {
   std::atomic<uint64_t> done_{0};
 };
 
-// Waits for all work on `device` if `in_flight` is set, and clears it: the first
-// step of every destructor whose memory queued work may still use.  cudaFree of
-// cudaMalloc memory waits for the device by itself; of stream-ordered memory it
-// hands the bytes to the next allocation at once.
-void wait_in_flight(std::atomic<bool> &in_flight, int device);
+// When the owner of device memory was last used by work that may still be queued
+// or running.  cudaFree of cudaMalloc memory waits for the device by itself; of
+// stream-ordered memory it hands the bytes to the next allocation at once, so a
+// destructor calls wait() before its first release.  Uses are numbered in the
+// order in which their calls return, and each wait for a device covers every
+// earlier one: of many owners freed in a row, the first one waits.
+class LastUse {
+ public:
+  void settled() { at_ = 0; }        // no work uses the owner
+  void touch();                      // everything that does has been queued
+  void wait(int device);
+
+ private:
+  static constexpr uint64_t kMaking = ~uint64_t(0);
+  std::atomic<uint64_t> at_{kMaking};   // until settled() or touch()
+};
+// Held by a call that queues work on the owner's memory.  One that waits for its
+// work sets `done` then, so that only a failure half way counts as a use.
+struct InFlight {
+  LastUse &use;
+  bool done = false;
+  ~InFlight() {
+    if (!done) use.touch();
+  }
+};
 
 // Runtime knobs (hodlr_b200_set_option).
 double option(const char *name, double dflt);

@@ -16,7 +16,7 @@ std::unordered_map<const TreeHODLR *, std::shared_ptr<DeviceTree>> g_registry;
 }  // namespace
 
 DeviceTree::~DeviceTree() {
-  wait_in_flight(in_flight, device);
+  last_use.wait(device);
   graphs.clear();
   plans.clear();
   mixed.reset();
@@ -326,7 +326,7 @@ void dtree_upload(DeviceTree &t, HODLRInternalNode *root, cudaStream_t stream) {
     HB_CUDA(cudaMemcpyAsync(t.arena, img.data(), t.arena_elems * sizeof(double),
                             cudaMemcpyHostToDevice, stream));
   HB_CUDA(cudaStreamSynchronize(stream));
-  t.in_flight = false;
+  t.last_use.settled();
 }
 
 void dtree_download(const DeviceTree &t, TreeHODLR *host, cudaStream_t stream) {

@@ -3,7 +3,6 @@
 // TreeHODLR with its device copy.
 #pragma once
 
-#include <atomic>
 #include <cstdint>
 #include <map>
 #include <memory>
@@ -53,10 +52,7 @@ struct DeviceTree {
   MvItem *mv_items = nullptr;          // inside mv_woff's allocation
   int mv_nwide = 0, mv_nitems = 0;
   double *mv_w = nullptr;
-  // Work that uses the tree may be queued or running: set while the tree is being
-  // made and by every call that returns before its work has run; the destructor
-  // waits for the device then.
-  std::atomic<bool> in_flight{true};
+  LastUse last_use;
 
   DeviceTree() = default;
   DeviceTree(const DeviceTree &) = delete;

@@ -252,6 +252,7 @@ std::shared_ptr<DeviceTree> hxh_multiply(DeviceTree &A, DeviceTree &B, double to
   const Geometry &ga = A.g, &gbg = B.g;
   HB_REQUIRE(ga.h == gbg.h && ga.leaf_m == gbg.leaf_m, INPUT_ERROR,
              "multiply_hodlr_hodlr: trees of different heights or block sizes");
+  InFlight use_a{A.last_use}, use_b{B.last_use};
   const int h = ga.h, nb = ga.nblock(), nleaf = ga.nleaf(), n = ga.n;
   const int dense_max = (int)option("hxh_dense_max", 256);
   // option hxh_precision = 1: the subtree products (the bulk of the product's
@@ -482,7 +483,8 @@ std::shared_ptr<DeviceTree> hxh_multiply(DeviceTree &A, DeviceTree &B, double to
   HB_CUDA(cudaStreamSynchronize(s));
   dev_free(work, s);
   HB_CUDA(cudaStreamSynchronize(s));
-  out->in_flight = false;
+  out->last_use.settled();
+  use_a.done = use_b.done = true;
   return out;
 }
 

@@ -158,7 +158,7 @@ extern "C" int hodlr_b200_matvec_noalloc_dev(hodlr_b200_tree t, const double *d_
                                              void *stream) {
   using namespace hb;
   if (!t || !t->p || !d_x || !d_y) return INPUT_ERROR;
-  t->p->in_flight = true;
+  const InFlight use{t->p->last_use};
   // A CUDA error left behind by earlier asynchronous work (cudaGetLastError
   // also clears it) is reported as such rather than as a failure of this call.
   if (cudaGetLastError() != cudaSuccess) {

@@ -294,7 +294,6 @@ void run_graphed(DeviceTree &t, ProdOp op, int k, long long ldx, long long ldy, 
 void product_f64(DeviceTree &t, ProdOp op, const double *X, int k, long long ldx, double *Y,
                  long long ldy, cudaStream_t stream, int min_depth) {
   if (k <= 0 || t.g.n == 0) return;
-  t.in_flight = true;
   run_graphed(t, op, k, ldx, ldy, min_depth, X, Y, stream,
               [&] { product_f64_direct(t, op, X, k, ldx, Y, ldy, stream, min_depth); });
 }
@@ -302,7 +301,6 @@ void product_f64(DeviceTree &t, ProdOp op, const double *X, int k, long long ldx
 void product_f64_direct(DeviceTree &t, ProdOp op, const double *X, int k, long long ldx, double *Y,
                         long long ldy, cudaStream_t stream, int min_depth) {
   if (k <= 0 || t.g.n == 0) return;
-  t.in_flight = true;
   // one vector: the HBM-bound matvec kernels (option matvec_kernels = 0 keeps
   // the GEMM engine)
   if (k == 1 && op == ProdOp::N && min_depth == 0 && option("matvec_kernels", 1.0) != 0.0) {

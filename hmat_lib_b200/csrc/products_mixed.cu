@@ -580,6 +580,7 @@ DeviceTree &transposed_tree(DeviceTree &t, cudaStream_t s) {
     cudaFree(dbd);
     cudaFree(norms);
   }
+  tt->last_use.settled();   // the tree it belongs to waits for its uses
   t.transposed = tt;
   return *tt;
 }
@@ -588,7 +589,6 @@ DeviceTree &transposed_tree(DeviceTree &t, cudaStream_t s) {
 
 void product_mixed_op(DeviceTree &t, ProdOp op, const double *X, int k, long long ldx, double *Y,
                       long long ldy, cudaStream_t s, int min_depth) {
-  t.in_flight = true;
   if (op == ProdOp::N) {
     product_mixed(t, X, k, ldx, Y, ldy, s, min_depth);
     return;

@@ -537,7 +537,7 @@ struct SolvePlan {
 HodlrFactor::HodlrFactor() = default;
 
 HodlrFactor::~HodlrFactor() {
-  wait_in_flight(in_flight, tree ? tree->device : 0);
+  last_use.wait(tree ? tree->device : 0);
   plans.clear();
   if (buf) cudaFree(buf);
 }
@@ -710,7 +710,7 @@ std::unique_ptr<HodlrFactor> hodlr_factorize(std::shared_ptr<DeviceTree> tp, cud
   HB_CUDA(cudaMemcpyAsync(&st, d_status, sizeof(int), cudaMemcpyDeviceToHost, s));
   HB_CUDA(cudaStreamSynchronize(s));
   cudaFreeAsync(d_status, s);
-  f->in_flight = false;
+  f->last_use.settled();
   if (st) *status = INPUT_ERROR;
   return f;
 }
@@ -718,7 +718,7 @@ std::unique_ptr<HodlrFactor> hodlr_factorize(std::shared_ptr<DeviceTree> tp, cud
 void hodlr_solve(HodlrFactor &f, const double *B, int k, long long ldb, double *X,
                  long long ldx, cudaStream_t s) {
   if (k <= 0 || f.tree->g.n == 0) return;
-  f.in_flight = true;
+  const InFlight use{f.last_use};
   SolvePlan &P = solve_plan(f, k, ldb, ldx, s);
   const GemmBases b = solver_bases(f, X, B, P.T, P.Z);
   gemm_plan_run(P.leaves, b, s);

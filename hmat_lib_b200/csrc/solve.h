@@ -43,7 +43,7 @@ struct HodlrFactor {
   // Launch plans and scratch of hodlr_solve, per (k, ldb, ldx, stream).
   std::map<std::tuple<int, long long, long long, cudaStream_t>, std::unique_ptr<SolvePlan>> plans;
   std::mutex plan_mutex;
-  std::atomic<bool> in_flight{true};      // as for DeviceTree
+  LastUse last_use;
   HodlrFactor();
   ~HodlrFactor();
 };

@@ -172,7 +172,7 @@ int hodlr_b200_tree_load(const char *path, hodlr_b200_tree *out) {
       HB_CUDA(cudaMemcpyAsync(dt->arena, img.data(), sizeof(double) * dt->arena_elems,
                               cudaMemcpyHostToDevice, s));
     HB_CUDA(cudaStreamSynchronize(s));
-    dt->in_flight = false;
+    dt->last_use.settled();
     *out = new hodlr_b200_tree_s{dt};
     return SUCCESS;
   } catch (const Error &e) {

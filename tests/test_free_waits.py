@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 import fake_runtime as F
+from hmat_lib_b200 import hodlr
 from hmat_lib_b200 import workloads as W
 from hmat_lib_b200.hodlr import DeviceTree, matmat_batched
 
@@ -87,16 +88,47 @@ def test_factor_free_waits_for_solves(fake, tree_first):
         assert lib.fake_frees_under_work() == 0
 
 
-def test_free_of_what_no_call_uses_does_not_wait(fake):
+def test_free_of_what_no_queued_work_uses_does_not_wait(fake):
     with F.loaded(*fake) as lib:
         x = np.zeros((128, 128))
         t = DeviceTree.build(x.ctypes.data, 128, 128, 2, 1e-8, stream=64)
         loaded = F.device_tree()
         f = loaded.factorize(stream=64)
-        waits = lib.fake_device_waits()
-        for h in (f, loaded, t):
+        c = loaded.hxh(loaded, 1e-8)                    # waits for its work itself
+        host = hodlr.Tree.from_tree_data(F.tree_data(2, 32, 4))
+        host.matmat(x)                                  # on host buffers: so does this
+        waits, launches = lib.fake_device_waits(), lib.fake_launches()
+        for h in (f, c, loaded, t, host):
             h.free()
         assert lib.fake_device_waits() == waits
+        assert lib.fake_frees_under_work() == 0 and lib.fake_launches() == launches
+
+
+def test_of_many_frees_in_a_row_the_first_one_waits(fake):
+    with F.loaded(*fake) as lib:
+        trees = [F.device_tree() for _ in range(4)]
+        keep = [_product(lib, t, 128) for t in trees]
+        waits = lib.fake_device_waits()
+        for t in trees[:3]:
+            t.free()
+        assert lib.fake_device_waits() == waits + 1
+        keep.append(_product(lib, trees[3], 128))       # used again since
+        trees[3].free()
+        assert lib.fake_device_waits() == waits + 2
+        assert lib.fake_frees_under_work() == 0
+
+
+def test_waits_are_per_device(fake):
+    with F.loaded(*fake) as lib:
+        trees, keep = [], []
+        for dev in (0, 1):
+            lib.fake_set_device(dev)
+            trees.append(F.device_tree())
+            keep.append(_product(lib, trees[-1], 128))
+        lib.fake_set_device(0)
+        for t in trees:                                 # the second lives on device 1
+            t.free()
+        assert lib.fake_frees_under_work() == 0
 
 
 @pytest.mark.gpu
